@@ -1563,7 +1563,8 @@ __device__ __forceinline__ bool final_warp(const DecodeParams& p, uint32_t tb, u
     const uint8_t* stage = reinterpret_cast<const uint8_t*>(s_tab) + (stage_addr - tb);
     const uintptr_t base = (uintptr_t) p.out;
     unsigned long long a0 = wlo + ((16 - ((base + wlo) & 15)) & 15);
-    unsigned long long a1 = whi - ((base + whi) & 15);
+    // the range may end inside its first 16-byte line
+    unsigned long long a1 = whi - min(whi - wlo, (unsigned long long) ((base + whi) & 15));
     if (a0 > a1) a0 = a1 = whi;
     for (unsigned long long i = wlo + lane; i < a0; i += 32)
         p.out[i] = stage[sb + (i - wlo)];
