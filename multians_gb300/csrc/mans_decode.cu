@@ -54,6 +54,7 @@
 #include <vector>
 
 #include "mans_device.cuh"
+#include "mans_lattice.h"
 #include "mans_scan.cuh"
 #include "mans_tma.cuh"
 #include "mans_tune_table.h"
@@ -2245,6 +2246,15 @@ static int plan_core(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* h
          (kn ? (kn->capture && n_out > 0 && L <= kCaptureMaxL)
              : (n_out > 0 && L <= kCaptureMaxL && bps >= kCaptureMinBits &&
                 (n_units >= kCaptureMinUnits || (c.flags & MANS_DECODE_CAPTURE)))));
+    // the lattice decode where the plan is the planner's own (a plan given
+    // back as a hint keeps its choice)
+    const bool lattice =
+        !capture && n_out > 0 &&
+        ((c.flags & MANS_DECODE_LATTICE) ||
+         (c.block_units == 0 && c.region_blocks == 0 && c.walk_slots == 0 &&
+          !(c.flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS | MANS_DECODE_NO_CAPTURE |
+                       MANS_DECODE_CAPTURE | MANS_PLAN_MODEL))));
+    c.flags &= ~MANS_DECODE_LATTICE;
     if (kn && c.block_units == 0) c.block_units = kn->block_units;
     if (!capture) c.capture_bytes = 0;
     if (c.block_units == 0) {
@@ -2292,6 +2302,8 @@ static int plan_core(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* h
         const uint64_t R = (uint64_t) c.region_blocks * c.block_units;
         c.walk_slots = (uint32_t) std::min<uint64_t>(kMaxWalkSlots, std::max<uint64_t>(2, (tail + R - 1) / R + 1));
     }
+    // a lattice decode uses the records' memory for its slots
+    if (lattice && !(hint && hint->walk_slots)) c.walk_slots = kMaxWalkSlots;
     if (c.threads == 0) c.threads = 128;
     c.threads = std::min<uint32_t>(128, std::max<uint32_t>(32, c.threads & ~31u));
     if (capture && c.capture_bytes == 0) {
@@ -2310,6 +2322,7 @@ static int plan_core(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* h
     if (!(c.flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS)) && bps >= kSeedMinBits &&
         bps < (L >= 4096 ? kSeedMaxBitsLarge : kSeedMaxBits))
         c.flags |= MANS_DECODE_SEEDS;
+    if (lattice) c.flags |= MANS_DECODE_LATTICE;
     *out = c;
     return MANS_OK;
 }
@@ -2476,6 +2489,16 @@ static uint32_t start_pos(uint32_t first_bit, uint32_t flags) {
     return (flags & MANS_DECODE_START_OFFSET) ? first_bit : 32 - first_bit;
 }
 
+// The lattice geometry of a decode planned with `cfg` (false: not a lattice
+// decode, or none fits the workspace).  Trajectories side by side: 16 warps
+// on every SM.
+static bool lattice_plan(const mans_cfg& cfg, size_t n_units, size_t n_out, uint32_t L,
+                         size_t aux_bytes, LatPlan* out) {
+    if (!(cfg.flags & MANS_DECODE_LATTICE) || cfg.capture_bytes) return false;
+    const double bps = 32.0 * (double) n_units / (double) n_out;
+    return lat_plan(n_units, n_out, L, mean_meeting_units(L, bps), 152 * 16 * 32, aux_bytes, out);
+}
+
 // The decode's launch sequence; with sync_only the final pass is left out
 // (d_out is not used) and the parameters the passes ran with go to *p_out.
 static int decode_impl(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
@@ -2499,6 +2522,14 @@ static int decode_impl(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
     if ((uint64_t) nblk * cfg.block_units * 32 >= (1ull << 40)) return MANS_ERR_ARG;
 
     cudaStream_t st = (cudaStream_t) stream;
+    LatPlan lp;
+    if (!sync_only && lattice_plan(cfg, n_units, n_out, L, aux_bytes, &lp)) {
+        const LatCall call = {d_units, n_units, d_out, n_out, d_table, L, first_state - L,
+                              start_pos(first_bit, in_flags), cfg.flags};
+        g_last_launches = lat_decode(call, lp, d_aux, st, timing_mark);
+        if (g_timing.on && g_timing.used < g_timing.cap) ++g_timing.used;
+        return g_last_launches ? MANS_OK : MANS_ERR_CUDA;
+    }
     char* base = (char*) d_aux;
     DecodeParams p;
     p.units = d_units;
@@ -2763,6 +2794,23 @@ int mans_sync_stats_get(const void* d_aux, size_t aux_bytes, size_t n_units, siz
     const size_t nreg = (nblk + cfg.region_blocks - 1) / cfg.region_blocks;
     const AuxLayout lay = layout_for(nblk, nreg, cfg.walk_slots, cfg.capture_bytes);
     if (aux_bytes < lay.total) return MANS_ERR_AUX_SMALL;
+    LatPlan lp;
+    if (lattice_plan(cfg, n_units, n_out, L, aux_bytes, &lp)) {
+        // a lattice decode: trajectories in place of regions, the units they
+        // decoded past the first time as walks
+        mans_sync_stats s{};
+        uint64_t visits = 0, longest = 0;
+        if (!lat_stats(lp, d_aux, (cudaStream_t) stream, &visits, &longest)) return MANS_ERR_CUDA;
+        s.regions = lp.nseed;
+        s.blocks = lp.nblk;
+        s.walks = lp.nseed - 1;
+        s.walk_blocks = visits > lp.nblk ? visits - lp.nblk : 0;
+        s.walk_units = s.walk_blocks * lp.B;
+        s.walk_max_units = longest * lp.B;
+        s.metadata_bytes = visits * 8 + (uint64_t) lp.nblk * 12;
+        *out = s;
+        return MANS_OK;
+    }
     const size_t ntiles = (nreg + kScanTile - 1) / kScanTile;
     // the merge point of every region and the counters behind the scan
     // flags (flags, ticket, job count, next job, fallback warp count): all
@@ -2883,7 +2931,12 @@ int mans_decode_sync(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
                 c.flags |= MANS_DECODE_NO_CAPTURE;
                 continue;
             }
-            if (plan.walk_slots > 1) { c = plan; c.walk_slots = plan.walk_slots / 2; continue; }
+            if (plan.walk_slots > 1) {
+                c = plan;
+                c.walk_slots = plan.walk_slots / 2;
+                c.flags &= ~MANS_DECODE_LATTICE;
+                continue;
+            }
             return MANS_ERR_AUX_SMALL;
         }
         rc = mans_decode(d_units, n_units, d_out, n_out, d_table, L, first_state,
@@ -2898,6 +2951,7 @@ int mans_decode_sync(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
         c = plan;
         c.region_blocks = plan.region_blocks * 4;
         c.capture_bytes = 0;
+        c.flags &= ~MANS_DECODE_LATTICE;
     }
     if (status_out) *status_out = st;
     return mans_status_code(st);

@@ -1,0 +1,253 @@
+// Lattice decode: kernels and launches (the method is in mans_lattice.cuh).
+#include "mans_lattice.h"
+
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+
+#include "mans_lattice.cuh"
+
+namespace mans {
+namespace {
+
+// Tables (first CTA) and the zeroed words: counters, look-back words, slots.
+__global__ void __launch_bounds__(1024) k_lat_prep(LatParams p, uint4* zero, size_t n16) {
+    if (blockIdx.x == 0) lat_tables(p);
+    const size_t stride = (size_t) gridDim.x * blockDim.x;
+    for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride)
+        zero[i] = make_uint4(0, 0, 0, 0);
+}
+
+template <uint32_t kB>
+__global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
+    lat_sync_body<kB>(p);
+}
+
+template <uint32_t kD>
+__global__ void __launch_bounds__(kLatScanThreads) k_lat_scan(LatParams p) {
+    __shared__ uint32_t s_tile;
+    if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
+    __syncthreads();
+    lat_scan_body<kD>(p, s_tile);
+}
+
+template <bool kRev, uint32_t kB>
+__global__ void __launch_bounds__(kLatFinalThreads) k_lat_final(LatParams p) {
+    lat_final_body<kRev, kB>(p, blockIdx.x, gridDim.x);
+}
+
+// CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps, near
+// the rate its shared-memory lookups allow.
+constexpr uint32_t kLatCtas = 4;
+
+size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
+
+struct LatLayout {
+    size_t ctr, tile_map, tile_sum, key, zero_end, tab_cnt, tab_sym, node, start, total;
+};
+
+LatLayout lat_layout(size_t nblk, uint32_t D, uint32_t L) {
+    LatLayout a;
+    const size_t ntiles = (nblk + kLatScanTile - 1) / kLatScanTile;
+    size_t o = 256;   // status
+    a.ctr = o; o += 256;
+    a.tile_map = o; o += align256(ntiles * 8);
+    a.tile_sum = o; o += align256(ntiles * 8);
+    a.key = o; o += align256(nblk * D * 4);
+    a.zero_end = o;
+    a.tab_cnt = o; o += align256((size_t) L * 4);
+    a.tab_sym = o; o += align256((size_t) L * 4);
+    a.node = o; o += align256(nblk * D * 4);
+    a.start = o; o += align256(nblk * 8);
+    a.total = o;
+    return a;
+}
+
+size_t lat_sync_smem(uint32_t L, uint32_t B, uint32_t threads) {
+    return (size_t) L * 4 + lat_ring_bytes(B) * (threads / 32 + 1);
+}
+
+constexpr size_t kLatFinalSmemMax = 200 * 1024;
+size_t lat_final_smem(uint32_t L, uint32_t B, uint32_t stage_cap, uint32_t threads) {
+    return (size_t) L * 4 + (size_t) lat_final_warp_bytes(B) * (threads / 32 + 1) +
+           (size_t) (threads / 32) * (stage_cap + 16);
+}
+
+// Staging bytes per warp of the final pass: 1.25x the expected symbols of
+// 32 blocks, as far as eight warps fit an SM's shared memory.
+uint32_t lat_stage_cap(double per_unit, uint32_t B, uint32_t L) {
+    uint64_t cap = (uint64_t) (per_unit * 32.0 * B * 1.25) + 128;
+    cap = std::min<uint64_t>(std::max<uint64_t>(cap, 512), 16384);
+    const size_t warps = kLatFinalThreads / 32;
+    const size_t room = (kLatFinalSmemMax - lat_final_smem(L, B, 0, kLatFinalThreads)) / warps;
+    cap = std::min<uint64_t>(cap, room & ~(size_t) 15);
+    return (uint32_t) ((cap + 15) & ~(uint64_t) 15);
+}
+
+int sm_count() {
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+}
+
+// Opts the kernels in to large dynamic shared memory, once per device.
+void lat_attributes() {
+    static std::mutex mu;
+    static uint64_t done = 0;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 64 && ((done >> dev) & 1)) return;
+    const auto set = [](auto* k) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int) kLatFinalSmemMax);
+    };
+    set(k_lat_prep);
+    set(k_lat_sync<4>); set(k_lat_sync<8>); set(k_lat_sync<16>);
+    set(k_lat_final<false, 4>); set(k_lat_final<false, 8>); set(k_lat_final<false, 16>);
+    set(k_lat_final<true, 4>); set(k_lat_final<true, 8>); set(k_lat_final<true, 16>);
+    if (dev < 64) done |= 1ull << dev;
+}
+
+template <bool kRev>
+void (*final_kernel(uint32_t B))(LatParams) {
+    return B == 4 ? k_lat_final<kRev, 4> : (B == 8 ? k_lat_final<kRev, 8> : k_lat_final<kRev, 16>);
+}
+
+LatParams lat_params(const LatCall& call, const LatPlan& plan, char* base) {
+    const LatLayout a = lat_layout(plan.nblk, plan.D, call.L);
+    LatParams p{};
+    p.units = call.units;
+    p.out = call.out;
+    p.table = call.table;
+    p.status = (uint32_t*) base;
+    p.ctr = (uint32_t*) (base + a.ctr);
+    p.tile_map = (unsigned long long*) (base + a.tile_map);
+    p.tile_sum = (unsigned long long*) (base + a.tile_sum);
+    p.key = (uint32_t*) (base + a.key);
+    p.tab_cnt = (uint32_t*) (base + a.tab_cnt);
+    p.tab_sym = (uint32_t*) (base + a.tab_sym);
+    p.node = (uint32_t*) (base + a.node);
+    p.start = (unsigned long long*) (base + a.start);
+    p.n_out = call.n_out;
+    p.n_units = (uint32_t) call.n_units;
+    p.L = call.L;
+    p.first_idx = call.first_idx;
+    p.first_pos = call.first_pos;
+    p.B = plan.B;
+    p.nb = plan.nb;
+    p.D = plan.D;
+    p.nblk = plan.nblk;
+    p.nseed = plan.nseed;
+    p.stage_cap = lat_stage_cap((double) call.n_out / (double) call.n_units, plan.B, call.L);
+    p.flags = call.flags;
+    return p;
+}
+
+}  // namespace
+
+bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
+              LatPlan* out) {
+    if (n_out >> (63 - kLatEntBits)) return false;
+    // about 128 symbols per block: the final pass stages 32 blocks a warp,
+    // and a step's share of a block's bookkeeping stays below a tenth
+    const double spu = (double) n_out / (double) n_units;
+    uint32_t b_pref = 16;
+    while (b_pref > 4 && spu * b_pref > 192.0) b_pref /= 2;
+    // Starts every s units: as many as run side by side, but no closer than
+    // the slots allow (about 1.2 sqrt(2 meet / s) distinct trajectories are
+    // under way at a place on average, twice that at most over a long
+    // stream; data that meets later than the model has it costs repairs).
+    const double s_par = std::max((double) n_units / lanes, 4.0);
+    uint32_t D = s_par >= 4.0 * meet ? 4 : (s_par >= meet / 1.5 ? 8 : 12);
+    for (; D >= 4; D -= 4) {
+        const double s = std::max(s_par, D == 12 ? meet / 6.0 : (D == 8 ? meet / 1.5 : 4.0 * meet));
+        uint32_t B = b_pref;
+        while (B > 4 && B > s) B /= 2;
+        for (; B <= 16; B *= 2) {
+            const size_t nblk = n_units / B + 1;
+            if (nblk * D > 0xffffffffull) continue;
+            const size_t need = lat_layout(nblk, D, L).total;
+            if (need > bytes) continue;
+            out->B = B;
+            out->nb = (uint32_t) std::max(1.0, std::floor(s / B + 0.5));
+            out->D = D;
+            out->nblk = (uint32_t) nblk;
+            out->nseed = (uint32_t) ((nblk + out->nb - 1) / out->nb);
+            out->bytes = need;
+            return true;
+        }
+    }
+    return false;
+}
+
+uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaStream_t st,
+                    void (*mark)(int, cudaStream_t)) {
+    char* base = (char*) d_aux;
+    const LatLayout a = lat_layout(plan.nblk, plan.D, call.L);
+    LatParams p = lat_params(call, plan, base);
+    lat_attributes();
+    const int sms = sm_count();
+    const size_t n16 = (a.zero_end - a.ctr) / 16;
+    mark(0, st);
+    const unsigned gz = 1 + (unsigned) std::min<size_t>((n16 + 8191) / 8192, 2 * sms - 1);
+    k_lat_prep<<<gz, 1024, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
+    mark(1, st);
+    // sync pass
+    {
+        // few trajectories: narrow warps spread over the schedulers of all SMs
+        uint32_t th = kLatThreads, width = 32;
+        const uint32_t sched = 4u * sms;
+        if (plan.nseed <= 8 * sched) width = 8;
+        else if (plan.nseed <= 16 * sched) width = 16;
+        if (plan.nseed <= width * sched) th = 32;
+        p.width = width;
+        const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
+        const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
+        const size_t sm = lat_sync_smem(call.L, plan.B, th);
+        if (plan.B == 4) k_lat_sync<4><<<grid, th, sm, st>>>(p);
+        else if (plan.B == 8) k_lat_sync<8><<<grid, th, sm, st>>>(p);
+        else k_lat_sync<16><<<grid, th, sm, st>>>(p);
+    }
+    mark(2, st);
+    mark(3, st);
+    {
+        const unsigned g = (plan.nblk + kLatScanTile - 1) / kLatScanTile;
+        if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, 0, st>>>(p);
+        else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, 0, st>>>(p);
+        else k_lat_scan<12><<<g, kLatScanThreads, 0, st>>>(p);
+    }
+    mark(4, st);
+    {
+        const unsigned groups = (plan.nblk + 31) / 32;
+        uint32_t th = kLatFinalThreads;
+        while (th > 64 && groups < (th / 32) * 2u * sms) th /= 2;
+        const size_t sm = lat_final_smem(call.L, plan.B, p.stage_cap, th);
+        auto* k = (call.flags & MANS_DECODE_SOURCE_ORDER) ? final_kernel<true>(plan.B)
+                                                          : final_kernel<false>(plan.B);
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, th, sm) != cudaSuccess ||
+            per_sm < 1)
+            per_sm = 1;
+        const unsigned need = (groups + th / 32 - 1) / (th / 32);
+        k<<<std::min<unsigned>(need, (unsigned) (per_sm * sms)), th, sm, st>>>(p);
+    }
+    mark(5, st);
+    return cudaGetLastError() == cudaSuccess ? 4u : 0u;
+}
+
+bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t st, uint64_t* visits,
+               uint64_t* longest) {
+    uint32_t c[8] = {};
+    if (cudaMemcpyAsync(c, (const char*) d_aux + 256, sizeof(c), cudaMemcpyDeviceToHost, st) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return false;
+    (void) plan;
+    *visits = c[kLatVisits];
+    *longest = c[kLatMaxLife];
+    return true;
+}
+
+}  // namespace mans

@@ -1,0 +1,47 @@
+// Host interface of the lattice decode (mans_lattice.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace mans {
+
+struct LatPlan {
+    uint32_t B;       // units per block
+    uint32_t nb;      // blocks between starts
+    uint32_t D;       // slots per block
+    uint32_t nblk;
+    uint32_t nseed;
+    size_t bytes;     // workspace
+};
+
+// The geometry of a lattice decode of n_units units in at most `bytes` of
+// workspace; `meet` is the mean meeting distance in units and `lanes` the
+// trajectories the GPU runs side by side for this stream.  False when no
+// geometry fits.
+bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
+              LatPlan* out);
+
+struct LatCall {
+    const uint32_t* units;
+    size_t n_units;
+    uint8_t* out;
+    size_t n_out;
+    const uint32_t* table;
+    uint32_t L, first_idx, first_pos, flags;
+};
+
+// Enqueues the decode in the workspace at d_aux (its first word is the
+// status).  `mark(i)` is called before each of the five timed kernel slots
+// and after the last.  Returns the number of kernels, or 0 on a CUDA error.
+uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaStream_t stream,
+                    void (*mark)(int, cudaStream_t));
+
+// What the trajectories of the last lattice decode in d_aux cost (waits for
+// the stream): blocks decoded by all of them, blocks of the longest.
+bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t stream, uint64_t* visits,
+               uint64_t* longest);
+
+}  // namespace mans
