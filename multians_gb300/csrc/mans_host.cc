@@ -417,10 +417,39 @@ int mans_host_encode_tables(const uint64_t* hist, uint32_t L, uint32_t table_see
     for (int v = 0; v < 256; ++v) n += hist[v];
     if (n == 0) return MANS_ERR_ARG;
     auto d = ANSTableGenerator::generate_distribution_from_histogram(table_seed, L, hist);
-    auto t = ANSTableGenerator::generate_table(d.prob, d.dist, d.symbols, d.symbols->size(), L);
-    auto enc = ANSTableGenerator::generate_encoder_table(t);
-    auto dec = ANSTableGenerator::get_decoder_table(enc);
-    std::memcpy(dec_table, dec->get(), (size_t) L * sizeof(uint32_t));
+    const size_t K = d.symbols->size();
+    // The spread of generate_table: state L + i goes to the symbol with the
+    // smallest key (the first one on ties), whose key starts at 0.5 / p and
+    // grows by 1 / p per state it takes.  That order is the sorted order of
+    // all keys, one per unit of key length on average: the keys are put into
+    // a bucket per unit and each bucket sorted (L = 4096, 256 symbols: 29 ms
+    // through the 256 x L table of the class interface -> 0.1 ms).
+    struct Key {
+        double key;
+        uint32_t sym;   // index of the symbol
+    };
+    std::vector<Key> keys;
+    keys.reserve(L + K);
+    std::vector<uint32_t> start(L + 2, 0);
+    const auto bucket = [L](double k) { return k < (double) L ? (uint32_t) k : L; };
+    for (size_t i = 0; i < K; ++i) {
+        const double step = 1.0 / d.prob->at(i);
+        double k = 0.5 / d.prob->at(i);
+        // its count of keys, and one more in case the roundings favour it
+        for (size_t m = 0; m <= d.dist->at(i); ++m, k = k + step) {
+            keys.push_back({k, (uint32_t) i});
+            ++start[bucket(k) + 1];
+        }
+    }
+    for (uint32_t i = 0; i <= L; ++i) start[i + 1] += start[i];
+    std::vector<Key> order(keys.size());
+    std::vector<uint32_t> at(start.begin(), start.end() - 1);
+    for (const Key& k : keys) order[at[bucket(k.key)]++] = k;
+    for (uint32_t i = 0; i <= L; ++i)
+        std::sort(order.begin() + start[i], order.begin() + start[i + 1],
+                  [](const Key& x, const Key& y) {
+                      return x.key < y.key || (x.key == y.key && x.sym < y.sym);
+                  });
     // Compact encoder table (the encoder kernels' format).  Encoding byte s
     // from state X in [L, 2L) shifts out k low bits with (X >> k) in
     // [f, 2f) (f = the byte's normalised count) and moves to the spread
@@ -429,39 +458,38 @@ int mans_host_encode_tables(const uint64_t* hist, uint32_t L, uint32_t table_see
     // is next[base + (X >> k)] with base = (first slot of s) - f.
     //   words 0..511: per byte {delta, base} (base = ~0: byte absent)
     //   then L / 2 words: next states as uint16 (L + spread index)
-    const size_t K = d.symbols->size();
     uint32_t lg = 0;
     while ((1u << lg) < L) ++lg;
-    std::vector<uint32_t> first(256, 0), cnt(256, 0);
+    for (int v = 0; v < 256; ++v) {
+        enc_blob[2 * v] = 0;
+        enc_blob[2 * v + 1] = ~0u;
+    }
+    std::vector<uint32_t> first(K), x_next(K);
     uint32_t slot = 0;
     for (size_t i = 0; i < K; ++i) {
-        const SYMBOL_TYPE sv = d.symbols->at(i);
-        cnt[sv] = (uint32_t) d.dist->at(i);
-        first[sv] = slot;
-        slot += cnt[sv];
+        const uint32_t f = (uint32_t) d.dist->at(i);
+        first[i] = slot;
+        x_next[i] = f;
+        slot += f;
+        uint32_t bl = 0;
+        while (bl < 32 && ((f - 1) >> bl) != 0) ++bl;
+        const uint32_t m = lg + 1 - bl;
+        const SYMBOL_TYPE s = d.symbols->at(i);
+        enc_blob[2 * s] = (m << 16) - (f << m);
+        enc_blob[2 * s + 1] = first[i] - f;
     }
     if (slot != L) return MANS_ERR_TABLE;
-    for (int v = 0; v < 256; ++v) {
-        if (cnt[v] == 0) {
-            enc_blob[2 * v] = 0;
-            enc_blob[2 * v + 1] = ~0u;
-            continue;
-        }
-        uint32_t bl = 0;
-        while (bl < 32 && ((cnt[v] - 1) >> bl) != 0) ++bl;
-        const uint32_t m = lg + 1 - bl;
-        enc_blob[2 * v] = (m << 16) - (cnt[v] << m);
-        enc_blob[2 * v + 1] = first[v] - cnt[v];
-    }
+    // the decoder entry of spread state L + i undoes the encoder step: the
+    // symbol, x = X >> k, and the k that brings x << k into [L, 2L)
     uint16_t* next = reinterpret_cast<uint16_t*>(enc_blob + 512);
-    for (int v = 0; v < 256; ++v) {
-        if (cnt[v] == 0) continue;
-        const auto& row = enc->table[v];
-        for (uint32_t X = L; X < 2 * L; ++X) {
-            const auto& e = row[X - L];
-            const uint32_t xs = X >> e.code_length;
-            next[first[v] + xs - cnt[v]] = (uint16_t) e.next_state;
-        }
+    for (uint32_t i = 0; i < L; ++i) {
+        const uint32_t q = order[i].sym;
+        const uint32_t f = (uint32_t) d.dist->at(q), x = x_next[q]++;
+        if (x >= 2 * f) return MANS_ERR_TABLE;   // one key too many: cannot be
+        uint32_t k = 0;
+        while ((x << k) < L) ++k;
+        dec_table[i] = x | ((uint32_t) d.symbols->at(q) << 16) | (k << 24);
+        next[first[q] + x - f] = (uint16_t) (L + i);
     }
     return MANS_OK;
 }
