@@ -485,10 +485,11 @@ int mans_host_encode(const uint8_t* sym, size_t n, uint32_t L, uint32_t table_se
  *                           (mans_encode_blob_words words)
  *   mans_encode             encodes n bytes (d_sym 16-byte aligned) into
  *                           d_units (mans_encode_max_units words); workspace
- *                           mans_encode_aux_size bytes; chunk_hint 0 = plan
+ *                           mans_encode_aux_size bytes; chunk_hint: bytes
+ *                           between the places encoding starts, 0 = plan
  *                           (async)
  *   mans_encode_result      n_units, first_bit, first_state (synchronous);
- *                           MANS_ERR_SYNC: merges ran out of slots, retry
+ *                           MANS_ERR_SYNC: the path ran out of slots, retry
  *                           with a larger chunk_hint */
 size_t mans_encode_blob_words(uint32_t L);
 int mans_histogram(const uint8_t* d_sym, size_t n, uint64_t* d_hist, void* stream);
@@ -501,8 +502,8 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
                 uint32_t chunk_hint, void* stream);
 int mans_encode_result(const void* d_aux, void* stream, uint64_t* n_units, uint32_t* first_bit,
                        uint32_t* first_state, uint32_t* dev_status);
-/* mans_encode + mans_encode_result, re-planning with 4x longer chunks while
- * the merges outrun their slots (workspace: mans_encode_aux_size(n, 0)). */
+/* mans_encode + mans_encode_result, re-planning with starts four times as
+ * far apart while the path runs out of slots (workspace: mans_encode_aux_size(n, 0)). */
 int mans_encode_sync(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint32_t L,
                      uint32_t* d_units, size_t cap_units, void* d_aux, size_t aux_bytes,
                      void* stream, uint64_t* n_units, uint32_t* first_bit,

@@ -6,360 +6,485 @@
 // Encoding is sequential in the state: x' = next(s, x >> k(s, x)), and the
 // code of each byte is the k low bits of x.  But two encodes of the same
 // bytes from different states meet after a while and agree from there on,
-// so the decoder's method carries over with symbol positions in place of
-// bit positions:
+// so the lattice decode's method carries over (mans_lattice.cuh), with byte
+// positions in place of bit positions and the state alone as the entry:
 //
-//  k_enc_g     one lane per chunk of Cs bytes encodes it from the initial
-//              state (the guess), recording at every block of Bs bytes the
-//              state and the code bits so far (rec_g), and its end record.
-//  k_enc_w     one lane per chunk k walks Gamma_k past its chunk end and
-//              compares it at every block start with Gamma_{k+1} (its
-//              records inside chunk k+1, a second cursor beyond) until the
-//              states agree: merge point m_k, bit difference delta_k.
-//  k_scan      M_k = max m_0..m_{k-1}, D_k = sum delta_0..delta_{k-1}
-//              (the decoder's scan).
-//  k_enc_total the owner of the stream end gives the total bit count T,
-//              n_units = floor(T / 32) + 1 and first_bit = T mod 32.
-//  k_enc_final one lane per block: its owner's record gives the true state
-//              and bit offset; it encodes the block again and writes the
-//              codes at that offset (units shared with a neighbour by
-//              atomicOr), in reversed unit order.
-//  k_enc_tail  the reference's flush puts more code bits below the last
-//              unit's valid bits (the last byte's code again when it fitted
-//              its unit, else the code of byte value 0 past the end); they
-//              are reproduced so the units match bit for bit.
+//  k_enc_zero  clears the counters, the look-back words and the slots.
+//  k_enc_sync  trajectories start from the initial state every S bytes and
+//              each ends at the first other one it meets at a block start;
+//              every (block, slot) node gets its code bits and the slot it
+//              leads to.
+//  k_enc_scan  the true path's slot, state and bit offset at every block; at
+//              its end the total bit count T, n_units = floor(T / 32) + 1 and
+//              first_bit = T mod 32.
+//  k_enc_final one lane per block encodes it from its true state and writes
+//              the codes at its bit offset, 32 blocks staged in shared memory
+//              and copied out in reversed unit order; the last lane adds the
+//              bits the reference's flush leaves below the last unit's valid
+//              bits (the last byte's code again when it fitted its unit, else
+//              the code of byte value 0 past the end).
 //
 // Tables: the compact encoder table built on the host from the byte
-// histogram (mans_host_encode_tables), loaded into shared memory per CTA:
-// per byte {delta, base} and the L next states (uint16).  L is a power of
-// two <= 8192.
+// histogram (mans_host_encode_tables), loaded into shared memory per CTA.
+// L is a power of two <= 8192.
+//
+// Measured on GB300, 64 MB at 3.8 bits per symbol and L = 4096: 359 us sync,
+// 31 scan, 109 final; chunks with merge walks took 195 + 1374 us, found their
+// slots too few, and again 744 + 1327 + 305 us with longer chunks.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 
-#include "mans_scan.cuh"
+#include "mans_lattice_scan.cuh"
+#include "mans_tma.cuh"
 #include "multians_gb300.h"
 
 namespace mans {
 namespace {
 
-constexpr uint32_t kEncThreads = 128;
-constexpr uint32_t kEncBlock = 256;        // bytes per block (records, final-pass lanes)
-constexpr uint32_t kEncSlots = 8;          // chunks a walk may cross
+constexpr uint32_t kEncThreads = 128;        // sync pass
+constexpr uint32_t kEncCtas = 3;             // per SM, of the persistent sync pass
+constexpr uint32_t kEncFinalThreads = 256;
+constexpr uint32_t kEncSmallBytes = 1u << 20;
 
 struct EncResult {
     unsigned long long total_bits;
     unsigned long long n_units;
     uint32_t first_bit, first_state;
     uint32_t last_code, last_len;          // the last byte's code
-    uint32_t owner_end;                    // chunk whose trajectory owns the end
-    uint32_t pad;
+};
+
+struct EncEnd {                            // a trajectory's end at the last block
+    uint32_t state, bits, code, len;
 };
 
 struct EncParams {
     const uint8_t* sym;
     unsigned long long n;
     const uint32_t* blob;                  // global compact table
-    uint32_t L, Cs, nb, nchunk, nblk, dmax;
-    uint2* rec_g;                          // [nblk] {state, bits since chunk start}
-    uint2* rec_w;                          // [nblk * dmax]
-    uint4* end_rec;                        // [nchunk] {state, bits lo, last code, last len}
-    unsigned long long* m;
-    long long* delta;
-    unsigned long long* Mpre;
-    long long* Dpre;
-    ScanTile* scan_tiles;
-    uint32_t* scan_flags;
+    uint32_t L, Bs, nb, D, nblk, nseed, width;
+    uint32_t* key;
+    uint32_t* node;
+    unsigned long long* start;
+    unsigned long long* tile_map;
+    unsigned long long* tile_sum;
+    uint32_t* ctr;
     uint32_t* status;
-    uint32_t nreg;                         // = nchunk (scan)
     EncResult* result;
+    EncEnd* end;                           // [D] by slot at the last block
     uint32_t* units;
     unsigned long long cap;                // units capacity (words)
+
+    // scan hooks (mans_lattice_scan.cuh): an entry is the state - L, an
+    // offset counts bits
+    __device__ __forceinline__ uint32_t repair_blocks() const { return n <= 16384 ? ~0u : 64u; }
+    __device__ __forceinline__ void set_result(const EncEnd& e, unsigned long long off) const {
+        const unsigned long long T = off + e.bits;
+        result->total_bits = T;
+        result->n_units = T / 32 + 1;
+        result->first_bit = (uint32_t) (T & 31);
+        result->first_state = e.state;
+        result->last_code = e.code;
+        result->last_len = e.len;
+        if (T / 32 + 1 + 4 > cap) atomicOr(status, MANS_DEV_COUNT_MISMATCH);
+    }
+    __device__ __forceinline__ void finish(uint32_t slot, unsigned long long off) const {
+        set_result(end[slot], off);
+    }
+    __device__ __forceinline__ void repair_load(uint32_t* sm) const {
+        for (uint32_t i = threadIdx.x; i < 512 + (L + 1) / 2; i += blockDim.x) sm[i] = __ldg(blob + i);
+    }
+    // one block, by one thread
+    __device__ __forceinline__ EncEnd block(const uint32_t* sm, uint32_t b, uint32_t ent) const {
+        EncEnd e = {L + min(ent, L - 1), 0, 0, 0};
+        const unsigned long long i1 = min((unsigned long long) (b + 1) * Bs, n);
+        const uint16_t* nx = reinterpret_cast<const uint16_t*>(sm + 512);
+        for (unsigned long long i = (unsigned long long) b * Bs; i < i1; ++i) {
+            const uint32_t s = sym[i];
+            e.len = min((e.state + sm[2 * s]) >> 16, 31u);
+            e.code = e.state & ((1u << e.len) - 1u);
+            e.bits += e.len;
+            const uint32_t next = nx[min(sm[2 * s + 1] + (e.state >> e.len), L - 1)];
+            e.state = min(max(next, L), 2 * L - 1);
+        }
+        return e;
+    }
+    __device__ __forceinline__ void advance(const uint32_t* sm, uint32_t b, uint32_t& ent,
+                                            unsigned long long& off) const {
+        const EncEnd e = block(sm, b, ent);
+        ent = e.state - L;
+        off += e.bits;
+    }
+    __device__ __forceinline__ void finish_seq(const uint32_t* sm, uint32_t ent,
+                                               unsigned long long off) const {
+        set_result(block(sm, nblk - 1, ent), off);
+    }
 };
 
-// Shared tables: 256 x uint2 {delta, base}, then L uint16 next states.
-__device__ __forceinline__ void load_enc_tables(uint2* s_sym, uint16_t* s_next,
-                                                const uint32_t* __restrict__ blob, uint32_t L) {
-    for (uint32_t v = threadIdx.x; v < 256; v += blockDim.x)
-        s_sym[v] = make_uint2(__ldg(blob + 2 * v), __ldg(blob + 2 * v + 1));
-    const uint32_t* nx = blob + 512;
-    uint32_t* s32 = reinterpret_cast<uint32_t*>(s_next);
-    for (uint32_t i = threadIdx.x; i < L / 2; i += blockDim.x) s32[i] = __ldg(nx + i);
+// Shared tables: per byte value {delta, shared address of the next state of
+// x >> k = 0}, then the L next states as uint16; k = (x + delta) >> 16.
+// Entries that do not have the table's form (absent bytes, which the data
+// does not hold) lead to the first next state with k = 31, so every address
+// stays inside the table.
+__device__ __forceinline__ void load_enc_tables(uint32_t tb, const uint32_t* __restrict__ blob,
+                                                uint32_t L) {
+    const uint32_t nx = tb + 256 * 8;
+    const uint32_t lg = 31 - __clz(L);
+    for (uint32_t v = threadIdx.x; v < 256; v += blockDim.x) {
+        const uint32_t delta = __ldg(blob + 2 * v), base = __ldg(blob + 2 * v + 1);
+        const uint32_t m = (delta + 0xffffu) >> 16;
+        const uint32_t thr = (m << 16) - delta;
+        const uint32_t f = m <= lg + 1 ? thr >> m : 0u;
+        const uint32_t first = base + f;
+        const bool ok = m >= 1 && f >= 1 && f <= L && thr == f << m &&
+                        m == lg + 1 - (f > 1 ? 32 - __clz(f - 1) : 0) && first <= L - f;
+        sts32(tb + v * 8, ok ? delta : 31u << 16);
+        sts32(tb + v * 8 + 4, ok ? nx + base * 2 : nx);
+    }
+    const uint32_t* g = blob + 512;
+    for (uint32_t i = threadIdx.x; i < (L + 1) / 2; i += blockDim.x) {
+        const uint32_t w = __ldg(g + i);
+        const uint32_t lo = min(max(w & 0xffffu, L), 2 * L - 1), hi = min(max(w >> 16, L), 2 * L - 1);
+        sts32(nx + i * 4, lo | hi << 16);
+    }
     __syncthreads();
 }
 
-// One encode step of byte s from state x: returns k (the code length) and
-// the code; x becomes the next state.  Bytes absent from the table never
-// occur in the data the table was built from.
-__device__ __forceinline__ uint32_t enc_step(uint32_t& x, uint32_t s, const uint2* s_sym,
-                                             const uint16_t* s_next, uint32_t L,
-                                             uint32_t& code) {
-    const uint2 q = s_sym[s];
+__host__ __device__ constexpr uint32_t enc_table_bytes(uint32_t L) {
+    return (256 * 8 + ((L + 1) / 2) * 4 + 15) & ~15u;
+}
+
+// Table loads: not volatile, so that the byte values' entries, which do not
+// depend on the state, are loaded ahead of the chain that does.
+__device__ __forceinline__ uint32_t lds_next(uint32_t a) {
+    uint32_t v;
+    asm("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds_entry(uint32_t a) {
+    uint2 v;
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+// 16 bytes global -> shared, zero-filled past `bytes`.
+__device__ __forceinline__ void cp16(uint32_t dst, const uint8_t* src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" :: "n"(kLeft) : "memory");
+}
+
+// One encode step of byte value s from state x: returns k; x becomes the
+// next state.  A chain of add, shift, shift, address and table load: 50
+// cycles a byte (the same with the code length chosen by a threshold test on
+// x, 60 with both of its shifts started from x at once), 5.8 a warp and byte
+// with 16 warps.
+__device__ __forceinline__ uint32_t enc_step(uint32_t& x, uint32_t s, uint32_t tb) {
+    const uint2 q = lds_entry(tb + s * 8);
     const uint32_t k = (x + q.x) >> 16;
-    code = x & ((1u << k) - 1u);
-    const uint32_t idx = min(q.y + (x >> k), L - 1);   // clamped: absent bytes stay in range
-    x = s_next[idx];
+    x = lds_next(q.y + 2 * (x >> k));
     return k;
 }
 
-// A lane's bytes [start, end), read 16 at a time (start is 16-byte aligned;
-// the group that crosses `end` is read byte by byte, so nothing past the
-// buffer is touched).
-struct ByteReader {
-    const uint8_t* p;
-    unsigned long long g, n;   // next 16-byte group, end
-    uint4 cur;
-    uint32_t pos;              // next byte within cur; 16 = empty
-    __device__ __forceinline__ void init(const uint8_t* base, unsigned long long start,
-                                         unsigned long long end) {
-        p = base;
-        g = start;
-        n = end;
-        pos = 16;
+// Copies block b of the source into a lane's row (bytes past the end zero).
+template <uint32_t kBs>
+__device__ __forceinline__ void enc_fetch(uint32_t row, const EncParams& p, uint32_t b) {
+    const unsigned long long i0 = (unsigned long long) b * kBs;
+#pragma unroll
+    for (uint32_t i = 0; i < kBs / 16; ++i) {
+        const unsigned long long at = i0 + 16 * i;
+        const uint32_t have = at < p.n ? (uint32_t) min(p.n - at, 16ull) : 0u;
+        cp16(row + 16 * i, p.sym + (have ? at : 0), have);
     }
-    __device__ __forceinline__ uint32_t next() {
-        if (pos == 16) {
-            if (g + 16 <= n) {
-                cur = __ldg(reinterpret_cast<const uint4*>(p + g));
-            } else {
-                uint32_t w[4] = {0, 0, 0, 0};
-                for (uint32_t t = 0; t < 16; ++t)
-                    if (g + t < n) w[t >> 2] |= (uint32_t) p[g + t] << (8 * (t & 3));
-                cur = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-            g += 16;
-            pos = 0;
-        }
-        const uint32_t w = pos < 8 ? (pos < 4 ? cur.x : cur.y) : (pos < 12 ? cur.z : cur.w);
-        const uint32_t b = (w >> (8 * (pos & 3))) & 0xffu;
-        ++pos;
-        return b;
-    }
-};
-
-__device__ __forceinline__ uint2 rec(uint32_t state, uint32_t bits) {
-    return make_uint2(state, bits);
+    cp_commit();
 }
 
-// G pass: chunk k from the initial state L.
-__global__ void __launch_bounds__(kEncThreads) k_enc_g(EncParams p) {
-    extern __shared__ __align__(16) uint2 s_sym[];
-    uint16_t* s_next = reinterpret_cast<uint16_t*>(s_sym + 256);
-    load_enc_tables(s_sym, s_next, p.blob, p.L);
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= p.nchunk) return;
-    const unsigned long long s0 = (unsigned long long) k * p.Cs;
-    const unsigned long long s1 = min(s0 + p.Cs, p.n);
-    uint32_t x = p.L, bits = 0, code = 0, len = 0;
-    ByteReader rd;
-    rd.init(p.sym, s0, s1);
-    uint32_t b = k * p.nb;
-    for (unsigned long long i = s0; i < s1; i += kEncBlock, ++b) {
-        p.rec_g[b] = rec(x, bits);
-        const unsigned long long e = min(i + kEncBlock, s1);
-        for (unsigned long long j = i; j < e; ++j) {
-            len = enc_step(x, rd.next(), s_sym, s_next, p.L, code);
-            bits += len;
-        }
-    }
-    if (k + 1 < p.nchunk) {
-        p.rec_w[(size_t) (k + 1) * p.nb * p.dmax] = rec(x, bits);   // Gamma_k at chunk k+1
-    } else {
-        p.m[k] = ~0ull;
-        p.delta[k] = 0;
-        p.end_rec[k] = make_uint4(x, bits, code, len);
-    }
-}
+// Rows padded by 16 bytes, so that the lanes' 16-byte reads spread over all
+// banks: two blocks of a lane in the sync pass, one in the final pass.
+__host__ __device__ constexpr uint32_t enc_pair_bytes(uint32_t Bs) { return 2 * Bs + 16; }
+__host__ __device__ constexpr uint32_t enc_row_bytes(uint32_t Bs) { return Bs + 16; }
 
-// Merge walk of chunk k (k + 1 < nchunk), one lane each.
-__global__ void __launch_bounds__(kEncThreads) k_enc_w(EncParams p) {
-    extern __shared__ __align__(16) uint2 s_sym[];
-    uint16_t* s_next = reinterpret_cast<uint16_t*>(s_sym + 256);
-    load_enc_tables(s_sym, s_next, p.blob, p.L);
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k + 1 >= p.nchunk) return;
-    uint32_t b = (k + 1) * p.nb;                        // block the cursors stand at
-    const uint2 r0 = p.rec_w[(size_t) b * p.dmax];
-    uint32_t xa = r0.x, ca = r0.y;                      // Gamma_k
-    uint32_t xg = 0, cg = 0;                            // Gamma_{k+1} past its chunk
-    bool g_on = false;
-    uint32_t code = 0, len = 0;
-    ByteReader rd;
-    rd.init(p.sym, (unsigned long long) b * kEncBlock, p.n);
+// Sync pass: one lane per trajectory, persistent (the flow of
+// lat_sync_body in mans_lattice.cuh).  Bound by the longest trajectory's
+// chain on small inputs and by shared-memory lookups on large ones.
+template <uint32_t kBs>
+__global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
+    extern __shared__ __align__(16) uint32_t enc_sm[];
+    const uint32_t tb = smem_addr(enc_sm);
+    load_enc_tables(tb, p.blob, p.L);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t row = tb + enc_table_bytes(p.L) + threadIdx.x * enc_pair_bytes(kBs);
+    const uint32_t D = p.D, L = p.L;
+
+    bool on = false, exhausted = false;
+    uint32_t b = 0, x = 0, q = 0, val = 0, cas = 0, prev = 0, pbits = 0, life = 0, max_life = 0;
+    bool has_prev = false, first = false;
     for (;;) {
-        const uint32_t d = b / p.nb - k;
-        if (d > p.dmax) {
-            atomicOr(p.status, MANS_DEV_SYNC_OVERFLOW);
-            p.m[k] = ~0ull;
-            p.delta[k] = 0;
-            return;
+        const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
+        if (!exhausted && __popc(idle) >= min(p.width, 8u)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(p.ctr + kLatNext, (uint32_t) __popc(idle));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            exhausted = base + __popc(idle) >= p.nseed;
+            const uint32_t k = base + __popc(idle & ((1u << lane) - 1));
+            if (!on && lane < p.width && k < p.nseed) {
+                on = true;
+                b = k * p.nb;
+                first = k == 0;
+                x = L;
+                val = kLatKeyUsed;
+                if (first) {
+                    q = 0;
+                    p.key[0] = val;
+                } else {
+                    bool found;
+                    q = lat_take(p.key + (size_t) b * D, 1, D, val, found);
+                    if (found || q == kLatDead) on = false;
+                }
+                cas = 0;
+                has_prev = false;
+                life = 0;
+                if (on) {
+                    cp_wait<0>();
+                    enc_fetch<kBs>(row + (b & 1u) * kBs, p, b);
+                }
+            }
         }
-        if (d >= 1 && b != (k + 1) * p.nb) p.rec_w[(size_t) b * p.dmax + (d - 1)] = rec(xa, ca);
-        uint32_t gx, gc;
-        if (d == 1) {
-            const uint2 rg = p.rec_g[b];
-            gx = rg.x;
-            gc = rg.y;
+        if (!__any_sync(0xffffffffu, on)) {
+            if (exhausted) break;
+            continue;
+        }
+        if (!on) continue;
+        uint4 kn = make_uint4(0, 0, 0, 0);
+        const bool more = b + 1 < p.nblk;
+        uint32_t* const knext = p.key + (size_t) (b + 1) * D;
+        if (more) kn = lat_ld_slots(knext);
+        // the block after this one on its way while this one is encoded
+        enc_fetch<kBs>(row + ((b + 1) & 1u) * kBs, p, more ? b + 1 : b);
+        cp_wait<1>();
+        const uint32_t src = row + (b & 1u) * kBs;
+        uint32_t bits = 0, x_in = x, len = 0;
+        if (more) {
+            uint4 v = lds128(src);
+#pragma unroll 1
+            for (uint32_t i = 16; i <= kBs; i += 16) {
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                if (i < kBs) v = lds128(src + i);
+#pragma unroll
+                for (uint32_t t = 0; t < 16; ++t)
+                    bits += enc_step(x, (w[t >> 2] >> (8 * (t & 3))) & 0xffu, tb);
+            }
         } else {
-            if (!g_on) {
-                const uint2 r1 = p.rec_w[(size_t) b * p.dmax];   // Gamma_{k+1} entering chunk k+2
-                xg = r1.x;
-                cg = r1.y;
-                g_on = true;
-            }
-            gx = xg;
-            gc = cg;
-        }
-        if (xa == gx) {
-            p.m[k] = (unsigned long long) b * kEncBlock;
-            p.delta[k] = (long long) ca - (long long) gc;
-            return;
-        }
-        const unsigned long long i0 = (unsigned long long) b * kEncBlock;
-        const unsigned long long i1 = min(i0 + kEncBlock, p.n);
-        for (unsigned long long j = i0; j < i1; ++j) {
-            const uint32_t s = rd.next();
-            len = enc_step(xa, s, s_sym, s_next, p.L, code);
-            ca += len;
-            if (g_on) {
-                uint32_t c2;
-                cg += enc_step(xg, s, s_sym, s_next, p.L, c2);
+            // the last block: as many bytes as there are
+            const uint32_t cnt = (uint32_t) (p.n - (unsigned long long) b * kBs);
+            for (uint32_t i = 0; i < cnt; ++i) {
+                x_in = x;
+                len = enc_step(x, (lds32(src + (i & ~3u)) >> (8 * (i & 3))) & 0xffu, tb);
+                bits += len;
             }
         }
+        ++life;
+        bool found = false;
+        if (cas != 0) {
+            if (cas == val) found = true;
+            else q = lat_take(p.key + (size_t) b * D, q + 1, D, val, found);
+        }
+        if (has_prev) p.node[prev] = pbits | (q << 28);
+        if (found || q == kLatDead || !more) {
+            if (!more && !found && q != kLatDead)
+                p.end[q] = {x, bits, x_in & ((1u << len) - 1u), len};
+            on = false;
+            max_life = max(max_life, life);
+            continue;
+        }
+        prev = b * D + q;
+        has_prev = true;
+        pbits = bits;
+        val = kLatKeyUsed | (x - L);
+        uint32_t hit = kLatDead;
+        if (kn.x == val) hit = 0;
+        if (kn.y == val) hit = 1;
+        if (kn.z == val) hit = 2;
+        if (kn.w == val) hit = 3;
         ++b;
-        if (b >= p.nblk) {
-            // the stream ends before the trajectories agree
-            p.m[k] = ~0ull;
-            p.delta[k] = 0;
-            p.end_rec[k] = make_uint4(xa, ca, code, len);
-            return;
+        if (hit != kLatDead) {
+            p.node[prev] = pbits | (hit << 28);
+            on = false;
+            max_life = max(max_life, life);
+            continue;
         }
+        // the true start's trajectory has slot 0 of every block to itself
+        q = first ? 0u : (kn.y == 0 ? 1u : (kn.z == 0 ? 2u : 3u));
+        cas = lat_cas(knext + q, val);
     }
+    cp_wait<0>();
+    max_life = __reduce_max_sync(0xffffffffu, max_life);
+    if (lane == 0 && max_life) atomicMax(p.ctr + kLatMaxLife, max_life);
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_enc_scan(EncParams p) {
+template <uint32_t kD>
+__global__ void __launch_bounds__(kLatScanThreads) k_enc_scan(EncParams p) {
     __shared__ uint32_t s_tile;
-    if (threadIdx.x == 0)
-        s_tile = atomicAdd(p.scan_flags + (p.nreg + kScanTile - 1) / kScanTile, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
-    scan_body(p, s_tile);
+    lat_scan_body<EncParams, kD>(p, s_tile);
 }
 
-// Owner of symbol position i: the largest chunk k <= chunk(i) with
-// M_k <= i; d = chunk(i) - k.
-__device__ __forceinline__ bool enc_owner(const EncParams& p, unsigned long long i, uint32_t c,
-                                          uint32_t& k, uint32_t& d) {
-    for (d = 0;; ++d) {
-        if (d > c || d > p.dmax) return false;
-        if (p.Mpre[c - d] <= i) break;
-    }
-    k = c - d;
-    return true;
+__global__ void __launch_bounds__(256) k_enc_zero(uint4* a, size_t na, uint32_t* units, size_t nu) {
+    const size_t stride = (size_t) gridDim.x * blockDim.x;
+    const size_t t = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = t; i < na; i += stride) a[i] = make_uint4(0, 0, 0, 0);
+    // the units (any word alignment): words to the first 16-byte boundary,
+    // vectors, the rest
+    const size_t head = min(nu, (size_t) ((16 - ((uintptr_t) units & 15)) & 15) / 4);
+    const size_t nv = (nu - head) / 4;
+    uint4* v = reinterpret_cast<uint4*>(units + head);
+    for (size_t i = t; i < nv; i += stride) v[i] = make_uint4(0, 0, 0, 0);
+    for (size_t i = t; i < head; i += stride) units[i] = 0;
+    for (size_t i = head + nv * 4 + t; i < nu; i += stride) units[i] = 0;
 }
 
-__global__ void k_enc_total(EncParams p) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint32_t k = 0, d = 0;
-    const uint32_t c = p.nchunk - 1;
-    if (!enc_owner(p, p.n, c, k, d)) {
-        atomicOr(p.status, MANS_DEV_SYNC_OVERFLOW);
-        return;
-    }
-    const uint4 e = p.end_rec[k];
-    const unsigned long long T = (unsigned long long) (p.Dpre[k] + (long long) e.y);
-    EncResult* r = p.result;
-    r->total_bits = T;
-    r->n_units = T / 32 + 1;
-    r->first_bit = (uint32_t) (T & 31);
-    r->first_state = e.x;
-    r->last_code = e.z;
-    r->last_len = e.w;
-    r->owner_end = k;
-    if (T / 32 + 1 + 4 > p.cap) atomicOr(p.status, MANS_DEV_COUNT_MISMATCH);
+__device__ __forceinline__ void red_or_shared(uint32_t a, uint32_t v) {
+    asm volatile("red.shared.or.b32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
 }
 
-// Unit u of the forward stream lives at units[n_units - 1 - u].
-__device__ __forceinline__ void put_unit(uint32_t* units, unsigned long long n_units,
-                                         unsigned long long u, uint32_t w, bool shared) {
-    if (u >= n_units) return;
-    uint32_t* a = units + (n_units - 1 - u);
-    if (shared) atomicOr(a, w);
-    else *a = w;
+// Unit words a warp's 32 blocks may span.
+__host__ __device__ constexpr uint32_t enc_stage_words(uint32_t Bs, uint32_t lg) {
+    return (Bs * lg + 2 + 3) & ~3u;
 }
 
-__global__ void __launch_bounds__(kEncThreads) k_enc_final(EncParams p) {
-    extern __shared__ __align__(16) uint2 s_sym[];
-    uint16_t* s_next = reinterpret_cast<uint16_t*>(s_sym + 256);
-    load_enc_tables(s_sym, s_next, p.blob, p.L);
+// Final pass: a warp per 32 blocks; bound by instruction issue (about 25 a
+// byte).  Their source bytes come in coalesced
+// (cp.async into padded rows), every lane packs its block's codes MSB-first
+// into the warp's staging words (words it shares with a neighbour by atomic
+// OR), and the warp writes the words out in reversed unit order, coalesced;
+// only its first and last word may be shared with other warps.
+template <uint32_t kBs>
+__global__ void __launch_bounds__(kEncFinalThreads) k_enc_final(EncParams p) {
+    extern __shared__ __align__(16) uint32_t enc_sm[];
     if (*(volatile uint32_t*) p.status & (MANS_DEV_SYNC_OVERFLOW | MANS_DEV_SCAN_TIMEOUT |
                                           MANS_DEV_COUNT_MISMATCH))
         return;
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= p.nblk) return;
-    const unsigned long long n_units = p.result->n_units;
-    const unsigned long long i0 = (unsigned long long) b * kEncBlock;
-    const unsigned long long i1 = min(i0 + kEncBlock, p.n);
-    uint32_t k = 0, d = 0;
-    if (!enc_owner(p, i0, b / p.nb, k, d)) {
-        atomicOr(p.status, MANS_DEV_SYNC_OVERFLOW);
-        return;
-    }
-    const uint2 r = d == 0 ? p.rec_g[b] : p.rec_w[(size_t) b * p.dmax + (d - 1)];
-    const unsigned long long o = (unsigned long long) (p.Dpre[k] + (long long) r.y);
-    uint32_t x = min(max(r.x, p.L), 2 * p.L - 1);
-    // codes MSB-first from bit o: acc holds the pending bits of unit u
-    unsigned long long acc = 0;
-    uint32_t nbits = (uint32_t) (o & 31);
-    unsigned long long u = o >> 5;
-    bool first = true;
-    uint32_t code = 0, len = 0;
-    ByteReader rd;
-    rd.init(p.sym, i0, i1);
-    for (unsigned long long j = i0; j < i1; ++j) {
-        len = enc_step(x, rd.next(), s_sym, s_next, p.L, code);
-        acc = (acc << len) | code;
-        nbits += len;
-        if (nbits >= 32) {
-            nbits -= 32;
-            put_unit(p.units, n_units, u, (uint32_t) (acc >> nbits), first);
-            acc &= (1ull << nbits) - 1ull;
-            first = false;
-            ++u;
+    const uint32_t tb = smem_addr(enc_sm);
+    load_enc_tables(tb, p.blob, p.L);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const uint32_t lg = 31 - __clz(p.L);
+    constexpr uint32_t kRow = enc_row_bytes(kBs);
+    const uint32_t words = enc_stage_words(kBs, lg);
+    const uint32_t rows = tb + enc_table_bytes(p.L) + warp * (32 * kRow + words * 4);
+    const uint32_t stage = rows + 32 * kRow;
+    const EncResult res = *p.result;
+    const unsigned long long n_units = res.n_units;
+    const uint32_t groups = (p.nblk + 31) >> 5;
+    for (uint32_t g = blockIdx.x * nwarp + warp; g < groups; g += gridDim.x * nwarp) {
+        const uint32_t b = (g << 5) + lane;
+        // 32 blocks of source: 16-byte chunks, consecutive lanes consecutive
+        const unsigned long long i0 = (unsigned long long) g * 32 * kBs;
+#pragma unroll
+        for (uint32_t j = 0; j < kBs / 16; ++j) {
+            const uint32_t c = j * 32 + lane;
+            const unsigned long long at = i0 + 16ull * c;
+            const uint32_t have = at < p.n ? (uint32_t) min(p.n - at, 16ull) : 0u;
+            cp16(rows + (c / (kBs / 16)) * kRow + (c % (kBs / 16)) * 16, p.sym + (have ? at : 0), have);
         }
+        cp_commit();
+        const bool live = b < p.nblk;
+        const unsigned long long st = live ? __ldg(p.start + b) : 0ull;
+        const unsigned long long o = live ? st >> kLatEntBits : res.total_bits;
+        const unsigned long long o0 = __shfl_sync(0xffffffffu, o, 0);
+        unsigned long long o1 = res.total_bits;
+        if ((g + 1) * 32 < p.nblk) o1 = __ldg(p.start + (g + 1) * 32) >> kLatEntBits;
+        const unsigned long long u0 = o0 >> 5;
+        const uint32_t span = (uint32_t) min(((o1 + 31) >> 5) - u0, (unsigned long long) words);
+        for (uint32_t i = lane; i < span; i += 32) sts32(stage + i * 4, 0);
+        cp_wait<0>();
+        __syncwarp();
+        if (live) {
+            uint32_t x = p.L + min((uint32_t) st & ((1u << kLatEntBits) - 1), p.L - 1);
+            const unsigned long long left = p.n - (unsigned long long) b * kBs;
+            const uint32_t cnt = (uint32_t) min(left, (unsigned long long) kBs);
+            uint32_t nbits = (uint32_t) o & 31u;
+            uint32_t at = stage + (uint32_t) min((o >> 5) - u0, (unsigned long long) words - 1) * 4;
+            const uint32_t at_max = stage + (words - 1) * 4;
+            bool shared_word = true;   // the first word: other lanes' bits may be in it
+            uint32_t hi = 0, lo = 0;   // pending bits, newest at the bottom of lo
+            const auto put = [&](uint32_t code, uint32_t len) {
+                hi = __funnelshift_lc(lo, hi, len);
+                lo = (lo << len) | code;
+                nbits += len;
+                if (nbits >= 32) {
+                    nbits -= 32;
+                    const uint32_t w = __funnelshift_rc(lo, hi, nbits);
+                    if (shared_word) red_or_shared(at, w);
+                    else sts32(at, w);
+                    shared_word = false;
+                    at = min(at + 4, at_max);
+                }
+            };
+            const uint32_t src = rows + lane * kRow;
+            if (cnt == kBs) {
+#pragma unroll 1
+                for (uint32_t i = 0; i < kBs; i += 16) {
+                    const uint4 v = lds128(src + i);
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (uint32_t t = 0; t < 16; ++t) {
+                        const uint32_t x0 = x;
+                        const uint32_t len = enc_step(x, (w[t >> 2] >> (8 * (t & 3))) & 0xffu, tb);
+                        put(x0 & ((1u << len) - 1u), len);
+                    }
+                }
+            } else {
+                for (uint32_t i = 0; i < cnt; ++i) {
+                    const uint32_t x0 = x;
+                    const uint32_t len = enc_step(x, (lds32(src + (i & ~3u)) >> (8 * (i & 3))) & 0xffu, tb);
+                    put(x0 & ((1u << len) - 1u), len);
+                }
+            }
+            if (nbits > 0) red_or_shared(at, lo << (32 - nbits));
+        }
+        __syncwarp();
+        // unit u of the forward stream lives at units[n_units - 1 - u]
+        for (uint32_t i = lane; i < span; i += 32) {
+            const unsigned long long u = u0 + i;
+            if (u < n_units) {
+                const uint32_t w = lds32(stage + i * 4);
+                uint32_t* a = p.units + (n_units - 1 - u);
+                if (i == 0 || i + 1 == span) atomicOr(a, w);
+                else *a = w;
+            }
+        }
+        __syncwarp();
     }
-    if (nbits > 0) put_unit(p.units, n_units, u, (uint32_t) (acc << (32 - nbits)), true);
-}
-
-// The flush of the reference encoder (src/ans_encoder.cc:40-66): below the
-// last unit's at = T mod 32 valid bits it adds the high bits of one more
-// code when that code reaches 32 - at bits: the last byte's code again when
-// the last byte's code fitted its unit (at the unit loop's exit it is still
-// the current entry), else the code of byte value 0 (the byte past the end)
-// from the final state.
-__global__ void k_enc_tail(EncParams p) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (*(volatile uint32_t*) p.status & (MANS_DEV_SYNC_OVERFLOW | MANS_DEV_SCAN_TIMEOUT |
-                                          MANS_DEV_COUNT_MISMATCH))
-        return;
-    const EncResult r = *p.result;
-    const uint32_t at = (uint32_t) (r.total_bits & 31);
-    const unsigned long long P = r.total_bits - r.last_len;   // start of the last code
-    uint32_t code, len;
-    if ((uint32_t) (P & 31) + r.last_len < 32) {
-        code = r.last_code;
-        len = r.last_len;
-    } else {
-        const uint32_t dq = __ldg(p.blob + 0), bq = __ldg(p.blob + 1);
-        if (bq == ~0u) return;                              // byte 0 absent: zero entry
-        const uint32_t x = r.first_state;
-        len = (x + dq) >> 16;
-        code = x & ((1u << len) - 1u);
-    }
-    if (at + len >= 32) {
-        const uint32_t spill = at + len - 32;
-        p.units[0] |= code >> spill;                        // forward unit n_units - 1
+    // The flush of the reference encoder (src/ans_encoder.cc:40-66): below
+    // the last unit's at = T mod 32 valid bits it adds the high bits of one
+    // more code when that code reaches 32 - at bits: the last byte's code
+    // again when it fitted its unit (at the unit loop's exit it is still the
+    // current entry), else the code of byte value 0 (the byte past the end)
+    // from the final state.
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint32_t at = (uint32_t) (res.total_bits & 31);
+        const unsigned long long P = res.total_bits - res.last_len;   // start of the last code
+        uint32_t code = res.last_code, len = res.last_len;
+        if ((uint32_t) (P & 31) + len >= 32) {
+            const uint32_t dq = __ldg(p.blob);
+            if (dq == 0) return;                                // byte 0 absent: zero entry
+            len = (res.first_state + dq) >> 16;
+            code = res.first_state & ((1u << len) - 1u);
+        }
+        if (at + len >= 32) atomicOr(p.units, code >> (at + len - 32));   // unit n_units - 1
     }
 }
 
@@ -398,38 +523,85 @@ __global__ void __launch_bounds__(256) k_hist(const uint8_t* __restrict__ sym,
 }
 
 struct EncLayout {
-    size_t status, result, rec_g, rec_w, end_rec, m, delta, Mpre, Dpre, tiles, flags, total;
+    size_t status, result, end, ctr, tile_map, tile_sum, key, zero_end, node, start, total;
 };
 
 size_t al256(size_t x) { return (x + 255) & ~(size_t) 255; }
 
-EncLayout enc_layout(size_t nchunk, size_t nblk, size_t dmax) {
+struct EncPlan {
+    uint32_t Bs, nb, D, nblk, nseed;
+};
+
+EncLayout enc_layout(const EncPlan& e) {
     EncLayout a;
     size_t o = 0;
+    const size_t ntiles = ((size_t) e.nblk + kLatScanTile - 1) / kLatScanTile;
     a.status = o; o += 256;
     a.result = o; o += 256;
-    a.rec_g = o; o += al256(nblk * 8);
-    a.rec_w = o; o += al256(nblk * dmax * 8);
-    a.end_rec = o; o += al256(nchunk * 16);
-    a.m = o; o += al256(nchunk * 8);
-    a.delta = o; o += al256(nchunk * 8);
-    a.Mpre = o; o += al256(nchunk * 8);
-    a.Dpre = o; o += al256(nchunk * 8);
-    const size_t ntiles = (nchunk + kScanTile - 1) / kScanTile;
-    a.tiles = o; o += al256(ntiles * sizeof(ScanTile));
-    a.flags = o; o += al256((ntiles + 1) * 4);
+    a.end = o; o += 256;
+    a.ctr = o; o += 256;
+    a.tile_map = o; o += al256(ntiles * 8);
+    a.tile_sum = o; o += al256(ntiles * 8);
+    a.key = o; o += al256((size_t) e.nblk * e.D * 4);
+    a.zero_end = o;
+    a.node = o; o += al256((size_t) e.nblk * e.D * 4);
+    a.start = o; o += al256((size_t) e.nblk * 8);
     a.total = o;
     return a;
 }
 
-// Chunk length: about 78 k chunks when the stream is long enough, at least
-// 2048 bytes, a multiple of the block.
-uint32_t enc_chunk(unsigned long long n, uint32_t hint) {
-    if (hint) return std::max<uint32_t>(kEncBlock, std::min<uint32_t>(hint, 1u << 30) / kEncBlock * kEncBlock);
-    unsigned long long c = (n + 78000 - 1) / 78000;
-    c = std::max<unsigned long long>(c, 2048);
-    c = std::min<unsigned long long>(c, 1u << 20);
-    return (uint32_t) ((c + kEncBlock - 1) / kEncBlock * kEncBlock);
+// Blocks of 128 bytes (64 on short inputs with small tables, whose encodes
+// meet within a few hundred bytes), and starts every `hint` bytes or as many
+// as run side by side (32 warps on every SM; 64 MB: 16 warps 414 us, 32 371),
+// but no closer than the slots allow: every L / 12 bytes keeps up to 15
+// distinct trajectories under way for the generator's data from 3.8 to 0.07
+// bits per symbol (CPU simulation: L = 4096, 0.67 bits, 16 at 341 bytes).
+// 1 MB at 1.5 bits, L = 4096: every 512 bytes 488 us, every 256 bytes 330.
+EncPlan enc_plan(unsigned long long n, uint32_t L, uint32_t hint) {
+    EncPlan e;
+    e.Bs = n <= kEncSmallBytes && L <= 1024 ? 64 : 128;
+    e.D = kLatSlotsMax;
+    const unsigned long long nblk = (n + e.Bs - 1) / e.Bs;
+    const unsigned long long par = n / (152ull * 32 * 32);
+    unsigned long long s = hint ? hint : std::max<unsigned long long>({par, L / 12, 128});
+    s = std::min<unsigned long long>(std::max<unsigned long long>(s / e.Bs, 1), 1u << 28);
+    e.nb = (uint32_t) s;
+    e.nblk = (uint32_t) std::min<unsigned long long>(nblk, 0xffffffffull);
+    e.nseed = (uint32_t) ((nblk + s - 1) / s);
+    return e;
+}
+
+size_t enc_sync_smem(uint32_t L, uint32_t Bs, uint32_t threads) {
+    return enc_table_bytes(L) + (size_t) threads * enc_pair_bytes(Bs);
+}
+
+size_t enc_final_smem(uint32_t L, uint32_t Bs, uint32_t threads) {
+    uint32_t lg = 0;
+    while ((1u << lg) < L) ++lg;
+    return enc_table_bytes(L) +
+           (size_t) (threads / 32) * (32 * enc_row_bytes(Bs) + enc_stage_words(Bs, lg) * 4);
+}
+
+int enc_sms() {
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+}
+
+// Opts the kernels in to large dynamic shared memory, once per device.
+void enc_attributes() {
+    static std::mutex mu;
+    static uint64_t done = 0;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 64 && ((done >> dev) & 1)) return;
+    cudaFuncSetAttribute(k_enc_sync<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_enc_sync<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_enc_final<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_enc_final<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    if (dev < 64) done |= 1ull << dev;
 }
 
 }  // namespace
@@ -449,10 +621,7 @@ size_t mans_encode_max_units(size_t n, uint32_t L) {
 
 size_t mans_encode_aux_size(size_t n, uint32_t chunk_hint) {
     if (n == 0) return 0;
-    const uint32_t Cs = enc_chunk(n, chunk_hint);
-    const size_t nchunk = (n + Cs - 1) / Cs;
-    const size_t nblk = (n + kEncBlock - 1) / kEncBlock;
-    return enc_layout(nchunk, nblk, kEncSlots).total;
+    return enc_layout(enc_plan(n, 2, chunk_hint)).total;   // the smallest blocks
 }
 
 int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint32_t L,
@@ -461,11 +630,9 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
     if (!d_sym || !d_enc_blob || !d_units || !d_aux || n == 0 || L < 2 || L > 8192 ||
         (L & (L - 1)) != 0 || ((uintptr_t) d_sym & 15) != 0 || ((uintptr_t) d_enc_blob & 3) != 0)
         return MANS_ERR_ARG;
-    const uint32_t Cs = enc_chunk(n, chunk_hint);
-    const size_t nchunk = (n + Cs - 1) / Cs;
-    const size_t nblk = (n + kEncBlock - 1) / kEncBlock;
-    if (nchunk > 0x7fffffffull || nblk > 0x7fffffffull) return MANS_ERR_ARG;
-    const EncLayout lay = enc_layout(nchunk, nblk, kEncSlots);
+    const EncPlan e = enc_plan(n, L, chunk_hint);
+    if ((unsigned long long) e.nblk * e.D > 0xffffffffull) return MANS_ERR_ARG;
+    const EncLayout lay = enc_layout(e);
     if (aux_bytes < lay.total) return MANS_ERR_AUX_SMALL;
     if (cap_units < mans_encode_max_units(n, L)) return MANS_ERR_AUX_SMALL;
     cudaStream_t st = (cudaStream_t) stream;
@@ -476,38 +643,54 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
     p.n = n;
     p.blob = d_enc_blob;
     p.L = L;
-    p.Cs = Cs;
-    p.nb = Cs / kEncBlock;
-    p.nchunk = (uint32_t) nchunk;
-    p.nblk = (uint32_t) nblk;
-    p.dmax = kEncSlots;
-    p.rec_g = (uint2*) (base + lay.rec_g);
-    p.rec_w = (uint2*) (base + lay.rec_w);
-    p.end_rec = (uint4*) (base + lay.end_rec);
-    p.m = (unsigned long long*) (base + lay.m);
-    p.delta = (long long*) (base + lay.delta);
-    p.Mpre = (unsigned long long*) (base + lay.Mpre);
-    p.Dpre = (long long*) (base + lay.Dpre);
-    p.scan_tiles = (ScanTile*) (base + lay.tiles);
-    p.scan_flags = (uint32_t*) (base + lay.flags);
+    p.Bs = e.Bs;
+    p.nb = e.nb;
+    p.D = e.D;
+    p.nblk = e.nblk;
+    p.nseed = e.nseed;
+    p.key = (uint32_t*) (base + lay.key);
+    p.node = (uint32_t*) (base + lay.node);
+    p.start = (unsigned long long*) (base + lay.start);
+    p.tile_map = (unsigned long long*) (base + lay.tile_map);
+    p.tile_sum = (unsigned long long*) (base + lay.tile_sum);
+    p.ctr = (uint32_t*) (base + lay.ctr);
     p.status = (uint32_t*) (base + lay.status);
-    p.nreg = (uint32_t) nchunk;
     p.result = (EncResult*) (base + lay.result);
+    p.end = (EncEnd*) (base + lay.end);
     p.units = d_units;
     p.cap = cap_units;
-    const size_t ntiles = (nchunk + kScanTile - 1) / kScanTile;
-    if (cudaMemsetAsync(base, 0, 512, st) != cudaSuccess ||
-        cudaMemsetAsync(base + lay.flags, 0, (ntiles + 1) * 4, st) != cudaSuccess ||
-        cudaMemsetAsync(d_units, 0, cap_units * 4, st) != cudaSuccess)
-        return MANS_ERR_CUDA;
-    const size_t smem = 256 * sizeof(uint2) + (size_t) L * 2;
-    const unsigned gc = (unsigned) ((nchunk + kEncThreads - 1) / kEncThreads);
-    k_enc_g<<<gc, kEncThreads, smem, st>>>(p);
-    if (nchunk > 1) k_enc_w<<<gc, kEncThreads, smem, st>>>(p);
-    k_enc_scan<<<(unsigned) ntiles, kScanThreads, 0, st>>>(p);
-    k_enc_total<<<1, 32, 0, st>>>(p);
-    k_enc_final<<<(unsigned) ((nblk + kEncThreads - 1) / kEncThreads), kEncThreads, smem, st>>>(p);
-    k_enc_tail<<<1, 32, 0, st>>>(p);
+    enc_attributes();
+    const uint32_t sms = (uint32_t) enc_sms();
+    const size_t words = lay.zero_end / 16 + cap_units / 4;
+    const unsigned gz = (unsigned) std::min<size_t>((words + 1023) / 1024, 4 * sms);
+    k_enc_zero<<<gz, 256, 0, st>>>((uint4*) base, lay.zero_end / 16, d_units, cap_units);
+    {
+        // few trajectories: narrow warps spread over the schedulers of all SMs
+        uint32_t th = kEncThreads;
+        p.width = e.nseed <= 32 * sms ? 8 : (e.nseed <= 64 * sms ? 16 : 32);
+        if (e.nseed <= p.width * 4 * sms) th = 32;
+        const uint32_t per_cta = (th / 32) * p.width;
+        const unsigned grid = std::min<unsigned>((e.nseed + per_cta - 1) / per_cta,
+                                                 sms * kEncCtas * (kEncThreads / th));
+        const size_t sm = enc_sync_smem(L, e.Bs, th);
+        if (e.Bs == 64) k_enc_sync<64><<<grid, th, sm, st>>>(p);
+        else k_enc_sync<128><<<grid, th, sm, st>>>(p);
+    }
+    k_enc_scan<kLatSlotsMax><<<(e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
+                               mans_encode_blob_words(L) * 4, st>>>(p);
+    {
+        const unsigned groups = (e.nblk + 31) / 32;
+        uint32_t th = kEncFinalThreads;
+        while (th > 64 && groups < (th / 32) * 2u * sms) th /= 2;
+        const size_t sm = enc_final_smem(L, e.Bs, th);
+        auto* k = e.Bs == 64 ? k_enc_final<64> : k_enc_final<128>;
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, th, sm) != cudaSuccess ||
+            per_sm < 1)
+            per_sm = 1;
+        const unsigned need = (groups + th / 32 - 1) / (th / 32);
+        k<<<std::min<unsigned>(need, (unsigned) per_sm * sms), th, sm, st>>>(p);
+    }
     return cudaGetLastError() == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }
 
@@ -536,8 +719,8 @@ int mans_encode_sync(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob,
                      uint32_t* d_units, size_t cap_units, void* d_aux, size_t aux_bytes,
                      void* stream, uint64_t* n_units, uint32_t* first_bit,
                      uint32_t* first_state) {
-    // merges that outrun their slots: the same workspace holds 4x longer
-    // chunks (fewer of them), so re-plan until the walks fit
+    // a true path that ran out of slots: starts four times as far apart, in
+    // the same workspace, until one trajectory encodes everything
     uint32_t chunk = 0;
     for (int attempt = 0; attempt < 8; ++attempt) {
         int rc = mans_encode(d_sym, n, d_enc_blob, L, d_units, cap_units, d_aux, aux_bytes, chunk,
@@ -546,9 +729,9 @@ int mans_encode_sync(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob,
         uint32_t dev = 0;
         rc = mans_encode_result(d_aux, stream, n_units, first_bit, first_state, &dev);
         if (rc != MANS_ERR_SYNC) return rc;
-        const uint32_t cur = enc_chunk(n, chunk);
-        if ((uint64_t) cur >= n) return rc;
-        chunk = (uint32_t) std::min<uint64_t>((uint64_t) cur * 4, 1u << 30);
+        const EncPlan e = enc_plan(n, L, chunk);
+        if (e.nseed <= 1) return rc;
+        chunk = (uint32_t) std::min<uint64_t>((uint64_t) e.nb * e.Bs * 4, 1u << 30);
     }
     return MANS_ERR_SYNC;
 }

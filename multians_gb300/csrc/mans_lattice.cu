@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(kLatScanThreads) k_lat_scan(LatParams p) {
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
-    lat_scan_body<kD>(p, s_tile);
+    lat_scan_body<LatParams, kD>(p, s_tile);
 }
 
 template <bool kRev, uint32_t kB>
@@ -214,9 +214,10 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     mark(3, st);
     {
         const unsigned g = (plan.nblk + kLatScanTile - 1) / kLatScanTile;
-        if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, 0, st>>>(p);
-        else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, 0, st>>>(p);
-        else k_lat_scan<12><<<g, kLatScanThreads, 0, st>>>(p);
+        const size_t sm = (size_t) call.L * 4;   // a repair's table
+        if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, sm, st>>>(p);
+        else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, sm, st>>>(p);
+        else k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
     }
     mark(4, st);
     {

@@ -35,6 +35,7 @@
 #include <cstdint>
 
 #include "mans_device.cuh"
+#include "mans_lattice_scan.cuh"
 #include "mans_tma.cuh"
 #include "multians_gb300.h"
 
@@ -47,14 +48,7 @@ namespace mans {
 //   bits  7..0   code length k
 // Half the size of the 8-byte entry: a 4-byte lookup by 32 lanes takes about
 // 3 shared wavefronts against 5, and a CTA's table half the room.
-constexpr uint32_t kLatSlotsMax = 12;
-constexpr uint32_t kLatDead = 15;          // node: no slot at the next block
-constexpr uint32_t kLatKeyUsed = 0x80000000u;
-constexpr uint32_t kLatEntBits = 21;       // entry: bit offset (8), state index (13)
 constexpr uint32_t kLatThreads = 128;      // sync pass
-constexpr uint32_t kLatScanThreads = 256;
-constexpr uint32_t kLatScanPer = 4;        // blocks per thread of the scan
-constexpr uint32_t kLatScanTile = kLatScanThreads * kLatScanPer;
 constexpr uint32_t kLatFinalThreads = 256;
 
 struct LatParams {
@@ -83,13 +77,34 @@ struct LatParams {
     uint32_t stage_cap;             // final-pass staging bytes per warp
     uint32_t flags;
     uint32_t width;                 // lanes of a sync-pass warp that run trajectories
-};
 
-// counters: next start, scan tile ticket, tiles done, longest trajectory
-// (blocks), blocks decoded by all trajectories, ~ the first block where the
-// true path has no slot
-enum : uint32_t {
-    kLatNext = 0, kLatTicket = 1, kLatDone = 2, kLatMaxLife = 3, kLatVisits = 4, kLatDeadBlock = 5
+    // scan hooks (mans_lattice_scan.cuh): an entry is the bit offset from the
+    // block start and the state index << 8, an offset counts symbols
+    __device__ __forceinline__ uint32_t repair_blocks() const {
+        return n_units <= 32768 ? ~0u : 1024u;
+    }
+    __device__ __forceinline__ void finish(uint32_t, unsigned long long) const {}
+    __device__ __forceinline__ void finish_seq(const uint32_t*, uint32_t, unsigned long long) const {}
+    __device__ __forceinline__ void repair_load(uint32_t* sm) const {
+        for (uint32_t j = threadIdx.x; j < L; j += blockDim.x) sm[j] = __ldg(tab_cnt + j);
+    }
+    __device__ __forceinline__ void advance(const uint32_t* sm, uint32_t b, uint32_t& ent,
+                                            unsigned long long& off) const {
+        const unsigned long long bbits = (unsigned long long) B * 32;
+        uint32_t idx = min(ent >> 8, L - 1);
+        unsigned long long pos = b * bbits + (ent & 0xffu);
+        while (pos < (b + 1) * bbits) {
+            const uint32_t e = sm[idx];
+            const unsigned long long u = pos >> 5;
+            const uint32_t w0 = u < n_units ? __ldg(units + u) : 0u;
+            const uint32_t w1 = u + 1 < n_units ? __ldg(units + u + 1) : 0u;
+            const uint32_t bits = __funnelshift_r(w0, w1, (uint32_t) pos & 31u);
+            idx = min((e >> 18) + (bits & ((1u << (e & 31u)) - 1u)), L - 1);
+            pos += e & 31u;
+            off += (e >> 8) & 255u;
+        }
+        ent = (uint32_t) (pos - (b + 1) * bbits) | (idx << 8);
+    }
 };
 
 // ---------------------------------------------------------------------------
@@ -254,56 +269,12 @@ __device__ __forceinline__ void lat_block(LatCursor& c, uint32_t col, uint32_t m
 // ---------------------------------------------------------------------------
 // sync pass
 
-__device__ __forceinline__ uint32_t lat_cas(uint32_t* a, uint32_t v) {
-    uint32_t r;
-    asm volatile("atom.relaxed.gpu.global.cas.b32 %0, [%1], %2, %3;"
-                 : "=r"(r) : "l"(a), "r"(0u), "r"(v) : "memory");
-    return r;
-}
-
-// Loads whose latency a block's decode hides: volatile, so that they are
-// issued where they stand and not where their result is first used.
-__device__ __forceinline__ uint4 lat_ld_slots(const uint32_t* a) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(a));
-    return v;
-}
+// Volatile, so that the load is issued where it stands, a block ahead.
 __device__ __forceinline__ uint4 lat_ld_units(const uint32_t* a) {
     uint4 v;
     asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(a));
     return v;
-}
-
-// Takes or finds the slot of entry `val` among slots [from, D) of a block:
-// the slots as they are now, four at a time, then a compare-and-swap on the
-// first free one.  Returns the slot (kLatDead: none free) and whether a
-// trajectory with that entry was there first.
-__device__ __forceinline__ uint32_t lat_take(uint32_t* __restrict__ key, uint32_t from, uint32_t D,
-                                             uint32_t val, bool& found) {
-    found = false;
-    uint32_t q = from;
-    while (q < D) {
-        const uint32_t g = q & ~3u;
-        const uint4 k = lat_ld_slots(key + g);
-        uint32_t at = g + 4;   // first slot that is free or holds val
-        if (k.w == 0 || k.w == val) at = g + 3;
-        if (g + 2 >= q && (k.z == 0 || k.z == val)) at = g + 2;
-        if (g + 1 >= q && (k.y == 0 || k.y == val)) at = g + 1;
-        if (g >= q && (k.x == 0 || k.x == val)) at = g;
-        if (at < g + 4) {
-            const uint32_t r = lat_cas(key + at, val);
-            if (r == 0) return at;
-            if (r == val) {
-                found = true;
-                return at;
-            }
-            ++at;
-        }
-        q = at;
-    }
-    return kLatDead;
 }
 
 // The units of block b of a lane into `r` (zero past the end).
@@ -482,364 +453,6 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p) {
         atomicMax(p.ctr + kLatMaxLife, max_life);
         atomicAdd(p.ctr + kLatVisits, visits);
     }
-}
-
-// ---------------------------------------------------------------------------
-// scan: the true path's slot at every block, then its output offsets
-
-// A slot map, one byte a slot: byte s = the slot a node in slot s leads to,
-// kLatDead (15, a fixed point) when it leads nowhere; slots from 4 * kW on
-// are fixed points too.
-template <uint32_t kW>
-struct LatMap {
-    uint32_t w[kW];
-};
-
-template <uint32_t kW>
-__device__ __forceinline__ LatMap<kW> lat_identity() {
-    LatMap<kW> m;
-#pragma unroll
-    for (uint32_t i = 0; i < kW; ++i) m.w[i] = 0x03020100u + i * 0x04040404u;
-    return m;
-}
-
-// g after f: byte permutes by f's bytes within the two halves of g's 16
-// entries, then the half by bit 3.
-template <uint32_t kW>
-__device__ __forceinline__ LatMap<kW> lat_compose(const LatMap<kW>& g, const LatMap<kW>& f) {
-    const uint32_t g1 = kW > 1 ? g.w[kW > 1 ? 1 : 0] : 0x07060504u;
-    const uint32_t g2 = kW > 2 ? g.w[kW > 2 ? 2 : 0] : 0x0b0a0908u;
-    LatMap<kW> h;
-#pragma unroll
-    for (uint32_t i = 0; i < kW; ++i) {
-        const uint32_t x = f.w[i], x7 = x & 0x07070707u;
-        const uint32_t sel = __byte_perm((x7 | (x7 >> 4)) & 0x00ff00ffu, 0, 0x4420);
-        const uint32_t lo = __byte_perm(g.w[0], g1, sel), hi = __byte_perm(g2, 0x0f0e0d0cu, sel);
-        const uint32_t up = ((x >> 3) & 0x01010101u) * 0xffu;
-        h.w[i] = (lo & ~up) | (hi & up);
-    }
-    return h;
-}
-
-template <uint32_t kW>
-__device__ __forceinline__ uint32_t lat_apply(const LatMap<kW>& m, uint32_t s) {
-    uint32_t x = s;
-#pragma unroll
-    for (uint32_t i = 0; i < kW; ++i)
-        if ((s >> 2) == i) x = (m.w[i] >> (8 * (s & 3u))) & 15u;
-    return x;
-}
-
-// look-back words: four bits a slot (12 slots), the state in bits 56..59
-// (bits 62..63 of a sum)
-constexpr unsigned long long kLatAgg = 1, kLatInc = 2;
-
-__device__ __forceinline__ unsigned long long lat_ld(const unsigned long long* a) {
-    return *(volatile const unsigned long long*) a;
-}
-
-// A tile of consecutive blocks in the scan: every thread's kLatScanPer
-// blocks, their slot maps, and the composition of the earlier threads' of
-// its warp; s_map holds each warp's whole map.
-template <uint32_t kD>
-struct LatTile {
-    static constexpr uint32_t kW = kD / 4;
-    static constexpr uint32_t kWarps = kLatScanThreads / 32;
-    struct Shared {
-        LatMap<kW> map[kWarps];
-        unsigned long long sum[kWarps];
-        unsigned long long base;
-        uint32_t slot, dead;
-    };
-    LatMap<kW> f[kLatScanPer], exc;
-    uint32_t b0;
-    uint32_t cnt[kLatScanPer], ent[kLatScanPer];
-    unsigned long long sum, run;
-
-    __device__ __forceinline__ void maps(const LatParams& p, Shared& sh, uint32_t first) {
-        const uint32_t t = threadIdx.x, lane = t & 31;
-        b0 = first + t * kLatScanPer;
-        LatMap<kW> inc = lat_identity<kW>();
-#pragma unroll
-        for (uint32_t i = 0; i < kLatScanPer; ++i) {
-            const uint32_t b = b0 + i;
-            f[i] = lat_identity<kW>();
-            if (b + 1 < p.nblk) {
-                const uint4* nd = reinterpret_cast<const uint4*>(p.node + (size_t) b * kD);
-#pragma unroll
-                for (uint32_t s = 0; s < kW; ++s) {
-                    const uint4 v = __ldg(nd + s);   // the top nibbles of four nodes
-                    f[i].w[s] = (__byte_perm(__byte_perm(v.x, v.y, 0x0073),
-                                             __byte_perm(v.z, v.w, 0x7300), 0x7610) >> 4) & 0x0f0f0f0fu;
-                }
-            }
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kLatScanPer; ++i) inc = lat_compose(f[i], inc);
-        // inclusive composition over the warp, earlier threads first
-#pragma unroll
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            LatMap<kW> g;
-#pragma unroll
-            for (uint32_t i = 0; i < kW; ++i) g.w[i] = __shfl_up_sync(0xffffffffu, inc.w[i], o);
-            if (lane >= o) inc = lat_compose(inc, g);
-        }
-        if (lane == 31) sh.map[t >> 5] = inc;
-        exc = lat_identity<kW>();
-#pragma unroll
-        for (uint32_t i = 0; i < kW; ++i) {
-            const uint32_t g = __shfl_up_sync(0xffffffffu, inc.w[i], 1);
-            if (lane > 0) exc.w[i] = g;
-        }
-    }
-
-    // With the slot at the tile's first block in sh.slot: the true slot,
-    // entry and count at every block of the thread, the warps' count sums,
-    // and the first block without a slot (sh.dead, ~0 before).
-    __device__ __forceinline__ void path(const LatParams& p, Shared& sh) {
-        const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        uint32_t s = sh.slot;
-        for (uint32_t w = 0; w < warp; ++w) s = lat_apply(sh.map[w], s);
-        s = lat_apply(exc, s);
-        sum = 0;
-        uint32_t dead = ~0u;
-#pragma unroll
-        for (uint32_t i = 0; i < kLatScanPer; ++i) {
-            const uint32_t b = b0 + i;
-            cnt[i] = ent[i] = 0;
-            if (b < p.nblk) {
-                if (s >= kD) dead = min(dead, b);
-                const size_t at = (size_t) b * kD + min(s, kD - 1);
-                ent[i] = __ldg(p.key + at) & ((1u << kLatEntBits) - 1);
-                if (b + 1 < p.nblk && s < kD) cnt[i] = __ldg(p.node + at) & 0x0fffffffu;
-                s = lat_apply(f[i], s);
-            }
-            sum += cnt[i];
-        }
-        dead = __reduce_min_sync(0xffffffffu, dead);
-        if (lane == 0 && dead != ~0u) atomicMin(&sh.dead, dead);
-        run = sum;
-#pragma unroll
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            const unsigned long long g = __shfl_up_sync(0xffffffffu, run, o);
-            if (lane >= o) run += g;
-        }
-        if (lane == 31) sh.sum[warp] = run;
-    }
-
-    // With the offset of the tile's first block in sh.base.
-    __device__ __forceinline__ void store(const LatParams& p, const Shared& sh) {
-        unsigned long long o = sh.base + run - sum;
-        for (uint32_t w = 0; w < threadIdx.x >> 5; ++w) o += sh.sum[w];
-#pragma unroll
-        for (uint32_t i = 0; i < kLatScanPer; ++i) {
-            if (b0 + i < p.nblk) p.start[b0 + i] = ent[i] | (o << kLatEntBits);
-            o += cnt[i];
-        }
-    }
-};
-
-// The true path goes through a block all of whose slots were taken (more
-// distinct trajectories than slots): from there one thread decodes it block
-// by block until it meets a trajectory that has a slot, and the CTA scans on
-// from that node, tile by tile.  Sequential work, so bounded: past
-// kLatRepairBlocks (any number on a short stream) the decode reports
-// MANS_DEV_SYNC_OVERFLOW.  Run by the last tile to finish.
-constexpr uint32_t kLatRepairBlocks = 4096;
-constexpr uint32_t kLatRepairUnits = 32768;   // short stream
-
-template <uint32_t kD>
-__device__ __noinline__ void lat_repair(const LatParams& p, typename LatTile<kD>::Shared& sh,
-                                        uint32_t dead) {
-    const unsigned long long bbits = (unsigned long long) p.B * 32;
-    uint32_t budget = p.n_units <= kLatRepairUnits ? ~0u : kLatRepairBlocks;
-    __shared__ uint32_t s_b;
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t b = dead - 1;   // its entry and offset are known
-            const volatile unsigned long long* st = p.start;
-            unsigned long long v = st[b];
-            uint32_t idx = (uint32_t) (v >> 8) & (kMaxStates - 1);
-            unsigned long long pos = b * bbits + (v & 255u), off = v >> kLatEntBits;
-            uint32_t slot = kLatDead;
-            while (slot == kLatDead && budget) {
-                while (pos < (b + 1) * bbits) {
-                    const uint32_t e = __ldg(p.tab_cnt + idx);
-                    const unsigned long long u = pos >> 5;
-                    const uint32_t w0 = u < p.n_units ? __ldg(p.units + u) : 0u;
-                    const uint32_t w1 = u + 1 < p.n_units ? __ldg(p.units + u + 1) : 0u;
-                    const uint32_t bits = __funnelshift_r(w0, w1, (uint32_t) pos & 31u);
-                    idx = min((e >> 18) + (bits & ((1u << (e & 31u)) - 1u)), p.L - 1);
-                    pos += e & 31u;
-                    off += (e >> 8) & 255u;
-                }
-                ++b;
-                --budget;
-                if (b >= p.nblk) break;
-                const uint32_t ent = (uint32_t) (pos - b * bbits) | (idx << 8);
-                p.start[b] = ent | (off << kLatEntBits);
-                for (uint32_t q = 0; q < kD; ++q)
-                    if (__ldg(p.key + (size_t) b * kD + q) == (ent | kLatKeyUsed)) slot = q;
-            }
-            s_b = b;
-            sh.slot = slot;
-            sh.base = off;
-            sh.dead = ~0u;
-        }
-        __syncthreads();
-        uint32_t b = s_b;
-        if (b >= p.nblk) break;                       // the stream's end
-        if (sh.slot == kLatDead) return;              // out of budget
-        dead = ~0u;
-        for (; b < p.nblk && dead == ~0u; b += kLatScanTile) {
-            LatTile<kD> tl;
-            tl.maps(p, sh, b);
-            __syncthreads();
-            tl.path(p, sh);
-            __syncthreads();
-            tl.store(p, sh);
-            dead = sh.dead;
-            uint32_t x = sh.slot;
-            unsigned long long base = sh.base;
-            for (uint32_t w = 0; w < LatTile<kD>::kWarps; ++w) {
-                x = lat_apply(sh.map[w], x);
-                base += sh.sum[w];
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                sh.slot = x;
-                sh.base = base;
-            }
-            __syncthreads();
-        }
-        if (dead == ~0u) break;
-    }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAnd(p.status, ~MANS_DEV_SYNC_OVERFLOW);
-    }
-}
-
-template <uint32_t kD>
-__device__ __forceinline__ void lat_scan_body(const LatParams& p, uint32_t tile) {
-    using Tile = LatTile<kD>;
-    constexpr uint32_t kWarps = Tile::kWarps;
-    __shared__ typename Tile::Shared sh;
-    const uint32_t st = *(volatile uint32_t*) p.status;
-    if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_DEGENERATE)) return;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) sh.dead = ~0u;
-    Tile tl;
-    tl.maps(p, sh, tile * kLatScanTile);
-    __syncthreads();
-    // the tile's map (lane s follows slot s), then the slot at its first block
-    if (warp == 0) {
-        uint32_t x = lane & 15u;
-        for (uint32_t w = 0; w < kWarps; ++w) x = lat_apply(sh.map[w], x);
-        uint32_t slot = 0;   // slot at the tile's first block
-        if (tile != 0) {
-            const unsigned long long own = lane < kD ? (unsigned long long) x << (4 * lane) : 0ull;
-            const unsigned long long agg =
-                (unsigned long long) __reduce_or_sync(0xffffffffu, (uint32_t) own) |
-                (unsigned long long) __reduce_or_sync(0xffffffffu, (uint32_t) (own >> 32)) << 32;
-            if (lane == 0) atomicExch(p.tile_map + tile, agg | (kLatAgg << 56));
-            // back over the predecessors, 32 at a time, to the nearest
-            // inclusive slot
-            uint32_t near = lane & 15u;   // where slot `lane` leads over the tiles passed so far
-            int32_t j = (int32_t) tile - 1;
-            uint32_t spins = 0;
-            for (;;) {
-                const int32_t q = j - (int32_t) lane;
-                const unsigned long long v = q >= 0 ? lat_ld(p.tile_map + q) : 0ull;
-                const uint32_t fl = (uint32_t) (v >> 56) & 15u;
-                const uint32_t incl = __ballot_sync(0xffffffffu, q >= 0 && fl == kLatInc);
-                const uint32_t stop = incl ? __ffs(incl) - 1 : 31u;
-                if (__ballot_sync(0xffffffffu, q >= 0 && fl == 0 && lane <= stop)) {
-                    if (++spins > (1u << 22)) {
-                        if (lane == 0) atomicOr(p.status, MANS_DEV_SCAN_TIMEOUT);
-                        break;
-                    }
-                    continue;
-                }
-                // lane s follows slot s (or all the inclusive slot) from the
-                // farthest tile to the nearest
-                uint32_t r = incl ? (uint32_t) __shfl_sync(0xffffffffu, v, stop) & 15u : (lane & 15u);
-                for (int32_t i = (int32_t) stop - (incl ? 1 : 0); i >= 0; --i) {
-                    const unsigned long long m = __shfl_sync(0xffffffffu, v, i);
-                    if (r < kD) r = (uint32_t) (m >> (4 * r)) & 15u;
-                }
-                const uint32_t to = __shfl_sync(0xffffffffu, near, r);
-                if (incl) {
-                    slot = to;
-                    break;
-                }
-                near = to;
-                j -= 32;
-            }
-        }
-        const uint32_t end = __shfl_sync(0xffffffffu, x, slot & 15u);
-        if (lane == 0) {
-            atomicExch(p.tile_map + tile, (unsigned long long) end | (kLatInc << 56));
-            sh.slot = slot;
-        }
-    }
-    __syncthreads();
-    tl.path(p, sh);
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long agg = 0;
-        for (uint32_t w = 0; w < kWarps; ++w) agg += sh.sum[w];
-        unsigned long long pre = 0;
-        if (tile != 0) {
-            if (lane == 0) atomicExch(p.tile_sum + tile, agg | (kLatAgg << 62));
-            int32_t j = (int32_t) tile - 1;
-            uint32_t spins = 0;
-            for (;;) {
-                const int32_t x = j - (int32_t) lane;
-                const unsigned long long v = x >= 0 ? lat_ld(p.tile_sum + x) : 0ull;
-                const uint32_t fl = (uint32_t) (v >> 62);
-                const uint32_t incl = __ballot_sync(0xffffffffu, x >= 0 && fl == kLatInc);
-                const uint32_t stop = incl ? __ffs(incl) - 1 : 31u;
-                if (__ballot_sync(0xffffffffu, x >= 0 && fl == 0 && lane <= stop)) {
-                    if (++spins > (1u << 22)) {
-                        if (lane == 0) atomicOr(p.status, MANS_DEV_SCAN_TIMEOUT);
-                        break;
-                    }
-                    continue;
-                }
-                unsigned long long w = lane <= stop ? v & ~(3ull << 62) : 0ull;
-#pragma unroll
-                for (uint32_t o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-                pre += w;
-                if (incl) break;
-                j -= 32;
-            }
-        }
-        if (lane == 0) {
-            atomicExch(p.tile_sum + tile, (pre + agg) | (kLatInc << 62));
-            sh.base = pre;
-        }
-    }
-    __syncthreads();
-    tl.store(p, sh);
-    if (threadIdx.x == 0 && sh.dead != ~0u) {
-        atomicOr(p.status, MANS_DEV_SYNC_OVERFLOW);
-        atomicMax(p.ctr + kLatDeadBlock, ~sh.dead);
-    }
-    // the last tile repairs a path that ran out of slots
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();   // the CTA's writes, ordered before by the barrier
-        const uint32_t ntiles = (p.nblk + kLatScanTile - 1) / kLatScanTile;
-        sh.slot = atomicAdd(p.ctr + kLatDone, 1u) == ntiles - 1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!sh.slot) return;
-    const uint32_t now = *(volatile uint32_t*) p.status;
-    if ((now & MANS_DEV_SYNC_OVERFLOW) && !(now & MANS_DEV_SCAN_TIMEOUT))
-        lat_repair<kD>(p, sh, ~*(volatile uint32_t*) (p.ctr + kLatDeadBlock));
 }
 
 // ---------------------------------------------------------------------------

@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 LATTICE = 0x80
-DEAD_BLOCK = 256 + 5 * 4   # byte of the workspace counter that a repair sets
+REPAIRED = 256 + 5 * 4   # byte of the workspace counter of repaired blocks
 
 
 def _dev(a):
@@ -34,7 +34,7 @@ def _decode(mg, st, n_out=None, shift=0, source_order=False):
                  st.first_state, st.first_bit, aux, plan)
     status = aux_status(aux)
     assert status & ~mg.DEV_DEGENERATE == 0, hex(status)
-    repaired = bool(aux[DEAD_BLOCK: DEAD_BLOCK + 4].cpu().numpy().any())
+    repaired = bool(aux[REPAIRED: REPAIRED + 4].cpu().numpy().any())
     b = big.cpu().numpy()
     assert (b[:shift] == 0xCD).all() and (b[shift + n_out:] == 0xCD).all()
     return b[shift: shift + n_out], repaired
