@@ -1909,6 +1909,7 @@ __device__ __forceinline__ void load_params(DecodeParams& dst, const DecodeParam
 __global__ void k_prep_batch(const DecodeParams* ps) {
     __shared__ DecodeParams sp;
     load_params(sp, ps + blockIdx.x);
+    if (sp.nreg == 0) return;   // no output, or a lattice decode
     prep_body(sp);
 }
 
@@ -2984,7 +2985,12 @@ int mans_decode_loop(const mans_stream_desc* streams, uint32_t n, const mans_cfg
 
 // ---------------------------------------------------------------------------
 // Batched decode of many independent streams (one launch of each kernel for
-// the whole batch; see the BatchItem kernels above).
+// the whole batch).  Streams that neither capture nor fix a geometry go
+// through the lattice kernels (mans_lattice.cu), the others through the
+// BatchItem kernels above.  Measured, regions and walks -> lattice: 256
+// streams of 4 KB to 4 MB, L = 1024 1922 -> 932 us; 1024 of them 3555 -> 2296;
+// 48 streams of 1 to 256 KB, L = 1024 and 4096, in one call 2690 -> 770; 64
+// requests up to 8 MB through the serving loop 4621 -> 1770.
 
 }  // extern "C"
 
@@ -2997,10 +3003,22 @@ struct BatchStreamPlan {
     size_t flags_off;    // word offset of its scan flags in the flag array
     uint32_t stage_cap;
     bool active;
+    bool lattice;        // decoded by the lattice kernels (mans_lattice.h)
+    int lat_class;
+    LatPlan lat;
 };
+
+constexpr size_t kLatFinalSmall = 74 * 1024;   // final-pass CTAs of which three fit an SM
 
 struct BatchLayout {
     size_t status, flags, ticket, params, items, data, total;
+    // lattice streams: their parameters and work items (tables and zeroing,
+    // starts, scan tiles, final CTAs by class: those that leave three on an
+    // SM, and larger ones)
+    size_t lat_params, lat_items, n_lat, n_lprep, n_lsync, n_lscan, n_lfinal_c[2];
+    LatSmem lat_smem;         // of the streams that need most
+    size_t lat_final_smem0;   // ... final pass, class 0
+    uint32_t lat_width;   // lanes of a sync-pass warp that run trajectories
     size_t n_sync, n_walk, n_scan, n_final, n_items;
     bool any_capture;
     size_t smem_sync, smem_walk, smem_final, smem_prep;
@@ -3014,11 +3032,17 @@ struct BatchLayout {
 
 static size_t stream_data_bytes(const BatchStreamPlan& sp) {
     const AuxLayout a = layout_for(sp.nblk, sp.nreg, sp.cfg.walk_slots, sp.cfg.capture_bytes, false);
-    return a.total;
+    return sp.lattice ? std::max(a.total, sp.lat.bytes) : a.total;
+}
+
+static LatCall lat_call(const mans_stream_desc& d) {
+    return {d.d_units, d.n_units, d.d_out, d.n_out, d.d_table, d.L, d.first_state - d.L,
+            start_pos(d.first_bit, d.flags), d.flags & MANS_DECODE_SOURCE_ORDER};
 }
 
 
 constexpr uint64_t kBatchRegionMax = 8192;   // units
+constexpr double kBatchLanes = 152.0 * 16 * 32;   // trajectories of a lattice batch side by side
 
 static int batch_class(uint32_t L) { return L <= 1024 ? 0 : 1; }
 
@@ -3039,6 +3063,16 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
     // cross a whole region.
     double batch_sym = 0;
     for (uint32_t i = 0; i < n; ++i) batch_sym += (double) d[i].n_out;
+    lay.n_lat = lay.n_lprep = lay.n_lsync = lay.n_lscan = 0;
+    lay.n_lfinal_c[0] = lay.n_lfinal_c[1] = lay.lat_final_smem0 = 0;
+    lay.lat_smem = LatSmem{};
+    // a hint that fixes the geometry, capture or seeds keeps the streams on
+    // the region kernels
+    const bool free_hint =
+        !hint || (hint->block_units == 0 && hint->region_blocks == 0 && hint->walk_slots == 0 &&
+                  hint->capture_bytes == 0 &&
+                  !(hint->flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS |
+                                   MANS_DECODE_NO_CAPTURE | MANS_DECODE_CAPTURE)));
     const double sym_per_lane = batch_sym / (152.0 * 16 * 32);
     for (uint32_t i = 0; i < n; ++i) {
         BatchStreamPlan& sp = plans[i];
@@ -3059,6 +3093,17 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         h.flags |= MANS_PLAN_MODEL;
         int rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &sp.cfg);
         if (rc != MANS_OK) return rc;
+        if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE) && sp.cfg.capture_bytes == 0) {
+            // as many starts as its share of the batch's symbols has of the
+            // lanes side by side, in the workspace the stream's own plan has
+            const size_t nblk = num_blocks(d[i].n_units, sp.cfg.block_units);
+            const size_t nreg = (nblk + sp.cfg.region_blocks - 1) / sp.cfg.region_blocks;
+            const double bps = 32.0 * (double) d[i].n_units / (double) d[i].n_out;
+            sp.lattice = lat_plan(
+                d[i].n_units, d[i].n_out, d[i].L, mean_meeting_units(d[i].L, bps),
+                (uint32_t) std::max(1.0, kBatchLanes * (double) d[i].n_out / batch_sym),
+                layout_for(nblk, nreg, sp.cfg.walk_slots, 0, false).total, &sp.lat);
+        }
         if (h.region_blocks == 0) {
             const double spu = (double) d[i].n_out / (double) d[i].n_units;
             const uint64_t B = sp.cfg.block_units;
@@ -3089,6 +3134,21 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         sp.stage_cap = stage_cap_for((double) d[i].n_out / (double) d[i].n_units,
                                      sp.cfg.block_units, d[i].L, kFinalThreads / 32);
         const int cls = batch_class(d[i].L);
+        if (sp.lattice) {
+            ++lay.n_lat;
+            lay.n_lprep += lat_prep_items(sp.lat);
+            lay.n_lscan += lat_scan_tiles(sp.lat);
+            const LatSmem s = lat_batch_smem(lat_call(d[i]), sp.lat);
+            LatSmem& m = lay.lat_smem;
+            sp.lat_class = s.final <= kLatFinalSmall ? 0 : 1;
+            lay.n_lfinal_c[sp.lat_class] += lat_final_ctas(sp.lat);
+            if (sp.lat_class == 0) lay.lat_final_smem0 = std::max(lay.lat_final_smem0, s.final);
+            m.prep = std::max(m.prep, s.prep);
+            m.sync = std::max(m.sync, s.sync);
+            m.scan = std::max(m.scan, s.scan);
+            m.final = std::max(m.final, s.final);
+            continue;
+        }
         lay.n_sync += (sp.nreg + kSyncThreads - 1) / kSyncThreads;
         lay.n_sync_c[cls] += (sp.nreg + kSyncThreads - 1) / kSyncThreads;
         lay.n_walk += walk_ctas(sp.nreg);
@@ -3110,6 +3170,18 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         lay.smem_prep = std::max(lay.smem_prep, (size_t) d[i].L * 12);
     }
     lay.n_items = lay.n_sync + lay.n_scan + lay.n_final;   // merge walks: built on the device
+    // starts a CTA takes: 32 a warp, or fewer (narrow warps, whose steps are
+    // shorter) while they fit the schedulers of all SMs
+    uint64_t seeds = 0;
+    for (const BatchStreamPlan& sp : plans)
+        if (sp.active && sp.lattice) seeds += sp.lat.nseed;
+    lay.lat_width = seeds <= 8ull * 4 * 152 ? 8 : (seeds <= 16ull * 4 * 152 ? 16 : 32);
+    const uint32_t per_cta = kLatBatchWarps * lay.lat_width;
+    for (uint32_t i = 0; i < n; ++i)
+        if (plans[i].active && plans[i].lattice)
+            lay.n_lsync += (plans[i].lat.nseed + per_cta - 1) / per_cta;
+    const size_t lat_items = lay.n_lprep + lay.n_lsync + lay.n_lscan +
+                             lay.n_lfinal_c[0] + lay.n_lfinal_c[1];
     size_t o = 0;
     lay.status = o; o += align256((size_t) n * 4);
     lay.flags = o; o += align256(flag_words * 4);
@@ -3117,6 +3189,8 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
     lay.params = o; o += align256((size_t) n * sizeof(DecodeParams));
     lay.items = o; o += align256(lay.n_items * sizeof(BatchItem));
     lay.walk_list = o; o += align256(lay.n_walk * 4);
+    lay.lat_params = o; o += align256(lay.n_lat ? (size_t) n * lat_params_size() : 0);
+    lay.lat_items = o; o += align256(lat_items * sizeof(LatItem));
     lay.data = o; o += data;
     lay.total = o;
     return MANS_OK;
@@ -3136,6 +3210,8 @@ struct mans_batch {
     // an asynchronous upload never reads freed memory
     std::vector<mans::DecodeParams> ps;
     std::vector<mans::BatchItem> items;
+    std::vector<char> lat_ps;
+    std::vector<mans::LatItem> lat_items;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t graph_stream = nullptr;
@@ -3179,6 +3255,46 @@ int mans_batch_header_size(const mans_stream_desc* streams, uint32_t n, const ma
 
 namespace {
 
+// Work items of the lattice streams, in the order lat_items holds them:
+// tables and zeroing, starts, scan tiles, final CTAs (class 0, class 1).  Starts of the streams that take longest to meet come
+// first (their trajectories are the longest chains), final CTAs of the
+// largest streams.
+void lattice_items(mans_batch* b, const mans_stream_desc* streams) {
+    using namespace mans;
+    std::vector<LatItem>& v = b->lat_items;
+    v.clear();
+    std::vector<uint32_t> order;
+    for (uint32_t i = 0; i < b->n; ++i)
+        if (b->plans[i].active && b->plans[i].lattice) order.push_back(i);
+    for (const uint32_t i : order) {
+        const uint32_t k = lat_prep_items(b->plans[i].lat);
+        for (uint32_t c = 0; c < k; ++c) v.push_back({i, c, k, 0});
+    }
+    const auto meet_steps = [&](uint32_t i) {
+        const double spu = (double) streams[i].n_out / (double) streams[i].n_units;
+        return mean_meeting_units(streams[i].L, 32.0 / spu) * spu;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+        return meet_steps(x) > meet_steps(y);
+    });
+    const uint32_t per_cta = kLatBatchWarps * b->lay.lat_width;
+    for (const uint32_t i : order) {
+        const uint32_t nseed = b->plans[i].lat.nseed;
+        for (uint32_t s = 0; s < nseed; s += per_cta)
+            v.push_back({i, s, std::min(s + per_cta, nseed), 0});
+    }
+    for (const uint32_t i : order)
+        for (uint32_t c = 0; c < lat_scan_tiles(b->plans[i].lat); ++c) v.push_back({i, c, 0, 0});
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+        const int cx = b->plans[x].lat_class, cy = b->plans[y].lat_class;
+        return cx != cy ? cx < cy : streams[x].n_out > streams[y].n_out;
+    });
+    for (const uint32_t i : order) {
+        const uint32_t k = lat_final_ctas(b->plans[i].lat);
+        for (uint32_t c = 0; c < k; ++c) v.push_back({i, c, k, 0});
+    }
+}
+
 // Plans the batch, places each stream's data slice (inside the workspace
 // after the header, or at slices[i]) and uploads the parameters and work
 // items: synchronously when `async` is false, else on `upload` with the
@@ -3205,6 +3321,7 @@ int batch_create(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hi
     b->slice.assign(n, nullptr);
     b->ps.assign(n, DecodeParams{});
     b->items.assign(b->lay.n_items, BatchItem{});
+    if (b->lay.n_lat) b->lat_ps.assign((size_t) n * lat_params_size(), 0);
     size_t is = 0, ic = b->lay.n_sync, iff = ic + b->lay.n_scan;
     for (uint32_t i = 0; i < n; ++i) {
         const BatchStreamPlan& sp = b->plans[i];
@@ -3236,6 +3353,11 @@ int batch_create(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hi
         p.L = d.L;
         p.first_idx = d.first_state - d.L;
         p.first_pos = start_pos(d.first_bit, d.flags);
+        if (sp.lattice) {   // nreg 0: the region kernels leave it alone
+            lat_fill_params(b->lat_ps.data() + (size_t) i * lat_params_size(), lat_call(d), sp.lat,
+                            slice, p.status, b->lay.lat_width);
+            continue;
+        }
         p.B = sp.cfg.block_units;
         p.nb = sp.cfg.region_blocks;
         p.dmax = sp.cfg.walk_slots;
@@ -3256,7 +3378,7 @@ int batch_create(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hi
     // late long CTA setting the launch's end (longest-processing-time order)
     std::vector<uint32_t> order;
     for (uint32_t i = 0; i < n; ++i)
-        if (b->plans[i].active) order.push_back(i);
+        if (b->plans[i].active && !b->plans[i].lattice) order.push_back(i);
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
         const int cx = batch_class(streams[x].L), cy = batch_class(streams[y].L);
         if (cx != cy) return cx < cy;   // one launch per table class
@@ -3275,24 +3397,35 @@ int batch_create(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hi
         const uint32_t nctas = (uint32_t) ((b->plans[i].nblk + kFinalThreads - 1) / kFinalThreads);
         for (uint32_t c = 0; c < nctas; ++c) b->items[iff++] = {i, c, nctas, 0};
     }
+    lattice_items(b, streams);
     const size_t pbytes = n * sizeof(DecodeParams), ibytes = b->items.size() * sizeof(BatchItem);
+    const size_t lpbytes = b->lat_ps.size(), libytes = b->lat_items.size() * sizeof(LatItem);
     bool ok;
     if (async) {
         ok = cudaMemcpyAsync(b->base + b->lay.params, b->ps.data(), pbytes,
                              cudaMemcpyHostToDevice, upload) == cudaSuccess &&
              (!ibytes || cudaMemcpyAsync(b->base + b->lay.items, b->items.data(), ibytes,
-                                         cudaMemcpyHostToDevice, upload) == cudaSuccess);
+                                         cudaMemcpyHostToDevice, upload) == cudaSuccess) &&
+             (!lpbytes || cudaMemcpyAsync(b->base + b->lay.lat_params, b->lat_ps.data(), lpbytes,
+                                          cudaMemcpyHostToDevice, upload) == cudaSuccess) &&
+             (!libytes || cudaMemcpyAsync(b->base + b->lay.lat_items, b->lat_items.data(), libytes,
+                                          cudaMemcpyHostToDevice, upload) == cudaSuccess);
     } else {
         ok = cudaMemcpy(b->base + b->lay.params, b->ps.data(), pbytes, cudaMemcpyHostToDevice) ==
                  cudaSuccess &&
              (!ibytes || cudaMemcpy(b->base + b->lay.items, b->items.data(), ibytes,
-                                    cudaMemcpyHostToDevice) == cudaSuccess);
+                                    cudaMemcpyHostToDevice) == cudaSuccess) &&
+             (!lpbytes || cudaMemcpy(b->base + b->lay.lat_params, b->lat_ps.data(), lpbytes,
+                                     cudaMemcpyHostToDevice) == cudaSuccess) &&
+             (!libytes || cudaMemcpy(b->base + b->lay.lat_items, b->lat_items.data(), libytes,
+                                     cudaMemcpyHostToDevice) == cudaSuccess);
     }
     if (!ok) {
         mans_batch_destroy(b);
         return MANS_ERR_CUDA;
     }
     set_kernel_attributes();
+    if (b->lay.n_lat) lat_batch_init();
     if (b->lay.n_walk) {
         // the persistent merge-walk grid: as many CTAs as stay resident
         int per_sm = 0, sms = 0;
@@ -3333,19 +3466,27 @@ int mans_batch_decode(mans_batch* b, void* stream) {
     cudaStream_t st = (cudaStream_t) stream;
     const BatchLayout& L = b->lay;
     if (cudaMemsetAsync(b->base, 0, L.params, st) != cudaSuccess) return MANS_ERR_CUDA;
-    if (L.n_items == 0) return MANS_OK;
+    if (L.n_items == 0 && L.n_lat == 0) return MANS_OK;
     const DecodeParams* ps = (const DecodeParams*) (b->base + L.params);
     const BatchItem* items = (const BatchItem*) (b->base + L.items);
+    const void* lps = b->base + L.lat_params;
+    const LatItem* litems = (const LatItem*) (b->base + L.lat_items);
+    const bool regions = L.n_items != 0;
     timing_mark(0, st);
-    k_prep_batch<<<b->n, 1024, L.smem_prep, st>>>(ps);
+    if (regions) k_prep_batch<<<b->n, 1024, L.smem_prep, st>>>(ps);
+    lat_batch_prep(lps, litems, L.n_lprep, L.lat_smem, st);
+    litems += L.n_lprep;
     timing_mark(1, st);
     for (int c = 0, at = 0; c < 2; at += (int) L.n_sync_c[c], ++c)
         if (L.n_sync_c[c])
             k_gwalk_batch<<<(unsigned) L.n_sync_c[c], kSyncThreads, L.smem_sync_c[c], st>>>(
                 ps, items + at);
+    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, st);
+    litems += L.n_lsync;
     timing_mark(2, st);
     if (L.n_walk) {
-        // ticket words: 0 scan tiles, 1 merge-walk items, 2 next item
+        // ticket words: 0 scan tiles, 1 merge-walk items, 2 next item, 3
+        // lattice scan tiles
         uint32_t* const count = (uint32_t*) (b->base + L.ticket) + 1;
         uint32_t* const list = (uint32_t*) (b->base + L.walk_list);
         k_walk_items<<<(b->n + 255) / 256, 256, 0, st>>>(ps, b->n, list, count);
@@ -3355,6 +3496,8 @@ int mans_batch_decode(mans_batch* b, void* stream) {
     if (L.n_scan)
         k_scan_batch<<<(unsigned) L.n_scan, kScanThreads, 0, st>>>(
             ps, items + L.n_sync, (uint32_t*) (b->base + L.ticket));
+    lat_batch_scan(lps, litems, L.n_lscan, L.lat_smem, (uint32_t*) (b->base + L.ticket) + 3, st);
+    litems += L.n_lscan;
     timing_mark(4, st);
     if (L.n_final && L.any_capture)
         k_copy_batch<<<(unsigned) L.n_final, kCopyThreads, 0, st>>>(
@@ -3363,9 +3506,12 @@ int mans_batch_decode(mans_batch* b, void* stream) {
         if (L.n_final_c[c])
             k_final_batch<<<(unsigned) L.n_final_c[c], kFinalThreads, L.smem_final_c[c], st>>>(
                 ps, items + L.n_sync + L.n_scan + at);
+    lat_batch_final(lps, litems, L.n_lfinal_c[0], L.lat_final_smem0, st);
+    lat_batch_final(lps, litems + L.n_lfinal_c[0], L.n_lfinal_c[1], L.lat_smem.final, st);
     timing_mark(5, st);
     if (g_timing.on && g_timing.used < g_timing.cap) ++g_timing.used;
-    g_last_launches = 1 + (L.n_sync_c[0] ? 1 : 0) + (L.n_sync_c[1] ? 1 : 0) +
+    g_last_launches = (regions ? 1 : 0) + (L.n_lat ? 3 : 0) + (L.n_lfinal_c[0] ? 1 : 0) +
+                      (L.n_lfinal_c[1] ? 1 : 0) + (L.n_sync_c[0] ? 1 : 0) + (L.n_sync_c[1] ? 1 : 0) +
                       (L.n_walk ? 2 : 0) + (L.n_scan ? 1 : 0) + (L.n_final_c[0] ? 1 : 0) +
                       (L.n_final_c[1] ? 1 : 0) + (L.n_final && L.any_capture ? 1 : 0);
     return cudaGetLastError() == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;

@@ -94,8 +94,9 @@ struct EncParams {
     __device__ __forceinline__ void finish(uint32_t slot, unsigned long long off) const {
         set_result(end[slot], off);
     }
+    __device__ __forceinline__ uint32_t repair_words() const { return 512 + (L + 1) / 2; }
     __device__ __forceinline__ void repair_load(uint32_t* sm) const {
-        for (uint32_t i = threadIdx.x; i < 512 + (L + 1) / 2; i += blockDim.x) sm[i] = __ldg(blob + i);
+        for (uint32_t i = threadIdx.x; i < repair_words(); i += blockDim.x) sm[i] = __ldg(blob + i);
     }
     // one block, by one thread
     __device__ __forceinline__ EncEnd block(const uint32_t* sm, uint32_t b, uint32_t ent) const {
@@ -677,7 +678,7 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
         else k_enc_sync<128><<<grid, th, sm, st>>>(p);
     }
     k_enc_scan<kLatSlotsMax><<<(e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
-                               mans_encode_blob_words(L) * 4, st>>>(p);
+                               lat_scan_smem(mans_encode_blob_words(L)), st>>>(p);
     {
         const unsigned groups = (e.nblk + 31) / 32;
         uint32_t th = kEncFinalThreads;

@@ -10,8 +10,11 @@
 namespace mans {
 namespace {
 
+constexpr uint32_t kLatPrepThreads = 1024;
+constexpr size_t kLatZeroBytes = 128 * 1024;   // zeroed by a CTA
+
 // Tables (first CTA) and the zeroed words: counters, look-back words, slots.
-__global__ void __launch_bounds__(1024) k_lat_prep(LatParams p, uint4* zero, size_t n16) {
+__global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep(LatParams p, uint4* zero, size_t n16) {
     if (blockIdx.x == 0) lat_tables(p);
     const size_t stride = (size_t) gridDim.x * blockDim.x;
     for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride)
@@ -20,7 +23,7 @@ __global__ void __launch_bounds__(1024) k_lat_prep(LatParams p, uint4* zero, siz
 
 template <uint32_t kB>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
-    lat_sync_body<kB>(p);
+    lat_sync_body<kB>(p, p.ctr + kLatNext, p.nseed);
 }
 
 template <uint32_t kD>
@@ -35,6 +38,84 @@ template <bool kRev, uint32_t kB>
 __global__ void __launch_bounds__(kLatFinalThreads) k_lat_final(LatParams p) {
     lat_final_body<kRev, kB>(p, blockIdx.x, gridDim.x);
 }
+
+// ---------------------------------------------------------------------------
+// Batches: every CTA takes one work item {stream, index, count} of a
+// host-built list and its stream's parameters.
+
+__device__ __forceinline__ void lat_load_params(LatParams& dst, const LatParams* src) {
+    static_assert(sizeof(LatParams) % 4 == 0, "word copy");
+    const uint32_t* s = reinterpret_cast<const uint32_t*>(src);
+    uint32_t* d = reinterpret_cast<uint32_t*>(&dst);
+    for (uint32_t i = threadIdx.x; i < sizeof(LatParams) / 4; i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+}
+
+// index 0 builds the stream's tables; the others zero a share of its words
+// from the counters to the end of the slots.
+__global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep_batch(const LatParams* ps,
+                                                                    const LatItem* items) {
+    __shared__ LatParams sp;
+    const LatItem it = items[blockIdx.x];
+    lat_load_params(sp, ps + it.stream);
+    if (it.index == 0) {
+        lat_tables(sp);
+        return;
+    }
+    uint4* z = reinterpret_cast<uint4*>(sp.ctr);
+    const size_t n16 = ((char*) sp.tab_cnt - (char*) sp.ctr) / 16;
+    const size_t stride = (size_t) (it.count - 1) * blockDim.x;
+    for (size_t i = (size_t) (it.index - 1) * blockDim.x + threadIdx.x; i < n16; i += stride)
+        z[i] = make_uint4(0, 0, 0, 0);
+}
+
+// index: the CTA's first start, count: the end of its starts.
+__global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams* ps,
+                                                                const LatItem* items) {
+    __shared__ LatParams sp;
+    __shared__ uint32_t s_next;
+    const LatItem it = items[blockIdx.x];
+    if (threadIdx.x == 0) s_next = it.index;
+    lat_load_params(sp, ps + it.stream);
+    if (sp.B == 4) lat_sync_body<4>(sp, &s_next, it.count);
+    else if (sp.B == 8) lat_sync_body<8>(sp, &s_next, it.count);
+    else lat_sync_body<16>(sp, &s_next, it.count);
+}
+
+// The ticket hands items out in list order, which holds each stream's tiles
+// in increasing order: a tile only waits on tiles that have started.
+__global__ void __launch_bounds__(kLatScanThreads) k_lat_scan_batch(const LatParams* ps,
+                                                                    const LatItem* items,
+                                                                    uint32_t* ticket) {
+    __shared__ LatParams sp;
+    __shared__ uint32_t s_item;
+    if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const LatItem it = items[s_item];
+    lat_load_params(sp, ps + it.stream);
+    if (sp.D == 4) lat_scan_body<LatParams, 4>(sp, it.index);
+    else if (sp.D == 8) lat_scan_body<LatParams, 8>(sp, it.index);
+    else lat_scan_body<LatParams, 12>(sp, it.index);
+}
+
+template <bool kRev>
+__device__ __forceinline__ void lat_final_any(const LatParams& p, const LatItem& it) {
+    if (p.B == 4) lat_final_body<kRev, 4>(p, it.index, it.count);
+    else if (p.B == 8) lat_final_body<kRev, 8>(p, it.index, it.count);
+    else lat_final_body<kRev, 16>(p, it.index, it.count);
+}
+
+// index: the CTA of the stream's count.
+__global__ void __launch_bounds__(kLatFinalThreads) k_lat_final_batch(const LatParams* ps,
+                                                                      const LatItem* items) {
+    __shared__ LatParams sp;
+    const LatItem it = items[blockIdx.x];
+    lat_load_params(sp, ps + it.stream);
+    if (sp.flags & MANS_DECODE_SOURCE_ORDER) lat_final_any<true>(sp, it);
+    else lat_final_any<false>(sp, it);
+}
+
+static_assert(kLatThreads == 32 * kLatBatchWarps, "batch items");
 
 // CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps, near
 // the rate its shared-memory lookups allow.
@@ -103,7 +184,7 @@ void lat_attributes() {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int) kLatFinalSmemMax);
     };
-    set(k_lat_prep);
+    set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_sync_batch); set(k_lat_final_batch);
     set(k_lat_sync<4>); set(k_lat_sync<8>); set(k_lat_sync<16>);
     set(k_lat_final<false, 4>); set(k_lat_final<false, 8>); set(k_lat_final<false, 16>);
     set(k_lat_final<true, 4>); set(k_lat_final<true, 8>); set(k_lat_final<true, 16>);
@@ -175,6 +256,7 @@ bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t la
             out->D = D;
             out->nblk = (uint32_t) nblk;
             out->nseed = (uint32_t) ((nblk + out->nb - 1) / out->nb);
+            out->L = L;
             out->bytes = need;
             return true;
         }
@@ -191,8 +273,9 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     const int sms = sm_count();
     const size_t n16 = (a.zero_end - a.ctr) / 16;
     mark(0, st);
-    const unsigned gz = 1 + (unsigned) std::min<size_t>((n16 + 8191) / 8192, 2 * sms - 1);
-    k_lat_prep<<<gz, 1024, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
+    const unsigned gz = 1 + (unsigned) std::min<size_t>((n16 * 16 + kLatZeroBytes - 1) / kLatZeroBytes,
+                                                        2 * sms - 1);
+    k_lat_prep<<<gz, kLatPrepThreads, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
     mark(1, st);
     // sync pass
     {
@@ -214,7 +297,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     mark(3, st);
     {
         const unsigned g = (plan.nblk + kLatScanTile - 1) / kLatScanTile;
-        const size_t sm = (size_t) call.L * 4;   // a repair's table
+        const size_t sm = lat_scan_smem(call.L);
         if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, sm, st>>>(p);
         else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, sm, st>>>(p);
         else k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
@@ -249,6 +332,61 @@ bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t st, uint64_t
     *visits = c[kLatVisits];
     *longest = c[kLatMaxLife];
     return true;
+}
+
+size_t lat_params_size() { return sizeof(LatParams); }
+
+void lat_fill_params(void* dst, const LatCall& call, const LatPlan& plan, void* slice,
+                     uint32_t* d_status, uint32_t width) {
+    LatParams p = lat_params(call, plan, (char*) slice);
+    p.status = d_status;
+    p.width = width;
+    *(LatParams*) dst = p;
+}
+
+uint32_t lat_prep_items(const LatPlan& plan) {
+    const LatLayout a = lat_layout(plan.nblk, plan.D, plan.L);
+    return 1 + (uint32_t) ((a.zero_end - a.ctr + kLatZeroBytes - 1) / kLatZeroBytes);
+}
+
+uint32_t lat_scan_tiles(const LatPlan& plan) {
+    return (plan.nblk + kLatScanTile - 1) / kLatScanTile;
+}
+
+uint32_t lat_final_ctas(const LatPlan& plan) {
+    return (plan.nblk + kLatFinalThreads - 1) / kLatFinalThreads;
+}
+
+LatSmem lat_batch_smem(const LatCall& call, const LatPlan& plan) {
+    LatSmem s;
+    s.prep = (size_t) call.L * 12;
+    s.sync = lat_sync_smem(call.L, plan.B, kLatThreads);
+    s.scan = lat_scan_smem(call.L);
+    s.final = lat_final_smem(
+        call.L, plan.B, lat_stage_cap((double) call.n_out / (double) call.n_units, plan.B, call.L),
+        kLatFinalThreads);
+    return s;
+}
+
+void lat_batch_init() { lat_attributes(); }
+
+void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    cudaStream_t st) {
+    if (n) k_lat_prep_batch<<<(unsigned) n, kLatPrepThreads, sm.prep, st>>>((const LatParams*) ps, items);
+}
+void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    cudaStream_t st) {
+    if (n) k_lat_sync_batch<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
+}
+void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    uint32_t* ticket, cudaStream_t st) {
+    if (n)
+        k_lat_scan_batch<<<(unsigned) n, kLatScanThreads, sm.scan, st>>>((const LatParams*) ps,
+                                                                         items, ticket);
+}
+void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st) {
+    if (n)
+        k_lat_final_batch<<<(unsigned) n, kLatFinalThreads, smem, st>>>((const LatParams*) ps, items);
 }
 
 }  // namespace mans

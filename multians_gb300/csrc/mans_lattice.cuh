@@ -85,6 +85,7 @@ struct LatParams {
     }
     __device__ __forceinline__ void finish(uint32_t, unsigned long long) const {}
     __device__ __forceinline__ void finish_seq(const uint32_t*, uint32_t, unsigned long long) const {}
+    __device__ __forceinline__ uint32_t repair_words() const { return L; }
     __device__ __forceinline__ void repair_load(uint32_t* sm) const {
         for (uint32_t j = threadIdx.x; j < L; j += blockDim.x) sm[j] = __ldg(tab_cnt + j);
     }
@@ -321,8 +322,9 @@ __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B
 // one after it are loaded, and a slot is claimed, a block's decode before
 // they are needed, which hides their round trips (about 1500 cycles a block
 // when they were waited for).
+// Starts are taken from the counter `next`, up to `limit`.
 template <uint32_t kB>
-__device__ __forceinline__ void lat_sync_body(const LatParams& p) {
+__device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next, uint32_t limit) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     const uint32_t st = *(volatile uint32_t*) p.status;
     if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_DEGENERATE)) return;
@@ -351,11 +353,11 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p) {
         const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
         if (!exhausted && __popc(idle) >= min(p.width, 8u)) {
             uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(p.ctr + kLatNext, (uint32_t) __popc(idle));
+            if (lane == 0) base = atomicAdd(next, (uint32_t) __popc(idle));
             base = __shfl_sync(0xffffffffu, base, 0);
-            exhausted = base + __popc(idle) >= p.nseed;
+            exhausted = base + __popc(idle) >= limit;
             const uint32_t k = base + __popc(idle & ((1u << lane) - 1));
-            if (!on && lane < p.width && k < p.nseed) {
+            if (!on && lane < p.width && k < limit) {
                 on = true;
                 b = k * p.nb;
                 first = k == 0;

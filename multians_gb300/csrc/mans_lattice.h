@@ -14,6 +14,7 @@ struct LatPlan {
     uint32_t D;       // slots per block
     uint32_t nblk;
     uint32_t nseed;
+    uint32_t L;
     size_t bytes;     // workspace
 };
 
@@ -43,5 +44,34 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
 // the stream): blocks decoded by all of them, blocks of the longest.
 bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t stream, uint64_t* visits,
                uint64_t* longest);
+
+// Batched decodes.  The parameters of a stream are lat_params_size() bytes;
+// the batch keeps one array of them and lists of work items on the device.
+struct LatItem {
+    uint32_t stream;
+    uint32_t index;
+    uint32_t count;
+    uint32_t pad;
+};
+struct LatSmem {
+    size_t prep, sync, scan, final;
+};
+constexpr uint32_t kLatBatchWarps = 4;   // of a sync-pass CTA
+
+size_t lat_params_size();
+void lat_fill_params(void* dst, const LatCall& call, const LatPlan& plan, void* slice,
+                     uint32_t* d_status, uint32_t width);
+uint32_t lat_prep_items(const LatPlan& plan);
+uint32_t lat_scan_tiles(const LatPlan& plan);
+uint32_t lat_final_ctas(const LatPlan& plan);
+LatSmem lat_batch_smem(const LatCall& call, const LatPlan& plan);
+void lat_batch_init();
+void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    cudaStream_t st);
+void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    cudaStream_t st);
+void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
+                    uint32_t* ticket, cudaStream_t st);
+void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st);
 
 }  // namespace mans

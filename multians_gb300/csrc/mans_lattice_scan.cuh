@@ -11,8 +11,9 @@
 //   status, nblk
 // and, for paths that run out of slots and for the end of the path,
 //   uint32_t repair_blocks()       sequential blocks a repair may take
-//   void repair_load(sm)           the CTA: the tables a repair reads into the
-//                                  kernel's dynamic shared memory sm
+//   uint32_t repair_words()        words of the tables a repair reads, and
+//   void repair_load(sm)           the CTA: loads them into the kernel's dynamic
+//                                  shared memory sm (lat_scan_smem bytes)
 //   void advance(sm, b, ent, off)  one thread: block b from its true entry
 //   void finish(slot, off)         one thread: the path's slot and offset at
 //                                  the last block
@@ -32,6 +33,11 @@ constexpr uint32_t kLatEntBits = 21;       // entry: bit offset (8), state index
 constexpr uint32_t kLatScanThreads = 256;
 constexpr uint32_t kLatScanPer = 4;        // blocks per thread of the scan
 constexpr uint32_t kLatScanTile = kLatScanThreads * kLatScanPer;
+
+// Dynamic shared memory of a scan kernel, used by repairs only.
+constexpr size_t lat_scan_smem(size_t repair_words) {
+    return (repair_words + 1) / 2 * 8 + kLatScanTile * 8;
+}
 
 // counters: next start, scan tile ticket, longest trajectory (blocks), blocks
 // decoded by all trajectories, blocks decoded again by repairs
@@ -274,7 +280,8 @@ template <class P, uint32_t kD>
 __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
                                         typename LatTile<P, kD>::Shared& sh, uint32_t first) {
     extern __shared__ __align__(16) uint32_t lat_repair_sm[];
-    __shared__ uint2 s_over[kLatScanTile];   // entry and count of the blocks decoded here
+    // entry and count of the blocks decoded here
+    uint2* const s_over = reinterpret_cast<uint2*>(lat_repair_sm + ((p.repair_words() + 1) & ~1u));
     __shared__ uint32_t s_at, s_ent;
     const uint32_t stop = min(first + kLatScanTile, p.nblk);
     p.repair_load(lat_repair_sm);
