@@ -111,11 +111,12 @@ typedef struct {
 #define MANS_DECODE_NO_SEEDS 0x40u
 
 /* Lattice decode, set by the planner in plans that fix no geometry, capture
- * or seeds and do not capture: trajectories start at many places and each
- * ends at the first other one it meets (a chain several times shorter than
- * a region and its merge walk).  The plan's geometry then stands for the
- * decode that follows when a path runs out of slots
- * (MANS_DEV_SYNC_OVERFLOW).  The output is identical either way. */
+ * or seeds: trajectories start at many places and each ends at the first
+ * other one it meets (a chain several times shorter than a region and its
+ * merge walk).  The plan's geometry and capture then stand for the decode
+ * that follows when the path runs out of slots (MANS_DEV_SYNC_OVERFLOW) or
+ * the workspace is too small for the lattice.  The output is identical
+ * either way. */
 #define MANS_DECODE_LATTICE 0x80u
 
 /* Fills `out` with the geometry the decoder uses for this call: the built-in

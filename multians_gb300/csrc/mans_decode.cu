@@ -2250,9 +2250,9 @@ static int plan_core(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* h
     // the lattice decode where the plan is the planner's own (a plan given
     // back as a hint keeps its choice)
     const bool lattice =
-        !capture && n_out > 0 &&
+        n_out > 0 &&
         ((c.flags & MANS_DECODE_LATTICE) ||
-         (c.block_units == 0 && c.region_blocks == 0 && c.walk_slots == 0 &&
+         (c.block_units == 0 && c.region_blocks == 0 && c.walk_slots == 0 && c.capture_bytes == 0 &&
           !(c.flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS | MANS_DECODE_NO_CAPTURE |
                        MANS_DECODE_CAPTURE | MANS_PLAN_MODEL))));
     c.flags &= ~MANS_DECODE_LATTICE;
@@ -2495,7 +2495,7 @@ static uint32_t start_pos(uint32_t first_bit, uint32_t flags) {
 // on every SM.
 static bool lattice_plan(const mans_cfg& cfg, size_t n_units, size_t n_out, uint32_t L,
                          size_t aux_bytes, LatPlan* out) {
-    if (!(cfg.flags & MANS_DECODE_LATTICE) || cfg.capture_bytes) return false;
+    if (!(cfg.flags & MANS_DECODE_LATTICE)) return false;
     const double bps = 32.0 * (double) n_units / (double) n_out;
     return lat_plan(n_units, n_out, L, mean_meeting_units(L, bps), 152 * 16 * 32, aux_bytes, out);
 }
@@ -2985,7 +2985,7 @@ int mans_decode_loop(const mans_stream_desc* streams, uint32_t n, const mans_cfg
 
 // ---------------------------------------------------------------------------
 // Batched decode of many independent streams (one launch of each kernel for
-// the whole batch).  Streams that neither capture nor fix a geometry go
+// the whole batch).  Streams that neither ask for capture nor fix a geometry go
 // through the lattice kernels (mans_lattice.cu), the others through the
 // BatchItem kernels above.  Measured, regions and walks -> lattice: 256
 // streams of 4 KB to 4 MB, L = 1024 1922 -> 932 us; 1024 of them 3555 -> 2296;
@@ -3093,7 +3093,7 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         h.flags |= MANS_PLAN_MODEL;
         int rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &sp.cfg);
         if (rc != MANS_OK) return rc;
-        if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE) && sp.cfg.capture_bytes == 0) {
+        if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE)) {
             // as many starts as its share of the batch's symbols has of the
             // lanes side by side, in the workspace the stream's own plan has
             const size_t nblk = num_blocks(d[i].n_units, sp.cfg.block_units);

@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams*
     lat_load_params(sp, ps + it.stream);
     if (sp.B == 4) lat_sync_body<4>(sp, &s_next, it.count);
     else if (sp.B == 8) lat_sync_body<8>(sp, &s_next, it.count);
-    else lat_sync_body<16>(sp, &s_next, it.count);
+    else if (sp.B == 16) lat_sync_body<16>(sp, &s_next, it.count);
+    else lat_sync_body<32>(sp, &s_next, it.count);
 }
 
 // The ticket hands items out in list order, which holds each stream's tiles
@@ -102,7 +103,8 @@ template <bool kRev>
 __device__ __forceinline__ void lat_final_any(const LatParams& p, const LatItem& it) {
     if (p.B == 4) lat_final_body<kRev, 4>(p, it.index, it.count);
     else if (p.B == 8) lat_final_body<kRev, 8>(p, it.index, it.count);
-    else lat_final_body<kRev, 16>(p, it.index, it.count);
+    else if (p.B == 16) lat_final_body<kRev, 16>(p, it.index, it.count);
+    else lat_final_body<kRev, 32>(p, it.index, it.count);
 }
 
 // index: the CTA of the stream's count.
@@ -117,8 +119,8 @@ __global__ void __launch_bounds__(kLatFinalThreads) k_lat_final_batch(const LatP
 
 static_assert(kLatThreads == 32 * kLatBatchWarps, "batch items");
 
-// CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps, near
-// the rate its shared-memory lookups allow.
+// CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps (20 with
+// blocks of 32 units), near the rate its shared-memory lookups allow.
 constexpr uint32_t kLatCtas = 4;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
@@ -185,15 +187,18 @@ void lat_attributes() {
                              (int) kLatFinalSmemMax);
     };
     set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_sync_batch); set(k_lat_final_batch);
-    set(k_lat_sync<4>); set(k_lat_sync<8>); set(k_lat_sync<16>);
+    set(k_lat_sync<4>); set(k_lat_sync<8>); set(k_lat_sync<16>); set(k_lat_sync<32>);
     set(k_lat_final<false, 4>); set(k_lat_final<false, 8>); set(k_lat_final<false, 16>);
+    set(k_lat_final<false, 32>); set(k_lat_final<true, 32>);
     set(k_lat_final<true, 4>); set(k_lat_final<true, 8>); set(k_lat_final<true, 16>);
     if (dev < 64) done |= 1ull << dev;
 }
 
 template <bool kRev>
 void (*final_kernel(uint32_t B))(LatParams) {
-    return B == 4 ? k_lat_final<kRev, 4> : (B == 8 ? k_lat_final<kRev, 8> : k_lat_final<kRev, 16>);
+    return B == 4 ? k_lat_final<kRev, 4>
+                  : (B == 8 ? k_lat_final<kRev, 8>
+                            : (B == 16 ? k_lat_final<kRev, 16> : k_lat_final<kRev, 32>));
 }
 
 LatParams lat_params(const LatCall& call, const LatPlan& plan, char* base) {
@@ -231,22 +236,26 @@ LatParams lat_params(const LatCall& call, const LatPlan& plan, char* base) {
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out) {
     if (n_out >> (63 - kLatEntBits)) return false;
-    // about 128 symbols per block: the final pass stages 32 blocks a warp,
-    // and a step's share of a block's bookkeeping stays below a tenth
+    // About 128 symbols per block: the final pass stages 32 blocks a warp, and
+    // a step's share of a block's bookkeeping stays below a tenth.  Blocks of
+    // 32 units from 5.3 bits per symbol on (256 MB at 6 bits: 691 -> 629 us,
+    // 512 MB at 8.6 bits 1511 -> 1192, the scan and the slots' traffic halved;
+    // more starts pay there, their trajectories meet soon).
     const double spu = (double) n_out / (double) n_units;
-    uint32_t b_pref = 16;
+    uint32_t b_pref = 32;
     while (b_pref > 4 && spu * b_pref > 192.0) b_pref /= 2;
+    const double side = lanes * (b_pref == 32 ? 1.5 : 1.0);
     // Starts every s units: as many as run side by side, but no closer than
     // the slots allow (about 1.2 sqrt(2 meet / s) distinct trajectories are
     // under way at a place on average, twice that at most over a long
     // stream; data that meets later than the model has it costs repairs).
-    const double s_par = std::max((double) n_units / lanes, 4.0);
+    const double s_par = std::max((double) n_units / side, 4.0);
     uint32_t D = s_par >= 4.0 * meet ? 4 : (s_par >= meet / 1.5 ? 8 : 12);
     for (; D >= 4; D -= 4) {
         const double s = std::max(s_par, D == 12 ? meet / 6.0 : (D == 8 ? meet / 1.5 : 4.0 * meet));
         uint32_t B = b_pref;
         while (B > 4 && B > s) B /= 2;
-        for (; B <= 16; B *= 2) {
+        for (; B <= 32; B *= 2) {
             const size_t nblk = n_units / B + 1;
             if (nblk * D > 0xffffffffull) continue;
             const size_t need = lat_layout(nblk, D, L).total;
@@ -287,11 +296,12 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
         if (plan.nseed <= width * sched) th = 32;
         p.width = width;
         const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
-        const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
+        const unsigned grid = std::min<unsigned>(need, (unsigned) sms * (plan.B == 32 ? kLatCtas + 1 : kLatCtas) * (kLatThreads / th));
         const size_t sm = lat_sync_smem(call.L, plan.B, th);
         if (plan.B == 4) k_lat_sync<4><<<grid, th, sm, st>>>(p);
         else if (plan.B == 8) k_lat_sync<8><<<grid, th, sm, st>>>(p);
-        else k_lat_sync<16><<<grid, th, sm, st>>>(p);
+        else if (plan.B == 16) k_lat_sync<16><<<grid, th, sm, st>>>(p);
+        else k_lat_sync<32><<<grid, th, sm, st>>>(p);
     }
     mark(2, st);
     mark(3, st);

@@ -27,9 +27,10 @@
 // times, so starts are spread no closer than the GPU has idle lanes for.
 //
 // Measured on GB300, whole decodes, regions and walks -> lattice: 4 KB 151 ->
-// 90 us, 128 KB at 3.8 bits per symbol 473 -> 168, 16 MB at 6 bits 324 ->
-// 190, 128 MB at 1.5 bits and L = 4096 4139 -> 1255, 256 MB at 0.67 bits
-// and L = 4096 2294 -> 998.
+// 87 us, 128 KB at 3.8 bits per symbol 463 -> 156, 16 MB at 6 bits 328 ->
+// 190, 128 MB at 1.5 bits and L = 4096 4171 -> 1133, 256 MB at 0.67 bits and
+// L = 4096 2478 -> 946; against regions with symbol capture, 256 MB at 6 bits
+// 693 -> 619, 512 MB at 8.6 bits 1440 -> 1168.
 #pragma once
 
 #include <cstdint>
@@ -69,7 +70,7 @@ struct LatParams {
     uint32_t L;
     uint32_t first_idx;
     uint32_t first_pos;
-    uint32_t B;                     // units per block: 4, 8 or 16
+    uint32_t B;                     // units per block: 4, 8, 16 or 32
     uint32_t nb;                    // blocks between starts
     uint32_t D;                     // slots per block: 4, 8 or 12
     uint32_t nblk;
@@ -241,53 +242,99 @@ struct LatCursor {
     }
 };
 
+// The state between the two steps of a pair: the window is the one before
+// the pair, `u` the unit a refill takes.
+struct LatMid {
+    uint32_t a, e, pos, w0, w1, u, base;
+    __device__ __forceinline__ void resume(LatCursor& c) const {
+        const bool r = ((pos ^ base) & 32u) != 0;
+        c.a = a;
+        c.e = e;
+        c.pos = pos;
+        c.w0 = r ? w1 : w0;
+        c.w1 = r ? u : w1;
+    }
+};
+
+// Two steps with one unit load and one refill: the second step's window is
+// cut from both units (offset < 32 + 16, code <= 16 bits), and two codes pass
+// at most one unit.  4.0 cycles a warp and step with the shared pipe full
+// against 4.5 for single steps, 47 against 47.5 alone.
+__device__ __forceinline__ void lat_pair(LatCursor& c, uint32_t col, uint32_t mask, uint32_t& y1,
+                                         uint32_t& y2, LatMid& m) {
+    m.u = lds32(col | ((c.pos << 2) & mask));
+    m.w0 = c.w0;
+    m.w1 = c.w1;
+    m.base = c.pos;
+    y1 = c.e;
+    m.a = (y1 >> 16) + (__funnelshift_r(c.w0, c.w1, c.pos) & lat_mask4(y1));
+    m.e = lds32(m.a);
+    m.pos = __dp4a(y1, 1u, c.pos);
+    const uint32_t o = __dp4a(y1, 1u, c.pos & 31u);
+    const uint32_t x = (uint32_t) ((((unsigned long long) c.w1 << 32) | c.w0) >> o);
+    y2 = m.e;
+    c.a = (y2 >> 16) + (x & lat_mask4(y2));
+    c.e = lds32(c.a);
+    c.pos = __dp4a(y2, 1u, m.pos);
+    const bool r = ((c.pos ^ m.base) & 32u) != 0;
+    c.w0 = r ? m.w1 : m.w0;
+    c.w1 = r ? m.u : m.w1;
+}
+
 // Decodes to the first codeword at or after position `be`, adding the
-// codewords stepped over to cnt.  Four steps a test, so the fourth may pass
-// the boundary: every step keeps its state in registers of its own and the
-// first one past the boundary is taken (a tail loop of single steps costs a
-// test per step and, lane against lane, a dozen steps a block).
+// codewords stepped over to cnt.  Two pairs a test, so the last steps may
+// pass the boundary: every step keeps its state in registers of its own and
+// the first one past the boundary is taken (a tail loop of single steps
+// costs a test per step and, lane against lane, a dozen steps a block).
 __device__ __forceinline__ void lat_block(LatCursor& c, uint32_t col, uint32_t mask, uint32_t be,
                                           uint32_t& cnt) {
-    LatCursor c0, c1, c2;
+    LatMid m0, m2;
+    LatCursor c1;
     uint32_t n0, n1, n2;
     do {
-        cnt = __dp4a(c.step(col, mask), 0x100u, cnt);   // + byte 1
-        c0 = c;
-        n0 = cnt;
-        cnt = __dp4a(c.step(col, mask), 0x100u, cnt);
+        uint32_t y1, y2;
+        lat_pair(c, col, mask, y1, y2, m0);
+        n0 = __dp4a(y1, 0x100u, cnt);   // + byte 1
+        n1 = __dp4a(y2, 0x100u, n0);
         c1 = c;
-        n1 = cnt;
-        cnt = __dp4a(c.step(col, mask), 0x100u, cnt);
-        c2 = c;
-        n2 = cnt;
-        cnt = __dp4a(c.step(col, mask), 0x100u, cnt);
+        lat_pair(c, col, mask, y1, y2, m2);
+        n2 = __dp4a(y1, 0x100u, n1);
+        cnt = __dp4a(y2, 0x100u, n2);
     } while ((int32_t) (be - c.pos) > 0);
-    if ((int32_t) (be - c2.pos) <= 0) { c = c2; cnt = n2; }
+    if ((int32_t) (be - m2.pos) <= 0) { m2.resume(c); cnt = n2; }
     if ((int32_t) (be - c1.pos) <= 0) { c = c1; cnt = n1; }
-    if ((int32_t) (be - c0.pos) <= 0) { c = c0; cnt = n0; }
+    if ((int32_t) (be - m0.pos) <= 0) { m0.resume(c); cnt = n0; }
 }
 
 // ---------------------------------------------------------------------------
 // sync pass
 
-// Volatile, so that the load is issued where it stands, a block ahead.
-__device__ __forceinline__ uint4 lat_ld_units(const uint32_t* a) {
-    uint4 v;
+// Loads of 16 or 32 bytes of units; volatile, so that they are issued where
+// they stand, a block ahead.
+__device__ __forceinline__ void lat_ld_units(uint32_t* r, const uint32_t* a) {
     asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(a));
-    return v;
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(a));
+}
+__device__ __forceinline__ void lat_ld_units8(uint32_t* r, const uint32_t* a) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                   "=r"(r[6]), "=r"(r[7]) : "l"(a));
 }
 
-// The units of block b of a lane into `r` (zero past the end).
+// The units of block b of a lane into `r` (zero past the end); wide: the
+// stream starts on a 32-byte boundary.  Lanes read apart, so a load costs the
+// L1 a pass for every lane whatever its width.
 template <uint32_t kB>
 __device__ __forceinline__ void lat_load_units(uint32_t (&r)[kB], const uint32_t* __restrict__ in,
-                                               uint32_t n, uint32_t b) {
+                                               uint32_t n, uint32_t b, bool wide) {
     const unsigned long long u = (unsigned long long) b * kB;
     if (u + kB <= n) {
+        if (kB >= 8 && wide) {
 #pragma unroll
-        for (uint32_t i = 0; i < kB / 4; ++i) {
-            const uint4 x = lat_ld_units(in + u + 4 * i);
-            r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
+            for (uint32_t i = 0; i < kB / 8; ++i) lat_ld_units8(r + 8 * i, in + u + 8 * i);
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < kB / 4; ++i) lat_ld_units(r + 4 * i, in + u + 4 * i);
         }
     } else {
 #pragma unroll
@@ -310,7 +357,7 @@ __device__ __forceinline__ void lat_store_units(const uint32_t (&r)[kB], uint32_
 }
 
 // Shared memory of a sync-pass CTA: the table, then per warp a ring of two
-// blocks for every lane, aligned to its size (at most 4 KB).
+// blocks for every lane, aligned to its size (at most 8 KB).
 __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B * 128; }
 
 // One lane per trajectory, persistent: a lane whose trajectory ended takes
@@ -336,6 +383,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     constexpr uint32_t kBits = kB * 32;
     const uint32_t col = ((tb + p.L * 4 + kRing - 1) & ~(kRing - 1)) + warp * kRing + lane * 4;
     const uint32_t D = p.D;
+    const bool wide = ((uintptr_t) p.units & 31) == 0;
 
     bool on = false, exhausted = false;
     LatCursor c{};
@@ -379,12 +427,12 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                 if (on) {
                     carry = 0;
                     uint32_t r0[kB];
-                    lat_load_units<kB>(r0, p.units, p.n_units, b);
-                    lat_load_units<kB>(nx, p.units, p.n_units, b + 1);
+                    lat_load_units<kB>(r0, p.units, p.n_units, b, wide);
+                    lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
                     const uint32_t s = (b & 1u) * kB;
                     lat_store_units<kB>(r0, col, s, carry);
                     lat_store_units<kB>(nx, col, s ^ kB, carry);
-                    lat_load_units<kB>(nx, p.units, p.n_units, b + 2);
+                    lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
                     c.pos = s * 32 + rel + 64;
                     be = s * 32 + kBits + 64;
                     const uint32_t u0 = s + (rel >> 5);
@@ -445,7 +493,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         // block b + 1 (one ahead again) into the half of the ring that is free
         const uint32_t s = (b & 1u) * kB;      // slots of block b
         lat_store_units<kB>(nx, col, s ^ kB, carry);
-        lat_load_units<kB>(nx, p.units, p.n_units, b + 2);
+        lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
         if (s == 0) c.pos -= 2 * kBits;
         be = s * 32 + kBits + 64;
     }
@@ -460,9 +508,12 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
 // ---------------------------------------------------------------------------
 // final pass
 
-// Unit slots of a lane's tile in the final pass: the block and at least
-// four units of look-ahead, a power of two (the cursor masks its slot).
-__host__ __device__ constexpr uint32_t lat_tile_slots(uint32_t B) { return B == 4 ? 8 : 2 * B; }
+// Unit slots of a lane's tile in the final pass, a power of two (the cursor
+// masks its slot): the block and four units of look-ahead; with blocks of 32
+// units the look-ahead takes the first slots once the cursor has left them.
+__host__ __device__ constexpr uint32_t lat_tile_slots(uint32_t B) {
+    return B == 4 ? 8 : (B == 32 ? 32 : 2 * B);
+}
 
 __device__ __forceinline__ void lat_sts8(uint32_t a, uint32_t v) {
     asm volatile("st.shared.u8 [%0], %1;" :: "r"(a), "r"(v) : "memory");
@@ -490,23 +541,18 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     if (b + 1 < p.nblk) off_nx = lane < 31 ? from_next : __ldg(p.start + b + 1) >> kLatEntBits;
     // units: the block's and four more (zero past the end)
     const uint32_t col = tile + lane * 4;
+    uint32_t ahead[4] = {0, 0, 0, 0}, carry = 0;
     if (have) {
-        uint32_t r[kB + 4];
-        const unsigned long long u = (unsigned long long) b * kB;
-        if (u + kB + 4 <= p.n_units) {
-            const uint4* v = reinterpret_cast<const uint4*>(p.units + u);
-#pragma unroll
-            for (uint32_t i = 0; i < kB / 4 + 1; ++i) {
-                const uint4 x = __ldg(v + i);
-                r[4 * i] = x.x; r[4 * i + 1] = x.y; r[4 * i + 2] = x.z; r[4 * i + 3] = x.w;
-            }
-        } else {
-#pragma unroll
-            for (uint32_t i = 0; i < kB + 4; ++i) r[i] = u + i < p.n_units ? __ldg(p.units + u + i) : 0u;
-        }
-        uint32_t carry = 0;
-        lat_store_units<kB + 4>(r, col, 0, carry);
+        const bool wide = ((uintptr_t) p.units & 31) == 0;
+        uint32_t r[kB];
+        lat_load_units<kB>(r, p.units, p.n_units, b, wide);
+        lat_load_units<4>(ahead, p.units, p.n_units, (b + 1) * (kB / 4), false);
+        lat_store_units<kB>(r, col, 0, carry);
+        if (kB < 32) lat_store_units<4>(ahead, col, kB, carry);
     }
+    const auto look_ahead = [&]() {
+        if (kB == 32) lat_store_units<4>(ahead, col, 0, carry);
+    };
     const unsigned long long off0 = __shfl_sync(0xffffffffu, off, 0);
     const uint32_t last_lane = min(31u, p.nblk - 1 - b0);
     const unsigned long long off_end = __shfl_sync(0xffffffffu, off_nx, last_lane);
@@ -536,34 +582,57 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
         c.w0 = lds32(col + (rel >> 5) * 128);
         c.w1 = lds32(col + ((rel >> 5) + 1) * 128);
         const uint32_t pos_cap = kB * 32 + kMaxBits + 1 + 64;
+        // past this position the first slots are free (kB = 32)
+        const uint32_t pos_half = kB == 32 ? 64 + 16 * 32 : pos_cap;
+        LatMid m;
         const uint32_t full = off_nx >= off ? (uint32_t) min(off_nx - off, 0xffffffffull) : 0u;
         uint32_t i = 0;
         if (staged && !kRev) {
             uint32_t q = stage_addr + sb + (uint32_t) (off - wlo);
             for (; i < cnt && (q & 3u) && c.pos < pos_cap; ++i, ++q)
                 lat_sts8(q, c.step(col, kMask) >> 8);
-            for (; i + 4 <= cnt && c.pos < pos_cap; i += 4, q += 4) {
-                const uint32_t y0 = c.step(col, kMask), y1 = c.step(col, kMask);
-                const uint32_t y2 = c.step(col, kMask), y3 = c.step(col, kMask);
-                sts32(q, __byte_perm(__byte_perm(y0, y1, 0x0051), __byte_perm(y2, y3, 0x5100), 0x7610));
+            const auto four = [&](uint32_t limit) {
+                for (; i + 4 <= cnt && c.pos < limit; i += 4, q += 4) {
+                    uint32_t y0, y1, y2, y3;
+                    lat_pair(c, col, kMask, y0, y1, m);
+                    lat_pair(c, col, kMask, y2, y3, m);
+                    sts32(q, __byte_perm(__byte_perm(y0, y1, 0x0051), __byte_perm(y2, y3, 0x5100), 0x7610));
+                }
+            };
+            if (kB == 32) {
+                four(pos_half);
+                look_ahead();
             }
+            four(pos_cap);
             for (; i < cnt && c.pos < pos_cap; ++i, ++q) lat_sts8(q, c.step(col, kMask) >> 8);
         } else if (staged) {
             // decode index i goes to output n_out - 1 - i: downwards
             uint32_t q = stage_addr + sb + (uint32_t) (p.n_out - 1 - off - wlo);
             for (; i < cnt && (q & 3u) != 3u && c.pos < pos_cap; ++i, --q)
                 lat_sts8(q, c.step(col, kMask) >> 8);
-            for (; i + 4 <= cnt && c.pos < pos_cap; i += 4, q -= 4) {
-                const uint32_t y0 = c.step(col, kMask), y1 = c.step(col, kMask);
-                const uint32_t y2 = c.step(col, kMask), y3 = c.step(col, kMask);
-                sts32(q - 3, __byte_perm(__byte_perm(y3, y2, 0x0051), __byte_perm(y1, y0, 0x5100), 0x7610));
+            const auto four = [&](uint32_t limit) {
+                for (; i + 4 <= cnt && c.pos < limit; i += 4, q -= 4) {
+                    uint32_t y0, y1, y2, y3;
+                    lat_pair(c, col, kMask, y0, y1, m);
+                    lat_pair(c, col, kMask, y2, y3, m);
+                    sts32(q - 3, __byte_perm(__byte_perm(y3, y2, 0x0051), __byte_perm(y1, y0, 0x5100), 0x7610));
+                }
+            };
+            if (kB == 32) {
+                four(pos_half);
+                look_ahead();
             }
+            four(pos_cap);
             for (; i < cnt && c.pos < pos_cap; ++i, --q) lat_sts8(q, c.step(col, kMask) >> 8);
         } else if (!kRev) {
             uint8_t* dst = p.out + off;
+            for (; i < cnt && c.pos < pos_half; ++i) dst[i] = (uint8_t) (c.step(col, kMask) >> 8);
+            look_ahead();
             for (; i < cnt && c.pos < pos_cap; ++i) dst[i] = (uint8_t) (c.step(col, kMask) >> 8);
         } else {
             uint8_t* dst = p.out + (p.n_out - 1 - off);
+            for (; i < cnt && c.pos < pos_half; ++i) *(dst - i) = (uint8_t) (c.step(col, kMask) >> 8);
+            look_ahead();
             for (; i < cnt && c.pos < pos_cap; ++i) *(dst - i) = (uint8_t) (c.step(col, kMask) >> 8);
         }
         // a block decoded to its full count ends at the next block start

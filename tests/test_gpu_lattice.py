@@ -1,5 +1,5 @@
 """GPU parity of the lattice decode (the planner's own plan without symbol
-capture): streams at the edges of its blocks (4, 8, 16 units), scan tiles
+capture): streams at the edges of its blocks (4, 8, 16, 32 units), scan tiles
 (1024 blocks), slot counts (4, 8, 12) and warp widths, in both output orders
 and at odd output addresses, and data whose trajectories meet later than the
 planner expects, so that the true path runs out of slots and is repaired.
@@ -58,12 +58,13 @@ def test_block_edges(mg, oracle_lib, L, lam):
 
 @pytest.mark.parametrize("tiles", [1, 2, 33])
 @pytest.mark.parametrize("d", [-1, 0, 1])
-def test_scan_tile_edges(mg, oracle_lib, tiles, d):
-    """Streams of about 1024 blocks (16 units each) per scan tile, one unit
-    around the edge, and a look-back longer than 32 tiles."""
+@pytest.mark.parametrize("lam,bits,block", [(0.05, 6.0, 32), (0.2, 3.83, 16)])
+def test_scan_tile_edges(mg, oracle_lib, tiles, d, lam, bits, block):
+    """Streams of about 1024 blocks per scan tile, one unit around the edge,
+    and a look-back longer than 32 tiles."""
     O = oracle_lib
-    n_units = tiles * 1024 * 16 + d
-    st = O.make_stream(seed=tiles * 10 + d, lam=0.05, n=int(n_units * 32 / 6.0), L=1024)
+    n_units = tiles * 1024 * block + d
+    st = O.make_stream(seed=tiles * 10 + d, lam=lam, n=int(n_units * 32 / bits), L=1024)
     got, _ = _decode(mg, st)
     assert np.array_equal(got[::-1], st.symbols)
 
