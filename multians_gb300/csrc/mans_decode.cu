@@ -2412,7 +2412,14 @@ size_t mans_aux_size(size_t n_units, const mans_cfg* cfg) {
         return 0;
     const size_t nblk = num_blocks(n_units, cfg->block_units);
     const size_t nreg = (nblk + cfg->region_blocks - 1) / cfg->region_blocks;
-    return layout_for(nblk, nreg, cfg->walk_slots, cfg->capture_bytes).total;
+    const size_t with_capture = layout_for(nblk, nreg, cfg->walk_slots, cfg->capture_bytes).total;
+    const size_t regions = layout_for(nblk, nreg, cfg->walk_slots, 0).total;
+    // a lattice decode with all its slots (less when it gives up slots)
+    if ((cfg->flags & MANS_DECODE_LATTICE) && cfg->walk_slots == kMaxWalkSlots &&
+        cfg->block_units >= 8)
+        return with_capture - regions +
+               std::max(regions, lat_bytes(num_blocks(n_units, cfg->block_units)));
+    return with_capture;
 }
 
 size_t mans_aux_size_max(size_t n_units) {

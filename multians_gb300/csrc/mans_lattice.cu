@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
 }
 
 template <uint32_t kD>
-__global__ void __launch_bounds__(kLatScanThreads) k_lat_scan(LatParams p) {
+__global__ void __launch_bounds__(kLatScanThreads, 5) k_lat_scan(LatParams p) {
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(kLatScanThreads) k_lat_scan_batch(const LatPar
     lat_load_params(sp, ps + it.stream);
     if (sp.D == 4) lat_scan_body<LatParams, 4>(sp, it.index);
     else if (sp.D == 8) lat_scan_body<LatParams, 8>(sp, it.index);
-    else lat_scan_body<LatParams, 12>(sp, it.index);
+    else if (sp.D == 12) lat_scan_body<LatParams, 12>(sp, it.index);
+    else lat_scan_body<LatParams, 16>(sp, it.index);
 }
 
 template <bool kRev>
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(kLatFinalThreads) k_lat_final_batch(const LatP
 
 static_assert(kLatThreads == 32 * kLatBatchWarps, "batch items");
 
-// CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps (20 with
-// blocks of 32 units), near the rate its shared-memory lookups allow.
+// CTAs of kLatThreads a persistent sync pass keeps on an SM: 16 warps, near
+// the rate its shared-memory lookups allow.
 constexpr uint32_t kLatCtas = 4;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t) 255; }
@@ -147,13 +148,13 @@ LatLayout lat_layout(size_t nblk, uint32_t D, uint32_t L) {
 }
 
 size_t lat_sync_smem(uint32_t L, uint32_t B, uint32_t threads) {
-    return (size_t) L * 4 + lat_ring_bytes(B) * (threads / 32 + 1);
+    return (((size_t) L * 4 + 15) & ~(size_t) 15) + lat_ring_bytes(B) * (threads / 32);
 }
 
 constexpr size_t kLatFinalSmemMax = 200 * 1024;
 size_t lat_final_smem(uint32_t L, uint32_t B, uint32_t stage_cap, uint32_t threads) {
-    return (size_t) L * 4 + (size_t) lat_final_warp_bytes(B) * (threads / 32 + 1) +
-           (size_t) (threads / 32) * (stage_cap + 16);
+    return (((size_t) L * 4 + 15) & ~(size_t) 15) +
+           (size_t) (threads / 32) * (lat_final_warp_bytes(B) + stage_cap + 16);
 }
 
 // Staging bytes per warp of the final pass: 1.25x the expected symbols of
@@ -233,35 +234,41 @@ LatParams lat_params(const LatCall& call, const LatPlan& plan, char* base) {
 
 }  // namespace
 
+size_t lat_bytes(size_t nblk) { return lat_layout(nblk, kLatSlotsMax, kMaxStates).total; }
+
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out) {
     if (n_out >> (63 - kLatEntBits)) return false;
     // About 128 symbols per block: the final pass stages 32 blocks a warp, and
     // a step's share of a block's bookkeeping stays below a tenth.  Blocks of
     // 32 units from 5.3 bits per symbol on (256 MB at 6 bits: 691 -> 629 us,
-    // 512 MB at 8.6 bits 1511 -> 1192, the scan and the slots' traffic halved;
-    // more starts pay there, their trajectories meet soon).
+    // 512 MB at 8.6 bits 1511 -> 1192, the scan and the slots' traffic halved).
     const double spu = (double) n_out / (double) n_units;
     uint32_t b_pref = 32;
     while (b_pref > 4 && spu * b_pref > 192.0) b_pref /= 2;
-    const double side = lanes * (b_pref == 32 ? 1.5 : 1.0);
     // Starts every s units: as many as run side by side, but no closer than
-    // the slots allow (about 1.2 sqrt(2 meet / s) distinct trajectories are
-    // under way at a place on average, twice that at most over a long
-    // stream; data that meets later than the model has it costs repairs).
-    const double s_par = std::max((double) n_units / side, 4.0);
-    uint32_t D = s_par >= 4.0 * meet ? 4 : (s_par >= meet / 1.5 ? 8 : 12);
+    // the slots allow.  About 1.2 sqrt(2 T / s) distinct trajectories are under
+    // way at a place on average, and twice that at most over a long stream: s
+    // = meet / per_meet[D / 4 - 1] leaves room for a T 2.7 times the model's
+    // (symbols of equal frequency meet that late).  Closer ones run out of
+    // slots: 3 M of eight equally frequent symbols, L = 1024, 12 slots, s = meet
+    // / 4: 3 blocks repaired, 0.6 ms; meet / 8: 5812 blocks, 86 ms.
+    static const double per_meet[4] = {0.17, 1.0, 4.0, 6.8};
+    const double s_par = std::max((double) n_units / lanes, 4.0);
+    uint32_t D = 4;
+    while (D < kLatSlotsMax && s_par < meet / per_meet[D / 4 - 1]) D += 4;
     for (; D >= 4; D -= 4) {
-        const double s = std::max(s_par, D == 12 ? meet / 6.0 : (D == 8 ? meet / 1.5 : 4.0 * meet));
+        const double s = std::max(s_par, meet / per_meet[D / 4 - 1]);
         uint32_t B = b_pref;
-        while (B > 4 && B > s) B /= 2;
+        while (B > 4 && B > s && spu * B >= 96.0) B /= 2;
         for (; B <= 32; B *= 2) {
             const size_t nblk = n_units / B + 1;
             if (nblk * D > 0xffffffffull) continue;
             const size_t need = lat_layout(nblk, D, L).total;
             if (need > bytes) continue;
             out->B = B;
-            out->nb = (uint32_t) std::max(1.0, std::floor(s / B + 0.5));
+            // rounded up, so that starts never outnumber the lanes of one wave
+            out->nb = (uint32_t) std::max(1.0, s > s_par ? std::floor(s / B + 0.5) : std::ceil(s / B));
             out->D = D;
             out->nblk = (uint32_t) nblk;
             out->nseed = (uint32_t) ((nblk + out->nb - 1) / out->nb);
@@ -296,7 +303,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
         if (plan.nseed <= width * sched) th = 32;
         p.width = width;
         const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
-        const unsigned grid = std::min<unsigned>(need, (unsigned) sms * (plan.B == 32 ? kLatCtas + 1 : kLatCtas) * (kLatThreads / th));
+        const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
         const size_t sm = lat_sync_smem(call.L, plan.B, th);
         if (plan.B == 4) k_lat_sync<4><<<grid, th, sm, st>>>(p);
         else if (plan.B == 8) k_lat_sync<8><<<grid, th, sm, st>>>(p);
@@ -310,7 +317,8 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
         const size_t sm = lat_scan_smem(call.L);
         if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, sm, st>>>(p);
         else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, sm, st>>>(p);
-        else k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
+        else if (plan.D == 12) k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
+        else k_lat_scan<16><<<g, kLatScanThreads, sm, st>>>(p);
     }
     mark(4, st);
     {

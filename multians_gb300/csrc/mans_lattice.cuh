@@ -72,7 +72,7 @@ struct LatParams {
     uint32_t first_pos;
     uint32_t B;                     // units per block: 4, 8, 16 or 32
     uint32_t nb;                    // blocks between starts
-    uint32_t D;                     // slots per block: 4, 8 or 12
+    uint32_t D;                     // slots per block: 4, 8, 12 or 16
     uint32_t nblk;
     uint32_t nseed;
     uint32_t stage_cap;             // final-pass staging bytes per warp
@@ -82,7 +82,7 @@ struct LatParams {
     // scan hooks (mans_lattice_scan.cuh): an entry is the bit offset from the
     // block start and the state index << 8, an offset counts symbols
     __device__ __forceinline__ uint32_t repair_blocks() const {
-        return n_units <= 32768 ? ~0u : 1024u;
+        return n_units <= 32768 ? ~0u : 4096u;
     }
     __device__ __forceinline__ void finish(uint32_t, unsigned long long) const {}
     __device__ __forceinline__ void finish_seq(const uint32_t*, uint32_t, unsigned long long) const {}
@@ -92,20 +92,24 @@ struct LatParams {
     }
     __device__ __forceinline__ void advance(const uint32_t* sm, uint32_t b, uint32_t& ent,
                                             unsigned long long& off) const {
-        const unsigned long long bbits = (unsigned long long) B * 32;
-        uint32_t idx = min(ent >> 8, L - 1);
-        unsigned long long pos = b * bbits + (ent & 0xffu);
-        while (pos < (b + 1) * bbits) {
-            const uint32_t e = sm[idx];
-            const unsigned long long u = pos >> 5;
-            const uint32_t w0 = u < n_units ? __ldg(units + u) : 0u;
-            const uint32_t w1 = u + 1 < n_units ? __ldg(units + u + 1) : 0u;
-            const uint32_t bits = __funnelshift_r(w0, w1, (uint32_t) pos & 31u);
-            idx = min((e >> 18) + (bits & ((1u << (e & 31u)) - 1u)), L - 1);
-            pos += e & 31u;
-            off += (e >> 8) & 255u;
+        const auto unit = [&](unsigned long long u) { return u < n_units ? __ldg(units + u) : 0u; };
+        uint32_t idx = min(ent >> 8, L - 1), pos = ent & 0xffu;
+        unsigned long long u = (unsigned long long) b * B + (pos >> 5);
+        uint32_t w0 = unit(u), w1 = unit(u + 1), w2 = unit(u + 2), n = 0;
+        while (pos < B * 32) {
+            const uint32_t e = sm[idx], k = e & 31u;
+            idx = min((e >> 18) + (__funnelshift_r(w0, w1, pos) & ((1u << k) - 1u)), L - 1);
+            n += (e >> 8) & 255u;
+            if (((pos + k) ^ pos) & 32u) {
+                ++u;
+                w0 = w1;
+                w1 = w2;
+                w2 = unit(u + 2);
+            }
+            pos += k;
         }
-        ent = (uint32_t) (pos - (b + 1) * bbits) | (idx << 8);
+        off += n;
+        ent = (pos - B * 32) | (idx << 8);
     }
 };
 
@@ -226,9 +230,9 @@ struct LatCursor {
     uint32_t w0, w1;     // shifted units under the cursor
     uint32_t pos;
 
-    // One step; `mask` = (slots - 1) * 128.  Returns the entry stepped over.
+    // One step; `mask` = (slots - 1) * 32.  Returns the entry stepped over.
     __device__ __forceinline__ uint32_t step(uint32_t col, uint32_t mask) {
-        const uint32_t u = lds32(col | ((pos << 2) & mask));
+        const uint32_t u = lds32(col + ((pos & mask) << 2));
         const uint32_t y = e;
         const uint32_t b4 = __funnelshift_r(w0, w1, pos) & lat_mask4(y);
         a = (y >> 16) + b4;
@@ -262,7 +266,7 @@ struct LatMid {
 // against 4.5 for single steps, 47 against 47.5 alone.
 __device__ __forceinline__ void lat_pair(LatCursor& c, uint32_t col, uint32_t mask, uint32_t& y1,
                                          uint32_t& y2, LatMid& m) {
-    m.u = lds32(col | ((c.pos << 2) & mask));
+    m.u = lds32(col + ((c.pos & mask) << 2));
     m.w0 = c.w0;
     m.w1 = c.w1;
     m.base = c.pos;
@@ -357,15 +361,19 @@ __device__ __forceinline__ void lat_store_units(const uint32_t (&r)[kB], uint32_
 }
 
 // Shared memory of a sync-pass CTA: the table, then per warp a ring of two
-// blocks for every lane, aligned to its size (at most 8 KB).
+// blocks for every lane.
 __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B * 128; }
 
 // One lane per trajectory, persistent: a lane whose trajectory ended takes
-// the next start.  Bound by the longest trajectory's chain of lookups on
+// the next start, and when there are none left the trajectories of a CTA
+// close up into fewer warps (128 MB at 1.5 bits per symbol, L = 4096: sync
+// pass 990 -> 893 us; 256 threads a CTA instead of 128: 16 MB 91 -> 106, a
+// batch 579 -> 683).  Bound by the longest trajectory's chain of lookups on
 // short streams (57 cycles a step with the block's bookkeeping, 47 for the
 // loop alone, against 62 to 83 for the 8-byte entries and a test per step)
-// and by the shared-memory lookups (4.5 cycles a warp and step) once 16
-// warps run on every SM.  The slots of the next block and the units of the
+// and by the L1 data pipe (4.0 passes a warp and step for the lookups, about
+// two more for the lanes' own loads of units and slots) once 16 warps run
+// on every SM.  The slots of the next block and the units of the
 // one after it are loaded, and a slot is claimed, a block's decode before
 // they are needed, which hides their round trips (about 1500 cycles a block
 // when they were waited for).
@@ -373,15 +381,19 @@ __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B
 template <uint32_t kB>
 __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next, uint32_t limit) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
+    __shared__ uint32_t s_live[kLatThreads / 32];
+    static_assert(kLatThreads * 28 <= (kLatThreads / 32) * lat_ring_bytes(kB), "states fit the rings");
     const uint32_t st = *(volatile uint32_t*) p.status;
     if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_DEGENERATE)) return;
     const uint32_t tb = smem_addr(lat_sm);
     lat_load_table(tb, p.tab_cnt, p.L);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t kRing = lat_ring_bytes(kB);
-    constexpr uint32_t kMask = kRing - 128;          // unit slots of the ring
+    constexpr uint32_t kSlots = 2 * kB;              // unit slots of a lane's ring
+    constexpr uint32_t kMask = (kSlots - 1) * 32;
     constexpr uint32_t kBits = kB * 32;
-    const uint32_t col = ((tb + p.L * 4 + kRing - 1) & ~(kRing - 1)) + warp * kRing + lane * 4;
+    const uint32_t rings = tb + ((p.L * 4 + 15) & ~15u);
+    const uint32_t col = rings + warp * kRing + lane * 4;
     const uint32_t D = p.D;
     const bool wide = ((uintptr_t) p.units & 31) == 0;
 
@@ -396,6 +408,32 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     bool has_prev = false, first = false;   // first: the true start's trajectory
     uint32_t carry = 0, life = 0, max_life = 0, visits = 0;
     uint32_t nx[kB];            // units of block b + 2, in flight
+    uint32_t room = blockDim.x; // lanes the CTA's trajectories are spread over
+
+    // the cursor at entry `val` of block b
+    const auto begin = [&]() {
+        const uint32_t rel = val & 0xffu, s = (b & 1u) * kB;
+        carry = 0;
+        if (kB <= 16) {   // both blocks' loads in flight together
+            uint32_t r0[kB];
+            lat_load_units<kB>(r0, p.units, p.n_units, b, wide);
+            lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
+            lat_store_units<kB>(r0, col, s, carry);
+        } else {
+            lat_load_units<kB>(nx, p.units, p.n_units, b, wide);
+            lat_store_units<kB>(nx, col, s, carry);
+            lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
+        }
+        lat_store_units<kB>(nx, col, s ^ kB, carry);
+        lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
+        c.pos = s * 32 + rel + 64;
+        be = s * 32 + kBits + 64;
+        const uint32_t u0 = s + (rel >> 5);
+        c.w0 = lds32(col + (u0 & (kSlots - 1)) * 128);
+        c.w1 = lds32(col + ((u0 + 1) & (kSlots - 1)) * 128);
+        c.a = tb + 4 * ((val >> 8) & (kMaxStates - 1));
+        c.e = lds32(c.a);
+    };
 
     for (;;) {
         const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
@@ -409,8 +447,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                 on = true;
                 b = k * p.nb;
                 first = k == 0;
-                const uint32_t rel = first ? p.first_pos : 0u;
-                val = kLatKeyUsed | rel | (p.first_idx << 8);
+                val = kLatKeyUsed | (first ? p.first_pos : 0u) | (p.first_idx << 8);
                 // the start's own node; a trajectory that came by with the
                 // same entry carries on instead
                 if (first) {
@@ -424,28 +461,51 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                 cas = 0;
                 has_prev = false;
                 life = 0;
-                if (on) {
-                    carry = 0;
-                    uint32_t r0[kB];
-                    lat_load_units<kB>(r0, p.units, p.n_units, b, wide);
-                    lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
-                    const uint32_t s = (b & 1u) * kB;
-                    lat_store_units<kB>(r0, col, s, carry);
-                    lat_store_units<kB>(nx, col, s ^ kB, carry);
-                    lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
-                    c.pos = s * 32 + rel + 64;
-                    be = s * 32 + kBits + 64;
-                    const uint32_t u0 = s + (rel >> 5);
-                    c.w0 = lds32(col | ((u0 * 128) & kMask));
-                    c.w1 = lds32(col | (((u0 + 1) * 128) & kMask));
-                    c.a = tb + 4 * p.first_idx;
-                    c.e = lds32(c.a);
-                }
+                if (on) begin();
             }
         }
-        if (!__any_sync(0xffffffffu, on)) {
-            if (exhausted) break;
+        const uint32_t n = __syncthreads_count(on);
+        if (n == 0) {
+            if (__syncthreads_and(exhausted)) break;
             continue;
+        }
+        // No starts left and half the lanes idle: the trajectories move
+        // together, into the CTA's first warps (a state is seven words; the
+        // units are staged again).  Without it two lanes of three idle.
+        if (2 * n <= room && room > 32 && p.width == 32 && __syncthreads_and(exhausted)) {
+            const uint32_t live = __ballot_sync(0xffffffffu, on);
+            if (lane == 0) s_live[warp] = __popc(live);
+            __syncthreads();
+            uint32_t r = __popc(live & ((1u << lane) - 1));
+            for (uint32_t w = 0; w < warp; ++w) r += s_live[w];
+            if (on) {
+                const uint32_t x = rings + r * 28;   // nobody reads the units any more
+                sts32(x, b);
+                sts32(x + 4, val);
+                sts32(x + 8, cas);
+                sts32(x + 12, prev);
+                sts32(x + 16, pcnt);
+                sts32(x + 20, q | (first ? 16u : 0u) | (has_prev ? 32u : 0u));
+                sts32(x + 24, life);
+            }
+            __syncthreads();
+            on = threadIdx.x < n;
+            if (on) {
+                const uint32_t x = rings + threadIdx.x * 28;
+                b = lds32(x);
+                val = lds32(x + 4);
+                cas = lds32(x + 8);
+                prev = lds32(x + 12);
+                pcnt = lds32(x + 16);
+                const uint32_t f = lds32(x + 20);
+                q = f & 15u;
+                first = (f & 16u) != 0;
+                has_prev = (f & 32u) != 0;
+                life = lds32(x + 24);
+            }
+            __syncthreads();
+            if (on) begin();
+            room = (n + 31) & ~31u;
         }
         if (!on) continue;
         // the slots of block b + 1 as they are now, in flight under the decode
@@ -530,7 +590,7 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
                                                uint32_t stage_addr, uint32_t g) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     const uint32_t lane = threadIdx.x & 31;
-    constexpr uint32_t kMask = (lat_tile_slots(kB) - 1) * 128;
+    constexpr uint32_t kMask = (lat_tile_slots(kB) - 1) * 32;
     const uint32_t b0 = g << 5, b = b0 + lane;
     const bool have = b < p.nblk;
     const unsigned long long start = have ? __ldg(p.start + b) : 0ull;
@@ -657,8 +717,7 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     return true;
 }
 
-// Shared memory of a final-pass CTA: table, unit tiles (aligned to their
-// size), staging buffers.
+// Shared memory of a final-pass CTA: table, unit tiles, staging buffers.
 __host__ __device__ constexpr uint32_t lat_final_warp_bytes(uint32_t B) {
     return lat_tile_slots(B) * 128;
 }
@@ -681,7 +740,7 @@ __device__ __forceinline__ void lat_final_body(const LatParams& p, uint32_t cta,
     lat_load_table(tb, p.tab_sym, p.L);
     const uint32_t warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     constexpr uint32_t kTile = lat_final_warp_bytes(kB);
-    const uint32_t tiles = (tb + p.L * 4 + kTile - 1) & ~(kTile - 1);
+    const uint32_t tiles = tb + ((p.L * 4 + 15) & ~15u);
     const uint32_t stage = tiles + nwarp * kTile + warp * (p.stage_cap + 16);
     const uint32_t groups = (p.nblk + 31) >> 5;
     for (uint32_t g = cta * nwarp + warp; g < groups; g += nctas * nwarp)

@@ -25,6 +25,9 @@ struct LatPlan {
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out);
 
+// Workspace of a lattice of nblk blocks with all slots.
+size_t lat_bytes(size_t nblk);
+
 struct LatCall {
     const uint32_t* units;
     size_t n_units;

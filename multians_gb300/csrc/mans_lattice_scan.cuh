@@ -307,8 +307,16 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
                 if (x + 1 < p.nblk) p.advance(lat_repair_sm, x, e, n);
                 s_over[x - first].y = (uint32_t) n;
                 if (++x >= stop) break;
-                for (uint32_t q = 0; q < kD; ++q)
-                    if (__ldg(p.key + (size_t) x * kD + q) == (e | kLatKeyUsed)) slot = q;
+                const uint4* keys = reinterpret_cast<const uint4*>(p.key + (size_t) x * kD);
+                const uint32_t want = e | kLatKeyUsed;
+#pragma unroll
+                for (uint32_t w = 0; w < kD / 4; ++w) {
+                    const uint4 k = __ldg(keys + w);
+                    if (k.x == want) slot = 4 * w;
+                    if (k.y == want) slot = 4 * w + 1;
+                    if (k.z == want) slot = 4 * w + 2;
+                    if (k.w == want) slot = 4 * w + 3;
+                }
                 if (slot != kLatDead) break;
             }
             const uint32_t used = atomicAdd(p.ctr + kLatRepaired, x - b) + (x - b);
