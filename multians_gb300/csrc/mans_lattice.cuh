@@ -568,11 +568,53 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
 // ---------------------------------------------------------------------------
 // final pass
 
-// Unit slots of a lane's tile in the final pass, a power of two (the cursor
-// masks its slot): the block and four units of look-ahead; with blocks of 32
-// units the look-ahead takes the first slots once the cursor has left them.
-__host__ __device__ constexpr uint32_t lat_tile_slots(uint32_t B) {
-    return B == 4 ? 8 : (B == 32 ? 32 : 2 * B);
+// Units of a warp's 32 blocks in the final pass.  The blocks are one contiguous
+// range: it comes in coalesced, as rows of a block each (cp.async of 16 bytes;
+// a row loaded by its own lane costs an L1 pass per lane and load: 256 MB at
+// 6 bits per symbol 231 -> 217 us, 512 MB at 8.6 500 -> 458), and is then
+// turned in place into the cursor's columns (rows read as they are cost
+// conflicts as the lanes drift apart: 240 us).  The rows' distance lets lanes
+// read 16 bytes of their own row without conflicts; a column holds the block
+// and four units of look-ahead.
+__host__ __device__ constexpr uint32_t lat_row_words(uint32_t B) { return B == 4 ? 4 : B + 4; }
+__host__ __device__ constexpr uint32_t lat_final_warp_bytes(uint32_t B) {
+    return 4 * (32 * lat_row_words(B) + 4 > 32 * (B + 4) ? 32 * lat_row_words(B) + 4 : 32 * (B + 4));
+}
+
+// Starts the copy of the units of blocks b0 .. b0 + 31 and the four behind
+// them into the rows of `tile`, zero past the stream's end.  Streams are
+// 16-byte aligned.
+template <uint32_t kB>
+__device__ __forceinline__ void lat_fill_rows(uint32_t tile, const LatParams& p, uint32_t b0,
+                                              uint32_t lane) {
+    constexpr uint32_t kPer = kB / 4;   // chunks of four units a row
+    const uint64_t u0 = (uint64_t) b0 * kB;
+    const auto chunk = [&](uint32_t q) {
+        const uint64_t u = u0 + q * 4;
+        const uint32_t left = u < p.n_units ? (uint32_t) min((uint64_t) 4, p.n_units - u) : 0u;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     :: "r"(tile + (q / kPer) * (lat_row_words(kB) * 4) + (q % kPer) * 16),
+                        "l"(p.units + (left ? u : 0)), "r"(left * 4) : "memory");
+    };
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) chunk(i * 32 + lane);
+    if (lane == 0) chunk(32 * kPer);
+}
+
+// Rows to columns, once the copies have landed.
+template <uint32_t kB>
+__device__ __forceinline__ void lat_turn_rows(uint32_t tile, uint32_t lane) {
+    constexpr uint32_t kRow = lat_row_words(kB) * 4;
+    uint32_t r[kB + 4], carry = 0;
+    const uint32_t row = tile + lane * kRow;
+#pragma unroll
+    for (uint32_t i = 0; i < kB + 4; i += 4)
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3])
+                     : "r"(i < kB ? row + i * 4 : row + kRow) : "memory");
+    __syncwarp();
+    lat_store_units<kB + 4>(r, tile + lane * 4, 0, carry);
+    __syncwarp();
 }
 
 __device__ __forceinline__ void lat_sts8(uint32_t a, uint32_t v) {
@@ -587,32 +629,19 @@ __device__ __forceinline__ void lat_sts8(uint32_t a, uint32_t v) {
 // stores (a range that does not fit is written byte by byte).
 template <bool kRev, uint32_t kB>
 __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, uint32_t tile,
-                                               uint32_t stage_addr, uint32_t g) {
+                                               uint32_t stage_addr, uint32_t g, uint32_t step) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     const uint32_t lane = threadIdx.x & 31;
-    constexpr uint32_t kMask = (lat_tile_slots(kB) - 1) * 32;
-    const uint32_t b0 = g << 5, b = b0 + lane;
+    constexpr uint32_t kMask = (2 * kB - 1) * 32;   // no slot wraps
+    const uint32_t b0 = g << 5, b = b0 + lane, col = tile + lane * 4;
     const bool have = b < p.nblk;
+    lat_fill_rows<kB>(tile, p, b0, lane);
     const unsigned long long start = have ? __ldg(p.start + b) : 0ull;
     const uint32_t ent = (uint32_t) start & ((1u << kLatEntBits) - 1);
     const unsigned long long off = start >> kLatEntBits;
     unsigned long long off_nx = max((unsigned long long) p.n_out, off);
     const unsigned long long from_next = __shfl_down_sync(0xffffffffu, off, 1);
     if (b + 1 < p.nblk) off_nx = lane < 31 ? from_next : __ldg(p.start + b + 1) >> kLatEntBits;
-    // units: the block's and four more (zero past the end)
-    const uint32_t col = tile + lane * 4;
-    uint32_t ahead[4] = {0, 0, 0, 0}, carry = 0;
-    if (have) {
-        const bool wide = ((uintptr_t) p.units & 31) == 0;
-        uint32_t r[kB];
-        lat_load_units<kB>(r, p.units, p.n_units, b, wide);
-        lat_load_units<4>(ahead, p.units, p.n_units, (b + 1) * (kB / 4), false);
-        lat_store_units<kB>(r, col, 0, carry);
-        if (kB < 32) lat_store_units<4>(ahead, col, kB, carry);
-    }
-    const auto look_ahead = [&]() {
-        if (kB == 32) lat_store_units<4>(ahead, col, 0, carry);
-    };
     const unsigned long long off0 = __shfl_sync(0xffffffffu, off, 0);
     const uint32_t last_lane = min(31u, p.nblk - 1 - b0);
     const unsigned long long off_end = __shfl_sync(0xffffffffu, off_nx, last_lane);
@@ -624,6 +653,7 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     const uint32_t sb = (uint32_t) (((uintptr_t) p.out + wlo) & 15u);
     const bool staged = whi - wlo + sb <= p.stage_cap;
     const bool lane_ok = !have || (off >= off0 && max(off_nx, off) <= max(off_end, off0));
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (__any_sync(0xffffffffu, !lane_ok)) {
         if (lane == 0) atomicOr(p.status, MANS_DEV_COUNT_MISMATCH);
         return false;
@@ -633,6 +663,16 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     // than L codewords
     const unsigned long long cap_sym = (unsigned long long) (kB * 32 + 17) * p.L;
     const uint32_t cnt = have && off < end ? (uint32_t) min(end - off, cap_sym) : 0u;
+    __syncwarp();
+    lat_turn_rows<kB>(tile, lane);
+    // the next group's units and starts on their way into L2 meanwhile
+    // (16 warps an SM don't cover the copy's latency: 217 -> 211 us)
+    if ((uint64_t) b + step * 32 < p.nblk) {
+        const uint32_t nx = b + step * 32;
+        if (kB == 32 || (lane & (32 / kB - 1)) == 0)
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(p.units + (uint64_t) nx * kB));
+        if ((lane & 15) == 0) asm volatile("prefetch.global.L2 [%0];" :: "l"(p.start + nx));
+    }
     if (have) {
         LatCursor c;
         const uint32_t rel = ent & 0xffu;
@@ -642,8 +682,6 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
         c.w0 = lds32(col + (rel >> 5) * 128);
         c.w1 = lds32(col + ((rel >> 5) + 1) * 128);
         const uint32_t pos_cap = kB * 32 + kMaxBits + 1 + 64;
-        // past this position the first slots are free (kB = 32)
-        const uint32_t pos_half = kB == 32 ? 64 + 16 * 32 : pos_cap;
         LatMid m;
         const uint32_t full = off_nx >= off ? (uint32_t) min(off_nx - off, 0xffffffffull) : 0u;
         uint32_t i = 0;
@@ -651,48 +689,30 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
             uint32_t q = stage_addr + sb + (uint32_t) (off - wlo);
             for (; i < cnt && (q & 3u) && c.pos < pos_cap; ++i, ++q)
                 lat_sts8(q, c.step(col, kMask) >> 8);
-            const auto four = [&](uint32_t limit) {
-                for (; i + 4 <= cnt && c.pos < limit; i += 4, q += 4) {
-                    uint32_t y0, y1, y2, y3;
-                    lat_pair(c, col, kMask, y0, y1, m);
-                    lat_pair(c, col, kMask, y2, y3, m);
-                    sts32(q, __byte_perm(__byte_perm(y0, y1, 0x0051), __byte_perm(y2, y3, 0x5100), 0x7610));
-                }
-            };
-            if (kB == 32) {
-                four(pos_half);
-                look_ahead();
+            for (; i + 4 <= cnt && c.pos < pos_cap; i += 4, q += 4) {
+                uint32_t y0, y1, y2, y3;
+                lat_pair(c, col, kMask, y0, y1, m);
+                lat_pair(c, col, kMask, y2, y3, m);
+                sts32(q, __byte_perm(__byte_perm(y0, y1, 0x0051), __byte_perm(y2, y3, 0x5100), 0x7610));
             }
-            four(pos_cap);
             for (; i < cnt && c.pos < pos_cap; ++i, ++q) lat_sts8(q, c.step(col, kMask) >> 8);
         } else if (staged) {
             // decode index i goes to output n_out - 1 - i: downwards
             uint32_t q = stage_addr + sb + (uint32_t) (p.n_out - 1 - off - wlo);
             for (; i < cnt && (q & 3u) != 3u && c.pos < pos_cap; ++i, --q)
                 lat_sts8(q, c.step(col, kMask) >> 8);
-            const auto four = [&](uint32_t limit) {
-                for (; i + 4 <= cnt && c.pos < limit; i += 4, q -= 4) {
-                    uint32_t y0, y1, y2, y3;
-                    lat_pair(c, col, kMask, y0, y1, m);
-                    lat_pair(c, col, kMask, y2, y3, m);
-                    sts32(q - 3, __byte_perm(__byte_perm(y3, y2, 0x0051), __byte_perm(y1, y0, 0x5100), 0x7610));
-                }
-            };
-            if (kB == 32) {
-                four(pos_half);
-                look_ahead();
+            for (; i + 4 <= cnt && c.pos < pos_cap; i += 4, q -= 4) {
+                uint32_t y0, y1, y2, y3;
+                lat_pair(c, col, kMask, y0, y1, m);
+                lat_pair(c, col, kMask, y2, y3, m);
+                sts32(q - 3, __byte_perm(__byte_perm(y3, y2, 0x0051), __byte_perm(y1, y0, 0x5100), 0x7610));
             }
-            four(pos_cap);
             for (; i < cnt && c.pos < pos_cap; ++i, --q) lat_sts8(q, c.step(col, kMask) >> 8);
         } else if (!kRev) {
             uint8_t* dst = p.out + off;
-            for (; i < cnt && c.pos < pos_half; ++i) dst[i] = (uint8_t) (c.step(col, kMask) >> 8);
-            look_ahead();
             for (; i < cnt && c.pos < pos_cap; ++i) dst[i] = (uint8_t) (c.step(col, kMask) >> 8);
         } else {
             uint8_t* dst = p.out + (p.n_out - 1 - off);
-            for (; i < cnt && c.pos < pos_half; ++i) *(dst - i) = (uint8_t) (c.step(col, kMask) >> 8);
-            look_ahead();
             for (; i < cnt && c.pos < pos_cap; ++i) *(dst - i) = (uint8_t) (c.step(col, kMask) >> 8);
         }
         // a block decoded to its full count ends at the next block start
@@ -718,10 +738,6 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
 }
 
 // Shared memory of a final-pass CTA: table, unit tiles, staging buffers.
-__host__ __device__ constexpr uint32_t lat_final_warp_bytes(uint32_t B) {
-    return lat_tile_slots(B) * 128;
-}
-
 template <bool kRev, uint32_t kB>
 __device__ __forceinline__ void lat_final_body(const LatParams& p, uint32_t cta, uint32_t nctas) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
@@ -744,7 +760,7 @@ __device__ __forceinline__ void lat_final_body(const LatParams& p, uint32_t cta,
     const uint32_t stage = tiles + nwarp * kTile + warp * (p.stage_cap + 16);
     const uint32_t groups = (p.nblk + 31) >> 5;
     for (uint32_t g = cta * nwarp + warp; g < groups; g += nctas * nwarp)
-        if (!lat_final_warp<kRev, kB>(p, tb, tiles + warp * kTile, stage, g)) return;
+        if (!lat_final_warp<kRev, kB>(p, tb, tiles + warp * kTile, stage, g, nctas * nwarp)) return;
 }
 
 }  // namespace mans
