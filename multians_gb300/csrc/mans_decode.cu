@@ -3182,7 +3182,7 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
     uint64_t seeds = 0;
     for (const BatchStreamPlan& sp : plans)
         if (sp.active && sp.lattice) seeds += sp.lat.nseed;
-    lay.lat_width = seeds <= 8ull * 4 * 152 ? 8 : (seeds <= 16ull * 4 * 152 ? 16 : 32);
+    lay.lat_width = lat_width(seeds, 152);
     const uint32_t per_cta = kLatBatchWarps * lay.lat_width;
     for (uint32_t i = 0; i < n; ++i)
         if (plans[i].active && plans[i].lattice)
@@ -3488,7 +3488,7 @@ int mans_batch_decode(mans_batch* b, void* stream) {
         if (L.n_sync_c[c])
             k_gwalk_batch<<<(unsigned) L.n_sync_c[c], kSyncThreads, L.smem_sync_c[c], st>>>(
                 ps, items + at);
-    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, st);
+    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, L.lat_width, st);
     litems += L.n_lsync;
     timing_mark(2, st);
     if (L.n_walk) {

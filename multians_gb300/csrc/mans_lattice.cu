@@ -21,9 +21,9 @@ __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep(LatParams p, uint4
         zero[i] = make_uint4(0, 0, 0, 0);
 }
 
-template <uint32_t kB>
+template <uint32_t kB, bool kNarrow>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
-    lat_sync_body<kB>(p, p.ctr + kLatNext, p.nseed);
+    lat_sync_body<kB, kNarrow>(p, p.ctr + kLatNext, p.nseed);
 }
 
 template <uint32_t kD>
@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep_batch(const LatPar
 }
 
 // index: the CTA's first start, count: the end of its starts.
+template <bool kNarrow>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams* ps,
                                                                 const LatItem* items) {
     __shared__ LatParams sp;
@@ -77,10 +78,10 @@ __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams*
     const LatItem it = items[blockIdx.x];
     if (threadIdx.x == 0) s_next = it.index;
     lat_load_params(sp, ps + it.stream);
-    if (sp.B == 4) lat_sync_body<4>(sp, &s_next, it.count);
-    else if (sp.B == 8) lat_sync_body<8>(sp, &s_next, it.count);
-    else if (sp.B == 16) lat_sync_body<16>(sp, &s_next, it.count);
-    else lat_sync_body<32>(sp, &s_next, it.count);
+    if (sp.B == 4) lat_sync_body<4, kNarrow>(sp, &s_next, it.count);
+    else if (sp.B == 8) lat_sync_body<8, kNarrow>(sp, &s_next, it.count);
+    else if (sp.B == 16) lat_sync_body<16, kNarrow>(sp, &s_next, it.count);
+    else lat_sync_body<32, kNarrow>(sp, &s_next, it.count);
 }
 
 // The ticket hands items out in list order, which holds each stream's tiles
@@ -175,6 +176,13 @@ int sm_count() {
     return std::max(sms, 1);
 }
 
+template <bool kNarrow>
+void (*sync_kernel(uint32_t B))(LatParams) {
+    return B == 4 ? k_lat_sync<4, kNarrow>
+                  : (B == 8 ? k_lat_sync<8, kNarrow>
+                            : (B == 16 ? k_lat_sync<16, kNarrow> : k_lat_sync<32, kNarrow>));
+}
+
 // Opts the kernels in to large dynamic shared memory, once per device.
 void lat_attributes() {
     static std::mutex mu;
@@ -187,8 +195,12 @@ void lat_attributes() {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int) kLatFinalSmemMax);
     };
-    set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_sync_batch); set(k_lat_final_batch);
-    set(k_lat_sync<4>); set(k_lat_sync<8>); set(k_lat_sync<16>); set(k_lat_sync<32>);
+    set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_final_batch);
+    set(k_lat_sync_batch<false>); set(k_lat_sync_batch<true>);
+    for (uint32_t B = 4; B <= 32; B *= 2) {
+        set(sync_kernel<false>(B));
+        set(sync_kernel<true>(B));
+    }
     set(k_lat_final<false, 4>); set(k_lat_final<false, 8>); set(k_lat_final<false, 16>);
     set(k_lat_final<false, 32>); set(k_lat_final<true, 32>);
     set(k_lat_final<true, 4>); set(k_lat_final<true, 8>); set(k_lat_final<true, 16>);
@@ -233,6 +245,17 @@ LatParams lat_params(const LatCall& call, const LatPlan& plan, char* base) {
 }
 
 }  // namespace
+
+uint32_t lat_width(uint64_t starts, uint32_t sms) {
+    // A warp waits for the slowest of its trajectories at every block, so with
+    // few of them each gets a warp (219 KB at 0.7 bits per symbol, L = 4096: 8
+    // lanes 277 us, 1 lane 253), and the CTA's barrier goes (48 streams: 400
+    // -> 393 us).  Past 16 warps an SM wider ones are as fast (16 lanes: 1.2
+    // MB 52 us either way).
+    uint32_t w = 1;
+    while (w <= 8 && starts > w * 16ull * sms) w *= 2;
+    return w <= 8 ? w : 32;
+}
 
 size_t lat_bytes(size_t nblk) { return lat_layout(nblk, kLatSlotsMax, kMaxStates).total; }
 
@@ -295,20 +318,13 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     mark(1, st);
     // sync pass
     {
-        // few trajectories: narrow warps spread over the schedulers of all SMs
-        uint32_t th = kLatThreads, width = 32;
-        const uint32_t sched = 4u * sms;
-        if (plan.nseed <= 8 * sched) width = 8;
-        else if (plan.nseed <= 16 * sched) width = 16;
-        if (plan.nseed <= width * sched) th = 32;
+        const uint32_t width = lat_width(plan.nseed, sms);
+        const uint32_t th = plan.nseed <= width * 4 * sms ? 32 : kLatThreads;
         p.width = width;
         const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
         const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
         const size_t sm = lat_sync_smem(call.L, plan.B, th);
-        if (plan.B == 4) k_lat_sync<4><<<grid, th, sm, st>>>(p);
-        else if (plan.B == 8) k_lat_sync<8><<<grid, th, sm, st>>>(p);
-        else if (plan.B == 16) k_lat_sync<16><<<grid, th, sm, st>>>(p);
-        else k_lat_sync<32><<<grid, th, sm, st>>>(p);
+        (width < 32 ? sync_kernel<true>(plan.B) : sync_kernel<false>(plan.B))<<<grid, th, sm, st>>>(p);
     }
     mark(2, st);
     mark(3, st);
@@ -393,8 +409,9 @@ void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSme
     if (n) k_lat_prep_batch<<<(unsigned) n, kLatPrepThreads, sm.prep, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    cudaStream_t st) {
-    if (n) k_lat_sync_batch<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
+                    uint32_t width, cudaStream_t st) {
+    auto* k = width < 32 ? k_lat_sync_batch<true> : k_lat_sync_batch<false>;
+    if (n) k<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
                     uint32_t* ticket, cudaStream_t st) {

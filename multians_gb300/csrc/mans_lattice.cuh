@@ -377,8 +377,13 @@ __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B
 // one after it are loaded, and a slot is claimed, a block's decode before
 // they are needed, which hides their round trips (about 1500 cycles a block
 // when they were waited for).
-// Starts are taken from the counter `next`, up to `limit`.
-template <uint32_t kB>
+// Starts are taken from the counter `next`, up to `limit`.  kNarrow: warps of
+// which only p.width lanes run, on inputs with few trajectories; no CTA
+// barriers then, and twice the slots are looked at ahead (a block with more
+// than three trajectories costs two exposed round trips otherwise: 146 KB at
+// 3.1 bits per symbol, L = 4096, 316 -> 290 us, 128 KB at 3.8 79 -> 67; all
+// sixteen looked at: 321 and 73; wide warps: a batch 579 -> 594).
+template <uint32_t kB, bool kNarrow>
 __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next, uint32_t limit) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     __shared__ uint32_t s_live[kLatThreads / 32];
@@ -392,6 +397,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     constexpr uint32_t kSlots = 2 * kB;              // unit slots of a lane's ring
     constexpr uint32_t kMask = (kSlots - 1) * 32;
     constexpr uint32_t kBits = kB * 32;
+    constexpr uint32_t kV = kNarrow ? 2 : 1;         // groups of four slots seen ahead
     const uint32_t rings = tb + ((p.L * 4 + 15) & ~15u);
     const uint32_t col = rings + warp * kRing + lane * 4;
     const uint32_t D = p.D;
@@ -435,44 +441,13 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         c.e = lds32(c.a);
     };
 
-    for (;;) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
-        if (!exhausted && __popc(idle) >= min(p.width, 8u)) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(next, (uint32_t) __popc(idle));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            exhausted = base + __popc(idle) >= limit;
-            const uint32_t k = base + __popc(idle & ((1u << lane) - 1));
-            if (!on && lane < p.width && k < limit) {
-                on = true;
-                b = k * p.nb;
-                first = k == 0;
-                val = kLatKeyUsed | (first ? p.first_pos : 0u) | (p.first_idx << 8);
-                // the start's own node; a trajectory that came by with the
-                // same entry carries on instead
-                if (first) {
-                    q = 0;
-                    p.key[0] = val;
-                } else {
-                    bool found;
-                    q = lat_take(p.key + (size_t) b * D, 1, D, val, found);
-                    if (found || q == kLatDead) on = false;
-                }
-                cas = 0;
-                has_prev = false;
-                life = 0;
-                if (on) begin();
-            }
-        }
+    // The CTA's trajectories, false if none is left.
+    // No starts left and half the lanes idle: the trajectories move
+    // together, into the CTA's first warps (a state is seven words; the
+    // units are staged again).  Without it two lanes of three idle.
+    const auto close_up = [&]() -> bool {
         const uint32_t n = __syncthreads_count(on);
-        if (n == 0) {
-            if (__syncthreads_and(exhausted)) break;
-            continue;
-        }
-        // No starts left and half the lanes idle: the trajectories move
-        // together, into the CTA's first warps (a state is seven words; the
-        // units are staged again).  Without it two lanes of three idle.
-        if (2 * n <= room && room > 32 && p.width == 32 && __syncthreads_and(exhausted)) {
+        if (n != 0 && 2 * n <= room && room > 32 && __syncthreads_and(exhausted)) {
             const uint32_t live = __ballot_sync(0xffffffffu, on);
             if (lane == 0) s_live[warp] = __popc(live);
             __syncthreads();
@@ -507,12 +482,57 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
             if (on) begin();
             room = (n + 31) & ~31u;
         }
+        return n != 0;
+    };
+
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
+        if (!exhausted && __popc(idle) >= min(p.width, 8u)) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(next, (uint32_t) __popc(idle));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            exhausted = base + __popc(idle) >= limit;
+            const uint32_t k = base + __popc(idle & ((1u << lane) - 1));
+            if (!on && lane < p.width && k < limit) {
+                on = true;
+                b = k * p.nb;
+                first = k == 0;
+                val = kLatKeyUsed | (first ? p.first_pos : 0u) | (p.first_idx << 8);
+                // the start's own node; a trajectory that came by with the
+                // same entry carries on instead
+                if (first) {
+                    q = 0;
+                    p.key[0] = val;
+                } else {
+                    bool found;
+                    q = lat_take(p.key + (size_t) b * D, 1, D, val, found);
+                    if (found || q == kLatDead) on = false;
+                }
+                cas = 0;
+                has_prev = false;
+                life = 0;
+                if (on) begin();
+            }
+        }
+        if (kNarrow) {
+            if (!__any_sync(0xffffffffu, on)) {
+                if (exhausted) break;
+                continue;
+            }
+        } else if (!close_up()) {
+            if (__syncthreads_and(exhausted)) break;
+            continue;
+        }
         if (!on) continue;
         // the slots of block b + 1 as they are now, in flight under the decode
-        uint4 kn = make_uint4(0, 0, 0, 0);
+        uint4 kn[kV];
         const bool more = b + 1 < p.nblk;
         uint32_t* const knext = p.key + (size_t) (b + 1) * D;
-        if (more) kn = lat_ld_slots(knext);
+#pragma unroll
+        for (uint32_t g = 0; g < kV; ++g) {
+            kn[g] = make_uint4(1, 1, 1, 1);
+            if (more && g * 4 < D) kn[g] = lat_ld_slots(knext + g * 4);
+        }
         uint32_t cnt = 0;
         if ((int32_t) (be - c.pos) > 0) lat_block(c, col, kMask, be, cnt);
         ++life;
@@ -534,11 +554,18 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         pcnt = cnt;
         // arrive at block b + 1
         val = kLatKeyUsed | (c.pos - be) | (((c.a - tb) << 6));
-        uint32_t hit = kLatDead;
-        if (kn.x == val) hit = 0;
-        if (kn.y == val) hit = 1;
-        if (kn.z == val) hit = 2;
-        if (kn.w == val) hit = 3;
+        uint32_t hit = kLatDead, open = kV * 4 - 1;
+#pragma unroll
+        for (uint32_t g = kV; g-- > 0;) {
+            if (kn[g].w == val) hit = 4 * g + 3;
+            if (kn[g].z == val) hit = 4 * g + 2;
+            if (kn[g].y == val) hit = 4 * g + 1;
+            if (kn[g].x == val) hit = 4 * g;
+            if (kn[g].w == 0) open = 4 * g + 3;
+            if (kn[g].z == 0) open = 4 * g + 2;
+            if (kn[g].y == 0) open = 4 * g + 1;
+            if (kn[g].x == 0 && g > 0) open = 4 * g;
+        }
         ++b;
         if (hit != kLatDead) {
             p.node[prev] = pcnt | (hit << 28);
@@ -548,8 +575,8 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
             continue;
         }
         // the true start's trajectory has slot 0 of every block to itself
-        q = first ? 0u : (kn.y == 0 ? 1u : (kn.z == 0 ? 2u : 3u));
-        cas = lat_cas(knext + q, val);
+        q = first ? 0u : min(open, kLatDead);
+        cas = q == kLatDead ? 0u : lat_cas(knext + q, val);
         // block b + 1 (one ahead again) into the half of the ring that is free
         const uint32_t s = (b & 1u) * kB;      // slots of block b
         lat_store_units<kB>(nx, col, s ^ kB, carry);

@@ -61,6 +61,10 @@ struct LatSmem {
 };
 constexpr uint32_t kLatBatchWarps = 4;   // of a sync-pass CTA
 
+// Lanes of a sync-pass warp that run trajectories: narrow warps while 16 of
+// them an SM hold every start.
+uint32_t lat_width(uint64_t starts, uint32_t sms);
+
 size_t lat_params_size();
 void lat_fill_params(void* dst, const LatCall& call, const LatPlan& plan, void* slice,
                      uint32_t* d_status, uint32_t width);
@@ -72,7 +76,7 @@ void lat_batch_init();
 void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
                     cudaStream_t st);
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    cudaStream_t st);
+                    uint32_t width, cudaStream_t st);
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
                     uint32_t* ticket, cudaStream_t st);
 void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st);
