@@ -554,7 +554,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         pcnt = cnt;
         // arrive at block b + 1
         val = kLatKeyUsed | (c.pos - be) | (((c.a - tb) << 6));
-        uint32_t hit = kLatDead, open = kV * 4 - 1;
+        uint32_t hit = kLatDead, open = min(kV * 4, D) - 1;
 #pragma unroll
         for (uint32_t g = kV; g-- > 0;) {
             if (kn[g].w == val) hit = 4 * g + 3;
