@@ -3025,6 +3025,7 @@ struct BatchLayout {
     size_t lat_params, lat_items, n_lat, n_lprep, n_lsync, n_lscan, n_lfinal_c[2];
     LatSmem lat_smem;         // of the streams that need most
     size_t lat_final_smem0;   // ... final pass, class 0
+    bool lat_deep;        // some stream has 32 slots a block
     uint32_t lat_width;   // lanes of a sync-pass warp that run trajectories
     size_t n_sync, n_walk, n_scan, n_final, n_items;
     bool any_capture;
@@ -3059,6 +3060,7 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
     size_t data = 0, flag_words = 0;
     lay.n_sync = lay.n_walk = lay.n_scan = lay.n_final = 0;
     lay.any_capture = false;
+    lay.lat_deep = false;
     for (int c = 0; c < 2; ++c)
         lay.n_sync_c[c] = lay.n_final_c[c] = lay.smem_sync_c[c] = lay.smem_final_c[c] = 0;
     lay.smem_sync = lay.smem_walk = lay.smem_final = lay.smem_prep = 0;
@@ -3143,6 +3145,7 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         const int cls = batch_class(d[i].L);
         if (sp.lattice) {
             ++lay.n_lat;
+            lay.lat_deep |= sp.lat.D > 16;
             lay.n_lprep += lat_prep_items(sp.lat);
             lay.n_lscan += lat_scan_tiles(sp.lat);
             const LatSmem s = lat_batch_smem(lat_call(d[i]), sp.lat);
@@ -3488,7 +3491,7 @@ int mans_batch_decode(mans_batch* b, void* stream) {
         if (L.n_sync_c[c])
             k_gwalk_batch<<<(unsigned) L.n_sync_c[c], kSyncThreads, L.smem_sync_c[c], st>>>(
                 ps, items + at);
-    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, L.lat_width, st);
+    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, L.lat_width, L.lat_deep, st);
     litems += L.n_lsync;
     timing_mark(2, st);
     if (L.n_walk) {
@@ -3503,7 +3506,7 @@ int mans_batch_decode(mans_batch* b, void* stream) {
     if (L.n_scan)
         k_scan_batch<<<(unsigned) L.n_scan, kScanThreads, 0, st>>>(
             ps, items + L.n_sync, (uint32_t*) (b->base + L.ticket));
-    lat_batch_scan(lps, litems, L.n_lscan, L.lat_smem, (uint32_t*) (b->base + L.ticket) + 3, st);
+    lat_batch_scan(lps, litems, L.n_lscan, L.lat_smem, L.lat_deep, (uint32_t*) (b->base + L.ticket) + 3, st);
     litems += L.n_lscan;
     timing_mark(4, st);
     if (L.n_final && L.any_capture)

@@ -48,6 +48,7 @@ namespace {
 constexpr uint32_t kEncThreads = 128;        // sync pass
 constexpr uint32_t kEncCtas = 3;             // per SM, of the persistent sync pass
 constexpr uint32_t kEncFinalThreads = 256;
+constexpr uint32_t kEncSlots = 16;           // a block
 constexpr uint32_t kEncSmallBytes = 1u << 20;
 
 struct EncResult {
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
                     p.key[0] = val;
                 } else {
                     bool found;
-                    q = lat_take(p.key + (size_t) b * D, 1, D, val, found);
+                    q = lat_take(p.key + (size_t) b * D, 1, lat_usable(kEncSlots), val, found);
                     if (found || q == kLatDead) on = false;
                 }
                 cas = 0;
@@ -300,9 +301,9 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
         bool found = false;
         if (cas != 0) {
             if (cas == val) found = true;
-            else q = lat_take(p.key + (size_t) b * D, q + 1, D, val, found);
+            else q = lat_take(p.key + (size_t) b * D, q + 1, lat_usable(kEncSlots), val, found);
         }
-        if (has_prev) p.node[prev] = pbits | (q << 28);
+        if (has_prev) p.node[prev] = pbits | (q << kLatNodeShift);
         if (found || q == kLatDead || !more) {
             if (!more && !found && q != kLatDead)
                 p.end[q] = {x, bits, x_in & ((1u << len) - 1u), len};
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
         if (kn.w == val) hit = 3;
         ++b;
         if (hit != kLatDead) {
-            p.node[prev] = pbits | (hit << 28);
+            p.node[prev] = pbits | (hit << kLatNodeShift);
             on = false;
             max_life = max(max_life, life);
             continue;
@@ -561,7 +562,7 @@ EncLayout enc_layout(const EncPlan& e) {
 EncPlan enc_plan(unsigned long long n, uint32_t L, uint32_t hint) {
     EncPlan e;
     e.Bs = n <= kEncSmallBytes && L <= 1024 ? 64 : 128;
-    e.D = kLatSlotsMax;
+    e.D = kEncSlots;
     const unsigned long long nblk = (n + e.Bs - 1) / e.Bs;
     const unsigned long long par = n / (152ull * 32 * 32);
     unsigned long long s = hint ? hint : std::max<unsigned long long>({par, L / 12, 128});
@@ -677,7 +678,7 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
         if (e.Bs == 64) k_enc_sync<64><<<grid, th, sm, st>>>(p);
         else k_enc_sync<128><<<grid, th, sm, st>>>(p);
     }
-    k_enc_scan<kLatSlotsMax><<<(e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
+    k_enc_scan<kEncSlots><<<(e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
                                lat_scan_smem(mans_encode_blob_words(L)), st>>>(p);
     {
         const unsigned groups = (e.nblk + 31) / 32;

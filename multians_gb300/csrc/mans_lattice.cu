@@ -21,13 +21,16 @@ __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep(LatParams p, uint4
         zero[i] = make_uint4(0, 0, 0, 0);
 }
 
-template <uint32_t kB, bool kNarrow>
+// Groups of four slots of the next block that a trajectory looks at ahead.
+constexpr uint32_t lat_ahead(uint32_t D, bool narrow) { return D > 16 ? 4 : (narrow ? 2 : 1); }
+
+template <uint32_t kB, bool kNarrow, uint32_t kV>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
-    lat_sync_body<kB, kNarrow>(p, p.ctr + kLatNext, p.nseed);
+    lat_sync_body<kB, kNarrow, kV>(p, p.ctr + kLatNext, p.nseed);
 }
 
 template <uint32_t kD>
-__global__ void __launch_bounds__(kLatScanThreads, 5) k_lat_scan(LatParams p) {
+__global__ void __launch_bounds__(kLatScanThreads, kD > 16 ? 2 : 5) k_lat_scan(LatParams p) {
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
@@ -69,8 +72,16 @@ __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep_batch(const LatPar
         z[i] = make_uint4(0, 0, 0, 0);
 }
 
+template <bool kNarrow, uint32_t kV>
+__device__ __forceinline__ void lat_sync_any(const LatParams& p, uint32_t* next, uint32_t limit) {
+    if (p.B == 4) lat_sync_body<4, kNarrow, kV>(p, next, limit);
+    else if (p.B == 8) lat_sync_body<8, kNarrow, kV>(p, next, limit);
+    else if (p.B == 16) lat_sync_body<16, kNarrow, kV>(p, next, limit);
+    else lat_sync_body<32, kNarrow, kV>(p, next, limit);
+}
+
 // index: the CTA's first start, count: the end of its starts.
-template <bool kNarrow>
+template <bool kNarrow, bool kDeep>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams* ps,
                                                                 const LatItem* items) {
     __shared__ LatParams sp;
@@ -78,14 +89,13 @@ __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams*
     const LatItem it = items[blockIdx.x];
     if (threadIdx.x == 0) s_next = it.index;
     lat_load_params(sp, ps + it.stream);
-    if (sp.B == 4) lat_sync_body<4, kNarrow>(sp, &s_next, it.count);
-    else if (sp.B == 8) lat_sync_body<8, kNarrow>(sp, &s_next, it.count);
-    else if (sp.B == 16) lat_sync_body<16, kNarrow>(sp, &s_next, it.count);
-    else lat_sync_body<32, kNarrow>(sp, &s_next, it.count);
+    if (kDeep && sp.D > 16) lat_sync_any<kNarrow, lat_ahead(32, kNarrow)>(sp, &s_next, it.count);
+    else lat_sync_any<kNarrow, lat_ahead(16, kNarrow)>(sp, &s_next, it.count);
 }
 
 // The ticket hands items out in list order, which holds each stream's tiles
 // in increasing order: a tile only waits on tiles that have started.
+template <bool kDeep>
 __global__ void __launch_bounds__(kLatScanThreads) k_lat_scan_batch(const LatParams* ps,
                                                                     const LatItem* items,
                                                                     uint32_t* ticket) {
@@ -95,7 +105,8 @@ __global__ void __launch_bounds__(kLatScanThreads) k_lat_scan_batch(const LatPar
     __syncthreads();
     const LatItem it = items[s_item];
     lat_load_params(sp, ps + it.stream);
-    if (sp.D == 4) lat_scan_body<LatParams, 4>(sp, it.index);
+    if (kDeep && sp.D == 32) lat_scan_body<LatParams, 32>(sp, it.index);
+    else if (sp.D == 4) lat_scan_body<LatParams, 4>(sp, it.index);
     else if (sp.D == 8) lat_scan_body<LatParams, 8>(sp, it.index);
     else if (sp.D == 12) lat_scan_body<LatParams, 12>(sp, it.index);
     else lat_scan_body<LatParams, 16>(sp, it.index);
@@ -176,11 +187,21 @@ int sm_count() {
     return std::max(sms, 1);
 }
 
-template <bool kNarrow>
+template <bool kNarrow, uint32_t kD>
 void (*sync_kernel(uint32_t B))(LatParams) {
-    return B == 4 ? k_lat_sync<4, kNarrow>
-                  : (B == 8 ? k_lat_sync<8, kNarrow>
-                            : (B == 16 ? k_lat_sync<16, kNarrow> : k_lat_sync<32, kNarrow>));
+    constexpr uint32_t kV = lat_ahead(kD, kNarrow);
+    return B == 4 ? k_lat_sync<4, kNarrow, kV>
+                  : (B == 8 ? k_lat_sync<8, kNarrow, kV>
+                            : (B == 16 ? k_lat_sync<16, kNarrow, kV> : k_lat_sync<32, kNarrow, kV>));
+}
+void (*sync_kernel(uint32_t B, uint32_t D, bool narrow))(LatParams) {
+    return D > 16 ? (narrow ? sync_kernel<true, 32>(B) : sync_kernel<false, 32>(B))
+                  : (narrow ? sync_kernel<true, 16>(B) : sync_kernel<false, 16>(B));
+}
+
+auto batch_sync(bool narrow, bool deep) {
+    return narrow ? (deep ? k_lat_sync_batch<true, true> : k_lat_sync_batch<true, false>)
+                  : (deep ? k_lat_sync_batch<false, true> : k_lat_sync_batch<false, false>);
 }
 
 // Opts the kernels in to large dynamic shared memory, once per device.
@@ -196,11 +217,13 @@ void lat_attributes() {
                              (int) kLatFinalSmemMax);
     };
     set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_final_batch);
-    set(k_lat_sync_batch<false>); set(k_lat_sync_batch<true>);
-    for (uint32_t B = 4; B <= 32; B *= 2) {
-        set(sync_kernel<false>(B));
-        set(sync_kernel<true>(B));
-    }
+    set(batch_sync(false, false)); set(batch_sync(false, true));
+    set(batch_sync(true, false)); set(batch_sync(true, true));
+    for (uint32_t B = 4; B <= 32; B *= 2)
+        for (uint32_t D = 16; D <= 32; D *= 2) {
+            set(sync_kernel(B, D, false));
+            set(sync_kernel(B, D, true));
+        }
     set(k_lat_final<false, 4>); set(k_lat_final<false, 8>); set(k_lat_final<false, 16>);
     set(k_lat_final<false, 32>); set(k_lat_final<true, 32>);
     set(k_lat_final<true, 4>); set(k_lat_final<true, 8>); set(k_lat_final<true, 16>);
@@ -257,7 +280,7 @@ uint32_t lat_width(uint64_t starts, uint32_t sms) {
     return w <= 8 ? w : 32;
 }
 
-size_t lat_bytes(size_t nblk) { return lat_layout(nblk, kLatSlotsMax, kMaxStates).total; }
+size_t lat_bytes(size_t nblk) { return lat_layout(nblk, 16, kMaxStates).total; }
 
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out) {
@@ -278,10 +301,8 @@ bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t la
     // / 4: 3 blocks repaired, 0.6 ms; meet / 8: 5812 blocks, 86 ms.
     static const double per_meet[4] = {0.17, 1.0, 4.0, 6.8};
     const double s_par = std::max((double) n_units / lanes, 4.0);
-    uint32_t D = 4;
-    while (D < kLatSlotsMax && s_par < meet / per_meet[D / 4 - 1]) D += 4;
-    for (; D >= 4; D -= 4) {
-        const double s = std::max(s_par, meet / per_meet[D / 4 - 1]);
+    const auto fit = [&](uint32_t D, double per, LatPlan* o) {
+        const double s = std::max(s_par, meet / per);
         uint32_t B = b_pref;
         while (B > 4 && B > s && spu * B >= 96.0) B /= 2;
         for (; B <= 32; B *= 2) {
@@ -289,18 +310,36 @@ bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t la
             if (nblk * D > 0xffffffffull) continue;
             const size_t need = lat_layout(nblk, D, L).total;
             if (need > bytes) continue;
-            out->B = B;
+            o->B = B;
             // rounded up, so that starts never outnumber the lanes of one wave
-            out->nb = (uint32_t) std::max(1.0, s > s_par ? std::floor(s / B + 0.5) : std::ceil(s / B));
-            out->D = D;
-            out->nblk = (uint32_t) nblk;
-            out->nseed = (uint32_t) ((nblk + out->nb - 1) / out->nb);
-            out->L = L;
-            out->bytes = need;
+            o->nb = (uint32_t) std::max(1.0, s > s_par ? std::floor(s / B + 0.5) : std::ceil(s / B));
+            o->D = D;
+            o->nblk = (uint32_t) nblk;
+            o->nseed = (uint32_t) ((nblk + o->nb - 1) / o->nb);
+            o->L = L;
+            o->bytes = need;
             return true;
         }
-    }
-    return false;
+        return false;
+    };
+    uint32_t D = 4;
+    while (D < 16 && s_par < meet / per_meet[D / 4 - 1]) D += 4;
+    bool ok = false;
+    for (; D >= 4 && !ok; D -= 4) ok = fit(D, per_meet[D / 4 - 1], out);
+    // Short streams leave the GPU idle at that spacing and take as long as
+    // their longest trajectory, which is shorter the more others it can meet:
+    // 32 slots, where the workspace has room for them, that brings the starts
+    // closer by a quarter at least, and the lanes (a quarter of them: more
+    // trajectories are more work) and blocks no shorter allow it.  Sync pass
+    // of 146 KB at 3.1 bits per symbol, L = 4096: 290 -> 132 us, of 5 MB at 2.5
+    // 576 -> 308; shorter blocks gain nothing (128 KB at 3.8 bits, L = 1024,
+    // blocks of 16 -> 8: 67 us both, and 6 us more in the scan); past the
+    // quarter a batch of 256 streams takes 633 us instead of 584.
+    LatPlan deep;
+    if (ok && out->D == 16 && fit(32, 29.0, &deep) && 4ull * deep.nseed <= lanes &&
+        deep.B >= out->B && 4ull * deep.nb * deep.B <= 3ull * out->nb * out->B)
+        *out = deep;
+    return ok;
 }
 
 uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaStream_t st,
@@ -324,7 +363,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
         const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
         const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
         const size_t sm = lat_sync_smem(call.L, plan.B, th);
-        (width < 32 ? sync_kernel<true>(plan.B) : sync_kernel<false>(plan.B))<<<grid, th, sm, st>>>(p);
+        sync_kernel(plan.B, plan.D, width < 32)<<<grid, th, sm, st>>>(p);
     }
     mark(2, st);
     mark(3, st);
@@ -334,7 +373,8 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
         if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, sm, st>>>(p);
         else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, sm, st>>>(p);
         else if (plan.D == 12) k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
-        else k_lat_scan<16><<<g, kLatScanThreads, sm, st>>>(p);
+        else if (plan.D == 16) k_lat_scan<16><<<g, kLatScanThreads, sm, st>>>(p);
+        else k_lat_scan<32><<<g, kLatScanThreads, sm, st>>>(p);
     }
     mark(4, st);
     {
@@ -409,15 +449,13 @@ void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSme
     if (n) k_lat_prep_batch<<<(unsigned) n, kLatPrepThreads, sm.prep, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t width, cudaStream_t st) {
-    auto* k = width < 32 ? k_lat_sync_batch<true> : k_lat_sync_batch<false>;
-    if (n) k<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
+                    uint32_t width, bool deep, cudaStream_t st) {
+    if (n) batch_sync(width < 32, deep)<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t* ticket, cudaStream_t st) {
-    if (n)
-        k_lat_scan_batch<<<(unsigned) n, kLatScanThreads, sm.scan, st>>>((const LatParams*) ps,
-                                                                         items, ticket);
+                    bool deep, uint32_t* ticket, cudaStream_t st) {
+    auto* k = deep ? k_lat_scan_batch<true> : k_lat_scan_batch<false>;
+    if (n) k<<<(unsigned) n, kLatScanThreads, sm.scan, st>>>((const LatParams*) ps, items, ticket);
 }
 void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st) {
     if (n)

@@ -59,7 +59,7 @@ struct LatParams {
     uint32_t* tab_cnt;              // [L] counting table (zero-bit runs folded)
     uint32_t* tab_sym;              // [L] symbol table
     uint32_t* key;                  // [nblk * D] entries (0: free slot)
-    uint32_t* node;                 // [nblk * D] count | next slot << 28
+    uint32_t* node;                 // [nblk * D] count | next slot << 27
     unsigned long long* start;      // [nblk] true entry (rel | idx << 8) | output offset << 21
     unsigned long long* tile_map;   // [ntiles] look-back words: slot maps
     unsigned long long* tile_sum;   // [ntiles] look-back words: counts
@@ -379,11 +379,12 @@ __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B
 // when they were waited for).
 // Starts are taken from the counter `next`, up to `limit`.  kNarrow: warps of
 // which only p.width lanes run, on inputs with few trajectories; no CTA
-// barriers then, and twice the slots are looked at ahead (a block with more
+// barriers then.  kV: groups of four slots looked at ahead, two in narrow
+// warps (a block with more
 // than three trajectories costs two exposed round trips otherwise: 146 KB at
 // 3.1 bits per symbol, L = 4096, 316 -> 290 us, 128 KB at 3.8 79 -> 67; all
 // sixteen looked at: 321 and 73; wide warps: a batch 579 -> 594).
-template <uint32_t kB, bool kNarrow>
+template <uint32_t kB, bool kNarrow, uint32_t kV>
 __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next, uint32_t limit) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     __shared__ uint32_t s_live[kLatThreads / 32];
@@ -397,10 +398,9 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     constexpr uint32_t kSlots = 2 * kB;              // unit slots of a lane's ring
     constexpr uint32_t kMask = (kSlots - 1) * 32;
     constexpr uint32_t kBits = kB * 32;
-    constexpr uint32_t kV = kNarrow ? 2 : 1;         // groups of four slots seen ahead
     const uint32_t rings = tb + ((p.L * 4 + 15) & ~15u);
     const uint32_t col = rings + warp * kRing + lane * 4;
-    const uint32_t D = p.D;
+    const uint32_t D = p.D, end = kV > 2 ? lat_usable(32) : min(D, lat_usable(16));
     const bool wide = ((uintptr_t) p.units & 31) == 0;
 
     bool on = false, exhausted = false;
@@ -447,7 +447,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     // units are staged again).  Without it two lanes of three idle.
     const auto close_up = [&]() -> bool {
         const uint32_t n = __syncthreads_count(on);
-        if (n != 0 && 2 * n <= room && room > 32 && __syncthreads_and(exhausted)) {
+        if (2 * n <= room && room > 32 && __syncthreads_and(exhausted)) {
             const uint32_t live = __ballot_sync(0xffffffffu, on);
             if (lane == 0) s_live[warp] = __popc(live);
             __syncthreads();
@@ -460,7 +460,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                 sts32(x + 8, cas);
                 sts32(x + 12, prev);
                 sts32(x + 16, pcnt);
-                sts32(x + 20, q | (first ? 16u : 0u) | (has_prev ? 32u : 0u));
+                sts32(x + 20, q | (first ? 32u : 0u) | (has_prev ? 64u : 0u));
                 sts32(x + 24, life);
             }
             __syncthreads();
@@ -473,9 +473,9 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                 prev = lds32(x + 12);
                 pcnt = lds32(x + 16);
                 const uint32_t f = lds32(x + 20);
-                q = f & 15u;
-                first = (f & 16u) != 0;
-                has_prev = (f & 32u) != 0;
+                q = f & 31u;
+                first = (f & 32u) != 0;
+                has_prev = (f & 64u) != 0;
                 life = lds32(x + 24);
             }
             __syncthreads();
@@ -505,7 +505,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
                     p.key[0] = val;
                 } else {
                     bool found;
-                    q = lat_take(p.key + (size_t) b * D, 1, D, val, found);
+                    q = lat_take(p.key + (size_t) b * D, 1, end, val, found);
                     if (found || q == kLatDead) on = false;
                 }
                 cas = 0;
@@ -540,9 +540,9 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         bool found = false;
         if (cas != 0) {
             if (cas == val) found = true;
-            else q = lat_take(p.key + (size_t) b * D, q + 1, D, val, found);
+            else q = lat_take(p.key + (size_t) b * D, q + 1, end, val, found);
         }
-        if (has_prev) p.node[prev] = pcnt | (q << 28);
+        if (has_prev) p.node[prev] = pcnt | (q << kLatNodeShift);
         if (found || q == kLatDead || !more) {
             on = false;
             max_life = max(max_life, life);
@@ -554,7 +554,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         pcnt = cnt;
         // arrive at block b + 1
         val = kLatKeyUsed | (c.pos - be) | (((c.a - tb) << 6));
-        uint32_t hit = kLatDead, open = min(kV * 4, D) - 1;
+        uint32_t hit = kLatDead, open = kV == 1 ? 3u : min(kV * 4, D) - 1;
 #pragma unroll
         for (uint32_t g = kV; g-- > 0;) {
             if (kn[g].w == val) hit = 4 * g + 3;
@@ -568,15 +568,15 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         }
         ++b;
         if (hit != kLatDead) {
-            p.node[prev] = pcnt | (hit << 28);
+            p.node[prev] = pcnt | (hit << kLatNodeShift);
             on = false;
             max_life = max(max_life, life);
             visits += life;
             continue;
         }
         // the true start's trajectory has slot 0 of every block to itself
-        q = first ? 0u : min(open, kLatDead);
-        cas = q == kLatDead ? 0u : lat_cas(knext + q, val);
+        q = first ? 0u : open;
+        cas = lat_cas(knext + q, val);
         // block b + 1 (one ahead again) into the half of the ring that is free
         const uint32_t s = (b & 1u) * kB;      // slots of block b
         lat_store_units<kB>(nx, col, s ^ kB, carry);

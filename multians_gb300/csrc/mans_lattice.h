@@ -25,7 +25,8 @@ struct LatPlan {
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out);
 
-// Workspace of a lattice of nblk blocks with all slots.
+// Workspace of a lattice of nblk blocks with 16 slots each; a plan uses what
+// it is given, 32 slots a block where they fit.
 size_t lat_bytes(size_t nblk);
 
 struct LatCall {
@@ -76,9 +77,9 @@ void lat_batch_init();
 void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
                     cudaStream_t st);
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t width, cudaStream_t st);
+                    uint32_t width, bool deep, cudaStream_t st);
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t* ticket, cudaStream_t st);
+                    bool deep, uint32_t* ticket, cudaStream_t st);
 void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st);
 
 }  // namespace mans

@@ -4,7 +4,7 @@
 //
 // P, the parameter block of either, has
 //   key    [nblk * D]  entries at each block, bit 31 set (0: free slot)
-//   node   [nblk * D]  count of the block (28 bits) | next slot << 28
+//   node   [nblk * D]  count of the block (27 bits) | next slot << 27
 //   start  [nblk]      out: true entry (kLatEntBits) | offset << kLatEntBits
 //   tile_map, tile_sum [ntiles]  look-back words, zero before
 //   ctr    [8]         counters, zero before
@@ -26,8 +26,15 @@
 
 namespace mans {
 
-constexpr uint32_t kLatSlotsMax = 16;     // 15 of them used: the last names no slot
-constexpr uint32_t kLatDead = 15;          // node: no slot at the next block
+constexpr uint32_t kLatSlotsMax = 32;
+constexpr uint32_t kLatNodeShift = 27;
+constexpr uint32_t kLatDead = 31;          // node: no slot at the next block
+// Slots that are taken: with 16 and 32 the last one is not, it stands for
+// "none" in the scan's maps of four and five bits a slot.
+__host__ __device__ constexpr uint32_t lat_none(uint32_t D) { return D > 16 ? 31 : 15; }
+__host__ __device__ constexpr uint32_t lat_usable(uint32_t D) {
+    return D < lat_none(D) ? D : lat_none(D);
+}
 constexpr uint32_t kLatKeyUsed = 0x80000000u;
 constexpr uint32_t kLatEntBits = 21;       // entry: bit offset (8), state index (13)
 constexpr uint32_t kLatScanThreads = 256;
@@ -62,14 +69,13 @@ __device__ __forceinline__ uint4 lat_ld_slots(const uint32_t* a) {
     return v;
 }
 
-// Takes or finds the slot of entry `val` among slots [from, D) of a block:
+// Takes or finds the slot of entry `val` among slots [from, end) of a block:
 // the slots as they are now, four at a time, then a compare-and-swap on the
 // first free one.  Returns the slot (kLatDead: none free) and whether a
 // trajectory with that entry was there first.
-__device__ __forceinline__ uint32_t lat_take(uint32_t* __restrict__ key, uint32_t from, uint32_t D,
+__device__ __forceinline__ uint32_t lat_take(uint32_t* __restrict__ key, uint32_t from, uint32_t end,
                                              uint32_t val, bool& found) {
     found = false;
-    const uint32_t end = min(D, kLatDead);
     uint32_t q = from;
     while (q < end) {
         const uint32_t g = q & ~3u;
@@ -97,8 +103,8 @@ __device__ __forceinline__ uint32_t lat_take(uint32_t* __restrict__ key, uint32_
 // scan: the true path's slot at every block, then its output offsets
 
 // A slot map, one byte a slot: byte s = the slot a node in slot s leads to,
-// kLatDead (15, a fixed point) when it leads nowhere; slots from 4 * kW on
-// are fixed points too.  With 16 slots the last is never taken.
+// lat_none (15 or 31, a fixed point) when it leads nowhere; slots from 4 * kW
+// on are fixed points too.
 template <uint32_t kW>
 struct LatMap {
     uint32_t w[kW];
@@ -112,21 +118,28 @@ __device__ __forceinline__ LatMap<kW> lat_identity() {
     return m;
 }
 
-// g after f: byte permutes by f's bytes within the two halves of g's 16
-// entries, then the half by bit 3.
+// g after f: byte permutes by f's bytes within each eight of g's entries,
+// then the eight by bits 3 and 4.
 template <uint32_t kW>
 __device__ __forceinline__ LatMap<kW> lat_compose(const LatMap<kW>& g, const LatMap<kW>& f) {
-    const uint32_t g1 = kW > 1 ? g.w[kW > 1 ? 1 : 0] : 0x07060504u;
-    const uint32_t g2 = kW > 2 ? g.w[kW > 2 ? 2 : 0] : 0x0b0a0908u;
-    const uint32_t g3 = kW > 3 ? g.w[kW > 3 ? 3 : 0] : 0x0f0e0d0cu;
+    constexpr uint32_t kAll = kW > 4 ? 8 : 4;
+    uint32_t t[kAll];
+#pragma unroll
+    for (uint32_t i = 0; i < kAll; ++i) t[i] = i < kW ? g.w[i < kW ? i : 0] : 0x03020100u + i * 0x04040404u;
     LatMap<kW> h;
 #pragma unroll
     for (uint32_t i = 0; i < kW; ++i) {
         const uint32_t x = f.w[i], x7 = x & 0x07070707u;
         const uint32_t sel = __byte_perm((x7 | (x7 >> 4)) & 0x00ff00ffu, 0, 0x4420);
-        const uint32_t lo = __byte_perm(g.w[0], g1, sel), hi = __byte_perm(g2, g3, sel);
         const uint32_t up = ((x >> 3) & 0x01010101u) * 0xffu;
-        h.w[i] = (lo & ~up) | (hi & up);
+        uint32_t v = (__byte_perm(t[0], t[1], sel) & ~up) | (__byte_perm(t[2], t[3], sel) & up);
+        if (kW > 4) {
+            const uint32_t v2 = (__byte_perm(t[kAll - 4], t[kAll - 3], sel) & ~up) |
+                                (__byte_perm(t[kAll - 2], t[kAll - 1], sel) & up);
+            const uint32_t far = ((x >> 4) & 0x01010101u) * 0xffu;
+            v = (v & ~far) | (v2 & far);
+        }
+        h.w[i] = v;
     }
     return h;
 }
@@ -136,11 +149,12 @@ __device__ __forceinline__ uint32_t lat_apply(const LatMap<kW>& m, uint32_t s) {
     uint32_t x = s;
 #pragma unroll
     for (uint32_t i = 0; i < kW; ++i)
-        if ((s >> 2) == i) x = (m.w[i] >> (8 * (s & 3u))) & 15u;
+        if ((s >> 2) == i) x = (m.w[i] >> (8 * (s & 3u))) & 31u;
     return x;
 }
 
-// look-back words: four bits a slot (15 slots), the state in bits 62..63
+// look-back words: four bits a slot (15 slots; none with more), the state in
+// bits 62..63
 constexpr unsigned long long kLatAgg = 1;     // the tile's map or sum
 constexpr unsigned long long kLatInc = 2;     // the slot at, or the sum to, its end
 constexpr unsigned long long kLatGhost = 3;   // the entry at its end, which has no slot
@@ -155,25 +169,26 @@ __device__ __forceinline__ unsigned long long lat_ld(const unsigned long long* a
 template <class P, uint32_t kD>
 struct LatTile {
     static constexpr uint32_t kW = kD / 4;
+    static constexpr uint32_t kNone = lat_none(kD);
     static constexpr uint32_t kWarps = kLatScanThreads / 32;
     struct Shared {
         LatMap<kW> map[kWarps];
         unsigned long long sum[kWarps];
         unsigned long long base;
-        uint32_t slot;     // at the tile's first block (kLatDead: none)
+        uint32_t slot;     // at the tile's first block (kNone: none)
         uint32_t ghost;    // its entry where the path has no slot there (~0: it has)
         uint32_t dead;     // first block without a slot (~0: none)
         uint32_t from;     // the path is followed from this block
         uint32_t end;      // slot after the tile
     };
     LatMap<kW> f[kLatScanPer], exc;
-    uint32_t b0, last;   // last: the slot at the stream's last block (kLatDead: not here)
+    uint32_t b0, last;   // last: the slot at the stream's last block (kNone: not here)
     uint32_t cnt[kLatScanPer], ent[kLatScanPer];
     unsigned long long sum, run;
 
     __device__ __forceinline__ void load(const P& p, uint32_t first) {
         b0 = first + threadIdx.x * kLatScanPer;
-        last = kLatDead;
+        last = kNone;
 #pragma unroll
         for (uint32_t i = 0; i < kLatScanPer; ++i) {
             const uint32_t b = b0 + i;
@@ -183,11 +198,12 @@ struct LatTile {
                 const uint4* nd = reinterpret_cast<const uint4*>(p.node + (size_t) b * kD);
 #pragma unroll
                 for (uint32_t s = 0; s < kW; ++s) {
-                    const uint4 v = __ldg(nd + s);   // the top nibbles of four nodes
+                    const uint4 v = __ldg(nd + s);   // the top five bits of four nodes
                     f[i].w[s] = (__byte_perm(__byte_perm(v.x, v.y, 0x0073),
-                                             __byte_perm(v.z, v.w, 0x7300), 0x7610) >> 4) & 0x0f0f0f0fu;
+                                             __byte_perm(v.z, v.w, 0x7300), 0x7610) >> 3) &
+                                (kNone * 0x01010101u);
                 }
-                if (kW == 4) f[i].w[kW - 1] |= 0x0f000000u;   // slot 15: dead
+                if (kD > kNone) f[i].w[kW - 1] |= kNone << 24;   // the slot that stands for none
             }
         }
     }
@@ -227,11 +243,11 @@ struct LatTile {
         for (uint32_t i = 0; i < kLatScanPer; ++i) {
             const uint32_t b = b0 + i;
             if (b < p.nblk && b >= sh.from) {
-                const bool ok = s < kD && s != kLatDead;
+                const bool ok = s < lat_usable(kD);
                 if (!ok) dead = min(dead, b);
                 const size_t at = (size_t) b * kD + min(s, kD - 1);
                 ent[i] = __ldg(p.key + at) & ((1u << kLatEntBits) - 1);
-                cnt[i] = b + 1 < p.nblk && ok ? __ldg(p.node + at) & 0x0fffffffu : 0u;
+                cnt[i] = b + 1 < p.nblk && ok ? __ldg(p.node + at) & ((1u << kLatNodeShift) - 1) : 0u;
                 if (b + 1 == p.nblk) last = s;
             }
             s = lat_apply(f[i], s);
@@ -263,7 +279,7 @@ struct LatTile {
 #pragma unroll
         for (uint32_t i = 0; i < kLatScanPer; ++i) {
             if (b0 + i < p.nblk) p.start[b0 + i] = ent[i] | (o << kLatEntBits);
-            if (b0 + i + 1 == p.nblk && last < kD && last != kLatDead) p.finish(last, o);
+            if (b0 + i + 1 == p.nblk && last < lat_usable(kD)) p.finish(last, o);
             o += cnt[i];
         }
     }
@@ -283,6 +299,7 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
     // entry and count of the blocks decoded here
     uint2* const s_over = reinterpret_cast<uint2*>(lat_repair_sm + ((p.repair_words() + 1) & ~1u));
     __shared__ uint32_t s_at, s_ent;
+    constexpr uint32_t kNone = lat_none(kD);
     const uint32_t stop = min(first + kLatScanTile, p.nblk);
     p.repair_load(lat_repair_sm);
     uint32_t b = first;          // the sequential stretch starts here
@@ -300,7 +317,7 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            uint32_t x = b, e = ent, slot = kLatDead;
+            uint32_t x = b, e = ent, slot = kNone;
             while (x < stop) {
                 unsigned long long n = 0;
                 s_over[x - first].x = e;
@@ -317,16 +334,16 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
                     if (k.z == want) slot = 4 * w + 2;
                     if (k.w == want) slot = 4 * w + 3;
                 }
-                if (slot != kLatDead) break;
+                if (slot != kNone) break;
             }
             const uint32_t used = atomicAdd(p.ctr + kLatRepaired, x - b) + (x - b);
             if (used > p.repair_blocks()) {
                 atomicOr(p.status, MANS_DEV_SYNC_OVERFLOW);
-                slot = kLatDead;
+                slot = kNone;
                 e = ~0u;
             }
             s_at = x;
-            sh.ghost = slot == kLatDead ? e : ~0u;   // leaves the tile without a slot
+            sh.ghost = slot == kNone ? e : ~0u;   // leaves the tile without a slot
             sh.end = slot;
             sh.dead = ~0u;
             sh.from = x;
@@ -343,7 +360,7 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
                 if (x + 1 == p.nblk) tl.last = kLatSlotsMax;   // the end, without a slot
             }
         }
-        if (slot == kLatDead) break;   // at the tile's end, or given up
+        if (slot == kNone) break;   // at the tile's end, or given up
         // follow the tile from block `at`: the blocks before it lead there
 #pragma unroll
         for (uint32_t i = 0; i < kLatScanPer; ++i)
@@ -354,7 +371,7 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
         __syncthreads();
         tl.path(p, sh);
         __syncthreads();
-        const bool dead = sh.dead != ~0u, end = sh.end == kLatDead;
+        const bool dead = sh.dead != ~0u, end = sh.end == kNone;
         __syncthreads();
         if (!dead && !end) break;
         // the last block leads to one without a slot: the next tile's
@@ -368,7 +385,7 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
 template <class P, uint32_t kD>
 __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
     using Tile = LatTile<P, kD>;
-    constexpr uint32_t kWarps = Tile::kWarps;
+    constexpr uint32_t kWarps = Tile::kWarps, kNone = Tile::kNone;
     __shared__ typename Tile::Shared sh;
     const uint32_t st = *(volatile uint32_t*) p.status;
     if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_DEGENERATE)) return;
@@ -384,12 +401,31 @@ __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
     __syncthreads();
     // the tile's map (lane s follows slot s), then the slot at its first block
     if (warp == 0) {
-        uint32_t x = lane & 15u;
+        uint32_t x = lane & kNone;
         for (uint32_t w = 0; w < kWarps; ++w) x = lat_apply(sh.map[w], x);
         uint32_t slot = 0, ghost = ~0u;
-        if (tile != 0) {
+        if (tile != 0 && kD > 16) {
+            // a map does not fit a look-back word: the tile before's end
+            uint32_t spins = 0;
+            for (;;) {
+                const unsigned long long v = lat_ld(p.tile_map + tile - 1);
+                if ((v >> 62) >= kLatInc) {
+                    const bool is_ghost = (v >> 62) == kLatGhost;
+                    if (is_ghost) ghost = (uint32_t) v & ((1u << kLatEntBits) - 1);
+                    slot = is_ghost ? kNone : (uint32_t) v & kNone;
+                    break;
+                }
+                if (++spins > (1u << 24)) {
+                    if (lane == 0) atomicOr(p.status, MANS_DEV_SCAN_TIMEOUT);
+                    slot = kNone;
+                    break;
+                }
+            }
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+            ghost = __shfl_sync(0xffffffffu, ghost, 0);
+        } else if (tile != 0) {
             const unsigned long long own =
-                lane < kD && lane < kLatDead ? (unsigned long long) x << (4 * lane) : 0ull;
+                lane < lat_usable(kD) ? (unsigned long long) x << (4 * lane) : 0ull;
             const unsigned long long agg =
                 (unsigned long long) __reduce_or_sync(0xffffffffu, (uint32_t) own) |
                 (unsigned long long) __reduce_or_sync(0xffffffffu, (uint32_t) (own >> 32)) << 32;
@@ -414,7 +450,7 @@ __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
                     uint32_t r = incl ? (uint32_t) e & 15u : (lane & 15u);
                     for (int32_t i = (int32_t) stop - (incl ? 1 : 0); i >= 0; --i) {
                         const unsigned long long m = __shfl_sync(0xffffffffu, v, i);
-                        if (r < kD && r != kLatDead) r = (uint32_t) (m >> (4 * r)) & 15u;
+                        if (r < lat_usable(kD)) r = (uint32_t) (m >> (4 * r)) & 15u;
                     }
                     const uint32_t to = __shfl_sync(0xffffffffu, near, r);
                     if (!incl) {
@@ -425,10 +461,10 @@ __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
                     const bool direct = j == (int32_t) tile - 1 && stop == 0;
                     if (direct) {   // the tile before: its end, whatever it is
                         if (is_ghost) ghost = (uint32_t) e & ((1u << kLatEntBits) - 1);
-                        slot = is_ghost ? kLatDead : (uint32_t) e & 15u;
+                        slot = is_ghost ? kNone : (uint32_t) e & 15u;
                         break;
                     }
-                    if (!is_ghost && to != kLatDead) {
+                    if (!is_ghost && to != kNone) {
                         slot = to;
                         break;
                     }
@@ -440,15 +476,15 @@ __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
                 }
                 if (++spins > (1u << 24)) {
                     if (lane == 0) atomicOr(p.status, MANS_DEV_SCAN_TIMEOUT);
-                    slot = kLatDead;
+                    slot = kNone;
                     break;
                 }
             }
         }
-        const uint32_t end = __shfl_sync(0xffffffffu, x, slot & 15u);
+        const uint32_t end = __shfl_sync(0xffffffffu, x, slot & kNone);
         if (lane == 0) {
             // a path that keeps a slot to the tile's end needs nothing more
-            if (end != kLatDead || (slot == kLatDead && ghost == ~0u))
+            if (end != kNone || (slot == kNone && ghost == ~0u))
                 atomicExch(p.tile_map + tile, (unsigned long long) end | (kLatInc << 62));
             sh.slot = slot;
             sh.ghost = ghost;
@@ -456,8 +492,8 @@ __device__ __forceinline__ void lat_scan_body(const P& p, uint32_t tile) {
         }
     }
     __syncthreads();
-    const bool lost = sh.slot == kLatDead && sh.ghost == ~0u;   // given up before
-    const bool broken = !lost && sh.end == kLatDead && first + kLatScanTile < p.nblk;
+    const bool lost = sh.slot == kNone && sh.ghost == ~0u;   // given up before
+    const bool broken = !lost && sh.end == kNone && first + kLatScanTile < p.nblk;
     if (!lost && sh.ghost == ~0u) tl.path(p, sh);
     __syncthreads();
     const bool repair = !lost && (sh.ghost != ~0u || sh.dead != ~0u || broken);

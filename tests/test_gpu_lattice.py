@@ -111,8 +111,8 @@ def test_repaired_path(mg, oracle_lib):
     ran = 0
     for seed in range(12):
         rng = np.random.default_rng(seed)
-        n = 200_000
-        sym = rng.integers(0, 8, n).astype(np.uint8)
+        n = 600_000
+        sym = rng.integers(0, 2, n).astype(np.uint8)
         sym[rng.random(n) < 0.0002 * (seed % 2)] = 200
         st = O.encode(sym, 1024)
         assert st.n_units <= 32768
