@@ -50,7 +50,9 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "mans_device.cuh"
@@ -2504,7 +2506,14 @@ static bool lattice_plan(const mans_cfg& cfg, size_t n_units, size_t n_out, uint
                          size_t aux_bytes, LatPlan* out) {
     if (!(cfg.flags & MANS_DECODE_LATTICE)) return false;
     const double bps = 32.0 * (double) n_units / (double) n_out;
-    return lat_plan(n_units, n_out, L, mean_meeting_units(L, bps), 152 * 16 * 32, aux_bytes, out);
+    const double meet = mean_meeting_units(L, bps);
+    if (!lat_plan(n_units, n_out, L, meet, 152 * 16 * 32, aux_bytes, out)) return false;
+    LatPlan deep;
+    if (lat_deep(n_units, n_out, L, meet, aux_bytes, *out, &deep) &&
+        lat_cost(n_units, n_out, meet, *out).chain_us >
+            2 * lat_cost(n_units, n_out, meet, deep).work_us)
+        *out = deep;
+    return true;
 }
 
 // The decode's launch sequence; with sync_only the final pass is left out
@@ -3083,6 +3092,26 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
                   !(hint->flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS |
                                    MANS_DECODE_NO_CAPTURE | MANS_DECODE_CAPTURE)));
     const double sym_per_lane = batch_sym / (152.0 * 16 * 32);
+    const auto stream_hint = [&](const mans_stream_desc& s) {
+        mans_cfg h = {0, 0, 0, 0, 0, 0};
+        if (hint) h = *hint;
+        h.flags |= s.flags & (MANS_DECODE_NO_CAPTURE | MANS_DECODE_CAPTURE);
+        // batches plan each stream with the model: the measured table is
+        // tuned for streams decoded alone (capture lost on batches of short
+        // streams: the capturing G pass holds fewer warps per SM)
+        h.flags |= MANS_PLAN_MODEL;
+        return h;
+    };
+    const auto meet = [&](uint32_t i) {
+        return mean_meeting_units(d[i].L, 32.0 * (double) d[i].n_units / (double) d[i].n_out);
+    };
+    // a lattice stays in the workspace the stream's own plan has
+    const auto room = [&](uint32_t i) {
+        const mans_cfg& c = plans[i].cfg;
+        const size_t nblk = num_blocks(d[i].n_units, c.block_units);
+        return layout_for(nblk, (nblk + c.region_blocks - 1) / c.region_blocks, c.walk_slots, 0,
+                          false).total;
+    };
     for (uint32_t i = 0; i < n; ++i) {
         BatchStreamPlan& sp = plans[i];
         sp.active = d[i].n_out > 0;
@@ -3093,26 +3122,47 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
             d[i].first_bit > ((d[i].flags & MANS_DECODE_START_OFFSET) ? 127u : 32u) ||
             ((uintptr_t) d[i].d_units & 15) != 0)
             return MANS_ERR_ARG;
-        mans_cfg h = {0, 0, 0, 0, 0, 0};
-        if (hint) h = *hint;
-        h.flags |= d[i].flags & (MANS_DECODE_NO_CAPTURE | MANS_DECODE_CAPTURE);
-        // batches plan each stream with the model: the measured table is
-        // tuned for streams decoded alone (capture lost on batches of short
-        // streams: the capturing G pass holds fewer warps per SM)
-        h.flags |= MANS_PLAN_MODEL;
+        const mans_cfg h = stream_hint(d[i]);
         int rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &sp.cfg);
         if (rc != MANS_OK) return rc;
-        if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE)) {
+        if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE))
             // as many starts as its share of the batch's symbols has of the
-            // lanes side by side, in the workspace the stream's own plan has
-            const size_t nblk = num_blocks(d[i].n_units, sp.cfg.block_units);
-            const size_t nreg = (nblk + sp.cfg.region_blocks - 1) / sp.cfg.region_blocks;
-            const double bps = 32.0 * (double) d[i].n_units / (double) d[i].n_out;
+            // lanes side by side
             sp.lattice = lat_plan(
-                d[i].n_units, d[i].n_out, d[i].L, mean_meeting_units(d[i].L, bps),
-                (uint32_t) std::max(1.0, kBatchLanes * (double) d[i].n_out / batch_sym),
-                layout_for(nblk, nreg, sp.cfg.walk_slots, 0, false).total, &sp.lat);
+                d[i].n_units, d[i].n_out, d[i].L, meet(i),
+                (uint32_t) std::max(1.0, kBatchLanes * (double) d[i].n_out / batch_sym), room(i),
+                &sp.lat);
+    }
+    // 32 slots for the longest chains, while they are twice as long as all the
+    // work (once: 64 served streams 1192 us, but a batch of 256 1113 instead of
+    // 815, whose work hides its chains)
+    {
+        double work = 0;
+        std::vector<std::pair<double, uint32_t>> chains;
+        for (uint32_t i = 0; i < n; ++i)
+            if (plans[i].active && plans[i].lattice) {
+                const LatCost c = lat_cost(d[i].n_units, d[i].n_out, meet(i), plans[i].lat);
+                work += c.work_us;
+                chains.emplace_back(c.chain_us, i);
+            }
+        std::sort(chains.begin(), chains.end(), std::greater<>());
+        for (const auto& [chain, i] : chains) {
+            if (chain <= 2 * work) break;
+            LatPlan deep;
+            if (!lat_deep(d[i].n_units, d[i].n_out, d[i].L, meet(i), room(i), plans[i].lat, &deep))
+                continue;
+            const double more = lat_cost(d[i].n_units, d[i].n_out, meet(i), deep).work_us -
+                                lat_cost(d[i].n_units, d[i].n_out, meet(i), plans[i].lat).work_us;
+            if (chain <= 2 * (work + more)) continue;
+            work += more;
+            plans[i].lat = deep;
         }
+    }
+    for (uint32_t i = 0; i < n; ++i) {
+        BatchStreamPlan& sp = plans[i];
+        if (!sp.active) continue;
+        mans_cfg h = stream_hint(d[i]);
+        int rc = MANS_OK;
         if (h.region_blocks == 0) {
             const double spu = (double) d[i].n_out / (double) d[i].n_units;
             const uint64_t B = sp.cfg.block_units;

@@ -282,64 +282,77 @@ uint32_t lat_width(uint64_t starts, uint32_t sms) {
 
 size_t lat_bytes(size_t nblk) { return lat_layout(nblk, 16, kMaxStates).total; }
 
-bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
-              LatPlan* out) {
-    if (n_out >> (63 - kLatEntBits)) return false;
+// Blocks and starts for starts every `s` units (s_par: the distance at which
+// they fill the lanes) and D slots.
+static bool lat_fit(size_t n_units, size_t n_out, uint32_t L, double s, double s_par, uint32_t D,
+                    size_t bytes, LatPlan* o) {
     // About 128 symbols per block: the final pass stages 32 blocks a warp, and
     // a step's share of a block's bookkeeping stays below a tenth.  Blocks of
     // 32 units from 5.3 bits per symbol on (256 MB at 6 bits: 691 -> 629 us,
     // 512 MB at 8.6 bits 1511 -> 1192, the scan and the slots' traffic halved).
     const double spu = (double) n_out / (double) n_units;
-    uint32_t b_pref = 32;
-    while (b_pref > 4 && spu * b_pref > 192.0) b_pref /= 2;
-    // Starts every s units: as many as run side by side, but no closer than
-    // the slots allow.  About 1.2 sqrt(2 T / s) distinct trajectories are under
-    // way at a place on average, and twice that at most over a long stream: s
-    // = meet / per_meet[D / 4 - 1] leaves room for a T 2.7 times the model's
-    // (symbols of equal frequency meet that late).  Closer ones run out of
-    // slots: 3 M of eight equally frequent symbols, L = 1024, 12 slots, s = meet
-    // / 4: 3 blocks repaired, 0.6 ms; meet / 8: 5812 blocks, 86 ms.
-    static const double per_meet[4] = {0.17, 1.0, 4.0, 6.8};
-    const double s_par = std::max((double) n_units / lanes, 4.0);
-    const auto fit = [&](uint32_t D, double per, LatPlan* o) {
-        const double s = std::max(s_par, meet / per);
-        uint32_t B = b_pref;
-        while (B > 4 && B > s && spu * B >= 96.0) B /= 2;
-        for (; B <= 32; B *= 2) {
-            const size_t nblk = n_units / B + 1;
-            if (nblk * D > 0xffffffffull) continue;
-            const size_t need = lat_layout(nblk, D, L).total;
-            if (need > bytes) continue;
-            o->B = B;
-            // rounded up, so that starts never outnumber the lanes of one wave
-            o->nb = (uint32_t) std::max(1.0, s > s_par ? std::floor(s / B + 0.5) : std::ceil(s / B));
-            o->D = D;
-            o->nblk = (uint32_t) nblk;
-            o->nseed = (uint32_t) ((nblk + o->nb - 1) / o->nb);
-            o->L = L;
-            o->bytes = need;
-            return true;
-        }
-        return false;
-    };
+    uint32_t B = 32;
+    while (B > 4 && spu * B > 192.0) B /= 2;
+    while (B > 4 && B > s && spu * B >= 96.0) B /= 2;
+    for (; B <= 32; B *= 2) {
+        const size_t nblk = n_units / B + 1;
+        if (nblk * D > 0xffffffffull) continue;
+        const size_t need = lat_layout(nblk, D, L).total;
+        if (need > bytes) continue;
+        o->B = B;
+        // rounded up, so that starts never outnumber the lanes of one wave
+        o->nb = (uint32_t) std::max(1.0, s > s_par ? std::floor(s / B + 0.5) : std::ceil(s / B));
+        o->D = D;
+        o->nblk = (uint32_t) nblk;
+        o->nseed = (uint32_t) ((nblk + o->nb - 1) / o->nb);
+        o->L = L;
+        o->bytes = need;
+        return true;
+    }
+    return false;
+}
+
+// Starts every s units: as many as run side by side, but no closer than the
+// slots allow.  About 1.2 sqrt(2 T / s) distinct trajectories are under way at
+// a place on average, and twice that at most over a long stream: s = meet /
+// kPerMeet[D / 4 - 1] leaves room for a T 2.7 times the model's (symbols of
+// equal frequency meet that late).  Closer ones run out of slots: 3 M of eight
+// equally frequent symbols, L = 1024, 12 slots, s = meet / 4: 3 blocks
+// repaired, 0.6 ms; meet / 8: 5812 blocks, 86 ms.
+static constexpr double kPerMeet[4] = {0.17, 1.0, 4.0, 6.8};
+static constexpr double kPerMeetDeep = 29.0;   // 32 slots
+static constexpr double kMinSpacing = 4.0;     // units
+
+bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
+              LatPlan* out) {
+    if (n_out >> (63 - kLatEntBits)) return false;
+    const double s_par = std::max((double) n_units / lanes, kMinSpacing);
     uint32_t D = 4;
-    while (D < 16 && s_par < meet / per_meet[D / 4 - 1]) D += 4;
-    bool ok = false;
-    for (; D >= 4 && !ok; D -= 4) ok = fit(D, per_meet[D / 4 - 1], out);
-    // Short streams leave the GPU idle at that spacing and take as long as
-    // their longest trajectory, which is shorter the more others it can meet:
-    // 32 slots, where the workspace has room for them, that brings the starts
-    // closer by a quarter at least, and the lanes (a quarter of them: more
-    // trajectories are more work) and blocks no shorter allow it.  Sync pass
-    // of 146 KB at 3.1 bits per symbol, L = 4096: 290 -> 132 us, of 5 MB at 2.5
-    // 576 -> 308; shorter blocks gain nothing (128 KB at 3.8 bits, L = 1024,
-    // blocks of 16 -> 8: 67 us both, and 6 us more in the scan); past the
-    // quarter a batch of 256 streams takes 633 us instead of 584.
-    LatPlan deep;
-    if (ok && out->D == 16 && fit(32, 29.0, &deep) && 4ull * deep.nseed <= lanes &&
-        deep.B >= out->B && 4ull * deep.nb * deep.B <= 3ull * out->nb * out->B)
-        *out = deep;
-    return ok;
+    while (D < 16 && s_par < meet / kPerMeet[D / 4 - 1]) D += 4;
+    for (; D >= 4; D -= 4)
+        if (lat_fit(n_units, n_out, L, std::max(s_par, meet / kPerMeet[D / 4 - 1]), s_par, D, bytes,
+                    out))
+            return true;
+    return false;
+}
+
+bool lat_deep(size_t n_units, size_t n_out, uint32_t L, double meet, size_t bytes,
+              const LatPlan& base, LatPlan* out) {
+    // shorter blocks gain nothing (128 KB at 3.8 bits, L = 1024, blocks of 16
+    // -> 8: 67 us both, and 6 us more in the scan)
+    const double s = std::max(meet / kPerMeetDeep, kMinSpacing);
+    return lat_fit(n_units, n_out, L, s, kMinSpacing, 32, bytes, out) && out->B >= base.B &&
+           4ull * out->nb * out->B <= 3ull * base.nb * base.B;
+}
+
+LatCost lat_cost(size_t n_units, size_t n_out, double meet, const LatPlan& plan) {
+    // a trajectory meets one of the m - 1 others at its place; the longest
+    // of a stream goes about four times as far as the mean (simulated)
+    const double s = (double) plan.nb * plan.B;
+    const double m = std::max(1.0, 1.2 * std::sqrt(2.0 * meet / s));
+    // zero-bit steps are folded: two bits a step at least
+    const double steps = std::min(n_out / (double) n_units, 15.5);
+    return {std::min(4.0 * m * s, (double) n_units) * steps * 0.024, n_units * m * steps * 1e-6};
 }
 
 uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaStream_t st,

@@ -25,6 +25,23 @@ struct LatPlan {
 bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t lanes, size_t bytes,
               LatPlan* out);
 
+// A short stream leaves the GPU idle and takes as long as its longest
+// trajectory, which ends sooner the more others it can meet: the geometry
+// with 32 slots a block and starts closer by a quarter at least.  False when
+// there is none in `bytes`.  For streams whose chain is longer than the work
+// of everything that runs beside it (lat_cost): sync pass of 146 KB at 3.1
+// bits per symbol, L = 4096: 290 -> 132 us, of 5 MB at 2.5 576 -> 308; on all
+// streams of a batch of 256 MB 584 -> 633.
+bool lat_deep(size_t n_units, size_t n_out, uint32_t L, double meet, size_t bytes,
+              const LatPlan& base, LatPlan* out);
+
+// Sync pass of a plan, estimated: its longest chain (24 ns a step), and its
+// steps at the rate of a full GPU (1 M a microsecond).
+struct LatCost {
+    double chain_us, work_us;
+};
+LatCost lat_cost(size_t n_units, size_t n_out, double meet, const LatPlan& plan);
+
 // Workspace of a lattice of nblk blocks with 16 slots each; a plan uses what
 // it is given, 32 slots a block where they fit.
 size_t lat_bytes(size_t nblk);
