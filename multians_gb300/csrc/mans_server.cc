@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "mans_arena.h"
+#include "mans_copy.cuh"
 #include "multians_gb300.h"
 
 namespace {
@@ -61,13 +62,18 @@ uint64_t clock_ns() {
 
 uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 
-bool is_pinned_host(const void* p) {
+// Whether p is pinned host memory, and the address kernels reach it at (null
+// if they do not).
+bool is_pinned_host(const void* p, void** device) {
     cudaPointerAttributes a;
+    *device = nullptr;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeHost;
+    if (a.type != cudaMemoryTypeHost) return false;
+    *device = a.devicePointer;
+    return true;
 }
 
 struct Table {
@@ -94,6 +100,7 @@ struct Req {
     bool checked = false;
     int check_rc = 0;
     bool host_in = false, host_out = false, pinned_out = false;
+    void *dev_in = nullptr, *dev_out = nullptr;   // small pinned buffers: copied by k_copy_list
     bool taken = false;            // chosen for the batch being built
     mans_stream_desc d{};
     char* slice = nullptr;
@@ -249,7 +256,10 @@ struct mans_server {
         const bool dev = (r.flags & MANS_REQ_DEVICE_IO) != 0;
         if (dev && ((uintptr_t) r.units & 15) != 0) return MANS_ERR_ARG;
         q->host_in = q->host_out = !dev;
-        q->pinned_out = q->host_out && is_pinned_host(r.out);
+        q->pinned_out = q->host_out && is_pinned_host(r.out, &q->dev_out);
+        if (r.n_out > mans::kCopyBytesMax) q->dev_out = nullptr;
+        if (q->host_in && r.n_units * 4 <= mans::kCopyBytesMax && ((uintptr_t) r.units & 3) == 0)
+            is_pinned_host(r.units, &q->dev_in);
         mans_stream_desc d{};
         d.d_units = dev ? r.units : (const uint32_t*) (uintptr_t) 256;   // sizing only
         d.n_units = r.n_units;
@@ -277,8 +287,25 @@ struct mans_server {
         return false;
     }
 
+    // Starts the input copies collected for a size class.
+    void flush(mans::CopyList& l, std::vector<Req*>& reqs, int cls) {
+        if (mans::copy_list(l, copy_stream[cls]) != cudaSuccess) {
+            cudaGetLastError();
+            for (Req* q : reqs) drop_ready(q, MANS_ERR_CUDA);
+        }
+        l.n = 0;
+        reqs.clear();
+    }
+
     // Admits queued requests in arrival order while their blocks fit.
     bool admit() {
+        mans::CopyList list[2];
+        std::vector<Req*> listed[2];
+        const bool progress = admit(list, listed);
+        for (int c = 0; c < 2; ++c) flush(list[c], listed[c], c);
+        return progress;
+    }
+    bool admit(mans::CopyList (&list)[2], std::vector<Req*> (&listed)[2]) {
         bool progress = false;
         while (!pending.empty()) {
             Req* q = pending.front();
@@ -323,7 +350,8 @@ struct mans_server {
             if (q->host_in) {
                 q->d.d_units = (const uint32_t*) p;
                 p += align256(q->r.n_units * 4);
-                if (cudaMemcpyAsync((void*) q->d.d_units, q->r.units, q->r.n_units * 4,
+                if (!q->dev_in &&
+                    cudaMemcpyAsync((void*) q->d.d_units, q->r.units, q->r.n_units * 4,
                                     cudaMemcpyHostToDevice, copy_stream[size_class(q)]) !=
                     cudaSuccess) {
                     cudaGetLastError();
@@ -335,6 +363,13 @@ struct mans_server {
             if (q->host_out) q->d.d_out = (uint8_t*) p;
             q->admit = clock_ns();
             ready.push_back(q);
+            if (q->dev_in) {
+                const int cls = size_class(q);
+                if (list[cls].n == mans::kCopyItems) flush(list[cls], listed[cls], cls);
+                list[cls].item[list[cls].n++] = {(const uint8_t*) q->dev_in,
+                                                 (uint8_t*) q->d.d_units, q->r.n_units * 4};
+                listed[cls].push_back(q);
+            }
             progress = true;
         }
         return progress;
@@ -413,13 +448,18 @@ struct mans_server {
                                          hbytes, slices.data(), s->stream, &b);
         if (rc == MANS_OK) rc = mans_batch_decode(b, s->stream);
         if (rc == MANS_OK) {
-            for (size_t i = 0; i < n; ++i) {
+            mans::CopyList list;
+            for (size_t i = 0; i < n && rc == MANS_OK; ++i) {
                 Req* q = take[i];
-                if (q->pinned_out &&
-                    cudaMemcpyAsync(q->r.out, q->d.d_out, q->r.n_out, cudaMemcpyDeviceToHost,
-                                    s->stream) != cudaSuccess) {
+                if (q->dev_out)
+                    list.item[list.n++] = {q->d.d_out, (uint8_t*) q->dev_out, q->r.n_out};
+                else if (q->pinned_out &&
+                         cudaMemcpyAsync(q->r.out, q->d.d_out, q->r.n_out, cudaMemcpyDeviceToHost,
+                                         s->stream) != cudaSuccess)
                     rc = MANS_ERR_CUDA;
-                    break;
+                if (list.n == mans::kCopyItems || i + 1 == n) {
+                    if (mans::copy_list(list, s->stream) != cudaSuccess) rc = MANS_ERR_CUDA;
+                    list.n = 0;
                 }
             }
         }
@@ -578,15 +618,17 @@ int mans_server_create(const mans_server_cfg* cfg, mans_server** out) {
         cudaFree(s->base);
         return rc;
     };
+    int least = 0, greatest = 0;
+    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return fail(MANS_ERR_CUDA);
+    // copies by kernel do not wait behind a decode's queued blocks either
     for (int i = 0; i < 2; ++i)
-        if (cudaStreamCreateWithFlags(&s->copy_stream[i], cudaStreamNonBlocking) != cudaSuccess ||
+        if (cudaStreamCreateWithPriority(&s->copy_stream[i], cudaStreamNonBlocking, greatest) !=
+                cudaSuccess ||
             cudaEventCreateWithFlags(&s->copy_ev[i], cudaEventDisableTiming) != cudaSuccess)
             return fail(MANS_ERR_CUDA);
     // the small-request slot first (it is offered the ready requests first),
     // on a stream of the highest priority: its blocks are scheduled ahead of
     // the waiting blocks of the larger batches' kernels
-    int least = 0, greatest = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess) return fail(MANS_ERR_CUDA);
     for (uint32_t i = s->small_bytes ? 0 : 1; i <= s->max_inflight; ++i) {
         auto sl = std::make_unique<Slot>();
         sl->srv = s.get();
