@@ -62,18 +62,31 @@ uint64_t clock_ns() {
 
 uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 
-// Whether p is pinned host memory, and the address kernels reach it at (null
-// if they do not).
-bool is_pinned_host(const void* p, void** device) {
+// Whether p is pinned host memory.
+bool is_pinned_host(const void* p) {
     cudaPointerAttributes a;
-    *device = nullptr;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    if (a.type != cudaMemoryTypeHost) return false;
-    *device = a.devicePointer;
-    return true;
+    return a.type == cudaMemoryTypeHost;
+}
+
+// The address kernels reach a buffer at, if it is pinned host memory from its
+// first byte to its last and small enough to be copied by k_copy_list (null if
+// not: a buffer that is registered in part stays with the copy engine).
+void* kernel_address(const void* p, uint64_t bytes) {
+    if (bytes == 0 || bytes > mans::kCopyBytesMax) return nullptr;
+    cudaPointerAttributes a, z;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+        cudaPointerGetAttributes(&z, (const char*) p + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer ||
+        (char*) z.devicePointer != (char*) a.devicePointer + (bytes - 1))
+        return nullptr;
+    return a.devicePointer;
 }
 
 struct Table {
@@ -256,10 +269,10 @@ struct mans_server {
         const bool dev = (r.flags & MANS_REQ_DEVICE_IO) != 0;
         if (dev && ((uintptr_t) r.units & 15) != 0) return MANS_ERR_ARG;
         q->host_in = q->host_out = !dev;
-        q->pinned_out = q->host_out && is_pinned_host(r.out, &q->dev_out);
-        if (r.n_out > mans::kCopyBytesMax) q->dev_out = nullptr;
-        if (q->host_in && r.n_units * 4 <= mans::kCopyBytesMax && ((uintptr_t) r.units & 3) == 0)
-            is_pinned_host(r.units, &q->dev_in);
+        q->pinned_out = q->host_out && is_pinned_host(r.out);
+        if (q->pinned_out) q->dev_out = kernel_address(r.out, r.n_out);
+        if (q->host_in && ((uintptr_t) r.units & 3) == 0)
+            q->dev_in = kernel_address(r.units, r.n_units * 4);
         mans_stream_desc d{};
         d.d_units = dev ? r.units : (const uint32_t*) (uintptr_t) 256;   // sizing only
         d.n_units = r.n_units;
