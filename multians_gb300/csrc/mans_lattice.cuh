@@ -211,31 +211,31 @@ __device__ __forceinline__ void lat_load_table(uint32_t tb, const uint32_t* __re
 // ---------------------------------------------------------------------------
 // cursor
 
-__device__ __forceinline__ uint32_t lat_mask4(uint32_t e) {
-    uint32_t m;   // k ones from bit 2, k = the low five bits of e
-    asm("bmsk.wrap.b32 %0, %1, %2;" : "=r"(m) : "r"(2u), "r"(e));
-    return m;
+// Shared address of the state after entry e: its address field and 4 b, b = the
+// low k bits of window w.  One instruction (k is the low five bits of e)
+// instead of a mask and an AND: it lies on the chain from lookup to lookup,
+// which is what a trajectory's time consists of.
+__device__ __forceinline__ uint32_t lat_next(uint32_t e, uint32_t w) {
+    uint32_t b;
+    asm("szext.wrap.u32 %0, %1, %2;" : "=r"(b) : "r"(w), "r"(e));
+    return (e >> 16) + 4 * b;
 }
 
 // Bit cursor over units in a lane's column of a warp-wide shared tile: unit
 // slot i of the lane lies at column + 128 i, so the 32 lanes of a warp read
-// 32 different banks wherever their cursors stand.  Units are stored
-// shifted up by two bits (the two top bits of the unit before below them):
-// the extracted window then holds the code's b at bit 2 and the next
-// entry's address is the entry's address field plus the masked window, no
-// shift between the lookups.  `pos` counts bits with the slot of the next
-// unit a refill takes at (pos >> 5): it is 64 bits ahead of the codeword.
+// 32 different banks wherever their cursors stand.  `pos` counts bits with the
+// slot of the next unit a refill takes at (pos >> 5): it is 64 bits ahead of
+// the codeword.
 struct LatCursor {
     uint32_t a, e;       // shared address of the current state's entry, the entry
-    uint32_t w0, w1;     // shifted units under the cursor
+    uint32_t w0, w1;     // units under the cursor
     uint32_t pos;
 
     // One step; `mask` = (slots - 1) * 32.  Returns the entry stepped over.
     __device__ __forceinline__ uint32_t step(uint32_t col, uint32_t mask) {
         const uint32_t u = lds32(col + ((pos & mask) << 2));
         const uint32_t y = e;
-        const uint32_t b4 = __funnelshift_r(w0, w1, pos) & lat_mask4(y);
-        a = (y >> 16) + b4;
+        a = lat_next(y, __funnelshift_r(w0, w1, pos));
         e = lds32(a);
         const uint32_t np = __dp4a(y, 1u, pos);   // + byte 0
         const bool r = ((np ^ pos) & 32u) != 0;   // k <= 16: at most one unit
@@ -271,13 +271,13 @@ __device__ __forceinline__ void lat_pair(LatCursor& c, uint32_t col, uint32_t ma
     m.w1 = c.w1;
     m.base = c.pos;
     y1 = c.e;
-    m.a = (y1 >> 16) + (__funnelshift_r(c.w0, c.w1, c.pos) & lat_mask4(y1));
+    m.a = lat_next(y1, __funnelshift_r(c.w0, c.w1, c.pos));
     m.e = lds32(m.a);
     m.pos = __dp4a(y1, 1u, c.pos);
     const uint32_t o = __dp4a(y1, 1u, c.pos & 31u);
     const uint32_t x = (uint32_t) ((((unsigned long long) c.w1 << 32) | c.w0) >> o);
     y2 = m.e;
-    c.a = (y2 >> 16) + (x & lat_mask4(y2));
+    c.a = lat_next(y2, x);
     c.e = lds32(c.a);
     c.pos = __dp4a(y2, 1u, m.pos);
     const bool r = ((c.pos ^ m.base) & 32u) != 0;
@@ -346,18 +346,11 @@ __device__ __forceinline__ void lat_load_units(uint32_t (&r)[kB], const uint32_t
     }
 }
 
-// Stores a block's units, shifted, from unit slot `s` of the lane's column;
-// `carry` is the unit before the first, the last unit on return.
+// Stores units from unit slot `s` of the lane's column.
 template <uint32_t kB>
-__device__ __forceinline__ void lat_store_units(const uint32_t (&r)[kB], uint32_t col, uint32_t s,
-                                                uint32_t& carry) {
-    uint32_t c = carry;
+__device__ __forceinline__ void lat_store_units(const uint32_t (&r)[kB], uint32_t col, uint32_t s) {
 #pragma unroll
-    for (uint32_t i = 0; i < kB; ++i) {
-        sts32(col + (s + i) * 128, __funnelshift_l(c, r[i], 2));
-        c = r[i];
-    }
-    carry = c;
+    for (uint32_t i = 0; i < kB; ++i) sts32(col + (s + i) * 128, r[i]);
 }
 
 // Shared memory of a sync-pass CTA: the table, then per warp a ring of two
@@ -412,25 +405,24 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
     uint32_t prev = 0;          // node of the block before: its index in the arrays fits 32 bits
     uint32_t pcnt = 0;          // symbols from there to block b
     bool has_prev = false, first = false;   // first: the true start's trajectory
-    uint32_t carry = 0, life = 0, max_life = 0, visits = 0;
+    uint32_t life = 0, max_life = 0, visits = 0;
     uint32_t nx[kB];            // units of block b + 2, in flight
     uint32_t room = blockDim.x; // lanes the CTA's trajectories are spread over
 
     // the cursor at entry `val` of block b
     const auto begin = [&]() {
         const uint32_t rel = val & 0xffu, s = (b & 1u) * kB;
-        carry = 0;
         if (kB <= 16) {   // both blocks' loads in flight together
             uint32_t r0[kB];
             lat_load_units<kB>(r0, p.units, p.n_units, b, wide);
             lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
-            lat_store_units<kB>(r0, col, s, carry);
+            lat_store_units<kB>(r0, col, s);
         } else {
             lat_load_units<kB>(nx, p.units, p.n_units, b, wide);
-            lat_store_units<kB>(nx, col, s, carry);
+            lat_store_units<kB>(nx, col, s);
             lat_load_units<kB>(nx, p.units, p.n_units, b + 1, wide);
         }
-        lat_store_units<kB>(nx, col, s ^ kB, carry);
+        lat_store_units<kB>(nx, col, s ^ kB);
         lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
         c.pos = s * 32 + rel + 64;
         be = s * 32 + kBits + 64;
@@ -579,7 +571,7 @@ __device__ __forceinline__ void lat_sync_body(const LatParams& p, uint32_t* next
         cas = lat_cas(knext + q, val);
         // block b + 1 (one ahead again) into the half of the ring that is free
         const uint32_t s = (b & 1u) * kB;      // slots of block b
-        lat_store_units<kB>(nx, col, s ^ kB, carry);
+        lat_store_units<kB>(nx, col, s ^ kB);
         lat_load_units<kB>(nx, p.units, p.n_units, b + 2, wide);
         if (s == 0) c.pos -= 2 * kBits;
         be = s * 32 + kBits + 64;
@@ -632,7 +624,7 @@ __device__ __forceinline__ void lat_fill_rows(uint32_t tile, const LatParams& p,
 template <uint32_t kB>
 __device__ __forceinline__ void lat_turn_rows(uint32_t tile, uint32_t lane) {
     constexpr uint32_t kRow = lat_row_words(kB) * 4;
-    uint32_t r[kB + 4], carry = 0;
+    uint32_t r[kB + 4];
     const uint32_t row = tile + lane * kRow;
 #pragma unroll
     for (uint32_t i = 0; i < kB + 4; i += 4)
@@ -640,7 +632,7 @@ __device__ __forceinline__ void lat_turn_rows(uint32_t tile, uint32_t lane) {
                      : "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3])
                      : "r"(i < kB ? row + i * 4 : row + kRow) : "memory");
     __syncwarp();
-    lat_store_units<kB + 4>(r, tile + lane * 4, 0, carry);
+    lat_store_units<kB + 4>(r, tile + lane * 4, 0);
     __syncwarp();
 }
 
