@@ -27,6 +27,8 @@
 // first codewords at each bit position, which is all the sync logic needs.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace mans {
@@ -60,6 +62,35 @@ __device__ __forceinline__ void load_prepared(uint2* s_tab, const uint2* __restr
 
 __device__ __forceinline__ uint32_t entry_index(uint32_t a, uint32_t tab_base) {
     return (a - tab_base) >> 3;
+}
+
+// Kernels of one call that follow each other on a stream may be launched while
+// the one before still runs (programmatic dependent launch): a kernel lets the
+// next one in as soon as all its CTAs have started, and waits for the end of
+// the one before, and its writes, ahead of everything else.  Both are no-ops
+// where the launch does not ask for it.
+__device__ __forceinline__ void follow_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launches k; `early`: before the kernel ahead of it on the stream has ended.
+// For short calls, of which the time between kernels is a part: CTAs that wait
+// would take room from other streams under a long kernel.
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*k)(P...), unsigned grid, unsigned threads, size_t smem,
+                                cudaStream_t st, bool early, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k, P(args)...);
 }
 
 }  // namespace mans

@@ -38,6 +38,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "mans_device.cuh"
 #include "mans_lattice_scan.cuh"
 #include "mans_tma.cuh"
 #include "multians_gb300.h"
@@ -224,6 +225,7 @@ __host__ __device__ constexpr uint32_t enc_row_bytes(uint32_t Bs) { return Bs + 
 template <uint32_t kBs>
 __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
     extern __shared__ __align__(16) uint32_t enc_sm[];
+    follow_previous();
     const uint32_t tb = smem_addr(enc_sm);
     load_enc_tables(tb, p.blob, p.L);
     const uint32_t lane = threadIdx.x & 31;
@@ -339,12 +341,14 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
 template <uint32_t kD>
 __global__ void __launch_bounds__(kLatScanThreads) k_enc_scan(EncParams p) {
     __shared__ uint32_t s_tile;
+    follow_previous();
     if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
     lat_scan_body<EncParams, kD>(p, s_tile);
 }
 
 __global__ void __launch_bounds__(256) k_enc_zero(uint4* a, size_t na, uint32_t* units, size_t nu) {
+    follow_previous();
     const size_t stride = (size_t) gridDim.x * blockDim.x;
     const size_t t = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t i = t; i < na; i += stride) a[i] = make_uint4(0, 0, 0, 0);
@@ -376,6 +380,7 @@ __host__ __device__ constexpr uint32_t enc_stage_words(uint32_t Bs, uint32_t lg)
 template <uint32_t kBs>
 __global__ void __launch_bounds__(kEncFinalThreads) k_enc_final(EncParams p) {
     extern __shared__ __align__(16) uint32_t enc_sm[];
+    follow_previous();
     if (*(volatile uint32_t*) p.status & (MANS_DEV_SYNC_OVERFLOW | MANS_DEV_SCAN_TIMEOUT |
                                           MANS_DEV_COUNT_MISMATCH))
         return;
@@ -666,6 +671,7 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
     const size_t words = lay.zero_end / 16 + cap_units / 4;
     const unsigned gz = (unsigned) std::min<size_t>((words + 1023) / 1024, 4 * sms);
     k_enc_zero<<<gz, 256, 0, st>>>((uint4*) base, lay.zero_end / 16, d_units, cap_units);
+    const bool early = e.nseed <= 64 * sms;   // narrow warps below
     {
         // few trajectories: narrow warps spread over the schedulers of all SMs
         uint32_t th = kEncThreads;
@@ -675,11 +681,10 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
         const unsigned grid = std::min<unsigned>((e.nseed + per_cta - 1) / per_cta,
                                                  sms * kEncCtas * (kEncThreads / th));
         const size_t sm = enc_sync_smem(L, e.Bs, th);
-        if (e.Bs == 64) k_enc_sync<64><<<grid, th, sm, st>>>(p);
-        else k_enc_sync<128><<<grid, th, sm, st>>>(p);
+        launch_after(e.Bs == 64 ? k_enc_sync<64> : k_enc_sync<128>, grid, th, sm, st, early, p);
     }
-    k_enc_scan<kEncSlots><<<(e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
-                               lat_scan_smem(mans_encode_blob_words(L)), st>>>(p);
+    launch_after(k_enc_scan<kEncSlots>, (e.nblk + kLatScanTile - 1) / kLatScanTile, kLatScanThreads,
+                 lat_scan_smem(mans_encode_blob_words(L)), st, early, p);
     {
         const unsigned groups = (e.nblk + 31) / 32;
         uint32_t th = kEncFinalThreads;
@@ -691,7 +696,7 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
             per_sm < 1)
             per_sm = 1;
         const unsigned need = (groups + th / 32 - 1) / (th / 32);
-        k<<<std::min<unsigned>(need, (unsigned) per_sm * sms), th, sm, st>>>(p);
+        launch_after(k, std::min<unsigned>(need, (unsigned) per_sm * sms), th, sm, st, early, p);
     }
     return cudaGetLastError() == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }

@@ -15,6 +15,7 @@ constexpr size_t kLatZeroBytes = 128 * 1024;   // zeroed by a CTA
 
 // Tables (first CTA) and the zeroed words: counters, look-back words, slots.
 __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep(LatParams p, uint4* zero, size_t n16) {
+    follow_previous();
     if (blockIdx.x == 0) lat_tables(p);
     const size_t stride = (size_t) gridDim.x * blockDim.x;
     for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride)
@@ -26,12 +27,14 @@ constexpr uint32_t lat_ahead(uint32_t D, bool narrow) { return D > 16 ? 4 : (nar
 
 template <uint32_t kB, bool kNarrow, uint32_t kV>
 __global__ void __launch_bounds__(kLatThreads) k_lat_sync(LatParams p) {
+    follow_previous();
     lat_sync_body<kB, kNarrow, kV>(p, p.ctr + kLatNext, p.nseed);
 }
 
 template <uint32_t kD>
 __global__ void __launch_bounds__(kLatScanThreads, kD > 16 ? 2 : 5) k_lat_scan(LatParams p) {
     __shared__ uint32_t s_tile;
+    follow_previous();
     if (threadIdx.x == 0) s_tile = atomicAdd(p.ctr + kLatTicket, 1u);
     __syncthreads();
     lat_scan_body<LatParams, kD>(p, s_tile);
@@ -39,6 +42,7 @@ __global__ void __launch_bounds__(kLatScanThreads, kD > 16 ? 2 : 5) k_lat_scan(L
 
 template <bool kRev, uint32_t kB>
 __global__ void __launch_bounds__(kLatFinalThreads) k_lat_final(LatParams p) {
+    follow_previous();
     lat_final_body<kRev, kB>(p, blockIdx.x, gridDim.x);
 }
 
@@ -368,26 +372,28 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
                                                         2 * sms - 1);
     k_lat_prep<<<gz, kLatPrepThreads, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
     mark(1, st);
+    const uint32_t width = lat_width(plan.nseed, sms);
+    const bool early = width < 32;   // short: the sync pass leaves room beside it
     // sync pass
     {
-        const uint32_t width = lat_width(plan.nseed, sms);
         const uint32_t th = plan.nseed <= width * 4 * sms ? 32 : kLatThreads;
         p.width = width;
         const unsigned need = (plan.nseed + (th / 32) * width - 1) / ((th / 32) * width);
         const unsigned grid = std::min<unsigned>(need, (unsigned) sms * kLatCtas * (kLatThreads / th));
         const size_t sm = lat_sync_smem(call.L, plan.B, th);
-        sync_kernel(plan.B, plan.D, width < 32)<<<grid, th, sm, st>>>(p);
+        launch_after(sync_kernel(plan.B, plan.D, width < 32), grid, th, sm, st, early, p);
     }
     mark(2, st);
     mark(3, st);
     {
         const unsigned g = (plan.nblk + kLatScanTile - 1) / kLatScanTile;
         const size_t sm = lat_scan_smem(call.L);
-        if (plan.D == 4) k_lat_scan<4><<<g, kLatScanThreads, sm, st>>>(p);
-        else if (plan.D == 8) k_lat_scan<8><<<g, kLatScanThreads, sm, st>>>(p);
-        else if (plan.D == 12) k_lat_scan<12><<<g, kLatScanThreads, sm, st>>>(p);
-        else if (plan.D == 16) k_lat_scan<16><<<g, kLatScanThreads, sm, st>>>(p);
-        else k_lat_scan<32><<<g, kLatScanThreads, sm, st>>>(p);
+        auto* k = plan.D == 4    ? k_lat_scan<4>
+                  : plan.D == 8  ? k_lat_scan<8>
+                  : plan.D == 12 ? k_lat_scan<12>
+                  : plan.D == 16 ? k_lat_scan<16>
+                                 : k_lat_scan<32>;
+        launch_after(k, g, kLatScanThreads, sm, st, early, p);
     }
     mark(4, st);
     {
@@ -402,7 +408,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
             per_sm < 1)
             per_sm = 1;
         const unsigned need = (groups + th / 32 - 1) / (th / 32);
-        k<<<std::min<unsigned>(need, (unsigned) (per_sm * sms)), th, sm, st>>>(p);
+        launch_after(k, std::min<unsigned>(need, (unsigned) (per_sm * sms)), th, sm, st, early, p);
     }
     mark(5, st);
     return cudaGetLastError() == cudaSuccess ? 4u : 0u;
