@@ -495,6 +495,10 @@ __global__ void __launch_bounds__(kEncFinalThreads) k_enc_final(EncParams p) {
     }
 }
 
+// Bytes of a histogram CTA at least (256 KB: one CTA for 100 KB, 10.8 us, and
+// half a wave for 64 MB, 25 us).
+constexpr size_t kHistBytes = 16 * 1024;
+
 // Byte histogram: per-CTA counts in shared memory (one copy per warp, so
 // lanes of different warps do not contend), merged into 64-bit totals.
 __global__ void __launch_bounds__(256) k_hist(const uint8_t* __restrict__ sym,
@@ -748,7 +752,7 @@ int mans_histogram(const uint8_t* d_sym, size_t n, uint64_t* d_hist, void* strea
     cudaStream_t st = (cudaStream_t) stream;
     if (cudaMemsetAsync(d_hist, 0, 256 * sizeof(uint64_t), st) != cudaSuccess) return MANS_ERR_CUDA;
     if (n == 0) return MANS_OK;
-    const unsigned grid = (unsigned) std::min<size_t>((n + 256 * 1024 - 1) / (256 * 1024), 152 * 8);
+    const unsigned grid = (unsigned) std::min<size_t>((n + kHistBytes - 1) / kHistBytes, 152 * 8);
     k_hist<<<grid, 256, 0, st>>>(d_sym, n, (unsigned long long*) d_hist);
     return cudaGetLastError() == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }
