@@ -213,19 +213,24 @@ def make_workload(args, rank):
     return st, time.time() - t0
 
 
-def profile_figures(workload: str, captured: bool):
+def profile_figures(workload: str, captured: bool, lattice: bool = False):
     """The committed ncu figures of a plain workload (profiles/traffic_*.txt
     and profiles/issue_*.txt, tab-separated rows): the kernel
     each timing slot of the decode stands for (with symbol capture the
-    final-pass slot is the copy pass), DRAM bytes per launch and instruction
-    issue utilisation (% of cycles) by kernel.  Rows are keyed by kernel,
-    workload and capture mode; where no profile of that workload and mode
+    final-pass slot is the copy pass; a lattice decode's sync pass is timed
+    in k_gwalk's slot, k_wwalk's is empty), DRAM bytes per launch and
+    instruction issue utilisation (% of cycles) by kernel.  Rows are keyed by
+    kernel, workload and mode; where no profile of that workload and mode
     is committed the dictionaries are empty (the bench line then says null,
     not another kernel's figure)."""
     key = workload + (" capture" if captured else " no-capture")
     kernel_of = ({"k_gwalk": "k_gwalk<1>", "k_wwalk": "k_wwalk<1>", "k_final": "k_copy<0>"}
                  if captured else
                  {"k_gwalk": "k_gwalk<0>", "k_wwalk": "k_wwalk<0>", "k_final": "k_final<0>"})
+    if lattice:
+        key = workload + " lattice"
+        kernel_of = {"k_prep": "k_lat_prep", "k_gwalk": "k_lat_sync", "k_scan": "k_lat_scan",
+                     "k_final": "k_lat_final"}
 
     def rows(prefix):
         out = {}
@@ -490,12 +495,13 @@ def run_ours(args, ws, rank, local):
     # algorithmic bytes; k_final writes the symbols (and without capture
     # reads the stream again; with capture it reads the captured symbols,
     # which like the G pass's capture writes are overhead)
-    captured = cfg.get("capture_bytes", 0) > 0
+    lattice = bool(cfg.get("flags", 0) & mg.DECODE_LATTICE)
+    captured = cfg.get("capture_bytes", 0) > 0 and not lattice
     alg = {"k_gwalk": comp_bytes, "k_wwalk": 0, "k_final": n if captured else comp_bytes + n,
            "k_prep": st.L * 4, "k_scan": 0}[dom]
     achieved = alg / (mean_k[dom] / 1e3) / 1e9
     wl = f"plain {args.mb:g}MiB lambda={args.lam} L={args.L}"
-    kernel_of, t_rows, issue, inst = profile_figures(wl, captured)
+    kernel_of, t_rows, issue, inst = profile_figures(wl, captured, lattice)
     traffic = t_rows.get(kernel_of.get(dom))
     per_sorted = sorted(per_ms)
     cpu = None

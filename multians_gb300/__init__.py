@@ -17,6 +17,7 @@ from ._lib import (  # noqa: F401
     DEV_DEGENERATE,
     DEV_COUNT_MISMATCH,
     DECODE_SOURCE_ORDER,
+    DECODE_LATTICE,
     DECODE_NO_CAPTURE,
     DECODE_CAPTURE,
     PLAN_MODEL,

@@ -39,6 +39,7 @@ class MansError(RuntimeError):
 
 DECODE_SOURCE_ORDER = 0x1
 DECODE_NO_CAPTURE = 0x2
+DECODE_LATTICE = 0x80
 DECODE_CAPTURE = 0x4
 DECODE_START_OFFSET = 0x10
 DECODE_SEEDS = 0x20
