@@ -3532,8 +3532,6 @@ int mans_batch_decode(mans_batch* b, void* stream) {
     const void* lps = b->base + L.lat_params;
     const LatItem* litems = (const LatItem*) (b->base + L.lat_items);
     const bool regions = L.n_items != 0;
-    // short: the sync pass leaves room beside it, and nothing stands between
-    const bool early = !regions && L.lat_width < 32;
     timing_mark(0, st);
     if (regions) k_prep_batch<<<b->n, 1024, L.smem_prep, st>>>(ps);
     lat_batch_prep(lps, litems, L.n_lprep, L.lat_smem, st);
@@ -3543,7 +3541,7 @@ int mans_batch_decode(mans_batch* b, void* stream) {
         if (L.n_sync_c[c])
             k_gwalk_batch<<<(unsigned) L.n_sync_c[c], kSyncThreads, L.smem_sync_c[c], st>>>(
                 ps, items + at);
-    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, L.lat_width, L.lat_deep, early, st);
+    lat_batch_sync(lps, litems, L.n_lsync, L.lat_smem, L.lat_width, L.lat_deep, st);
     litems += L.n_lsync;
     timing_mark(2, st);
     if (L.n_walk) {
@@ -3558,8 +3556,7 @@ int mans_batch_decode(mans_batch* b, void* stream) {
     if (L.n_scan)
         k_scan_batch<<<(unsigned) L.n_scan, kScanThreads, 0, st>>>(
             ps, items + L.n_sync, (uint32_t*) (b->base + L.ticket));
-    lat_batch_scan(lps, litems, L.n_lscan, L.lat_smem, L.lat_deep,
-                   (uint32_t*) (b->base + L.ticket) + 3, early, st);
+    lat_batch_scan(lps, litems, L.n_lscan, L.lat_smem, L.lat_deep, (uint32_t*) (b->base + L.ticket) + 3, st);
     litems += L.n_lscan;
     timing_mark(4, st);
     if (L.n_final && L.any_capture)
@@ -3569,7 +3566,8 @@ int mans_batch_decode(mans_batch* b, void* stream) {
         if (L.n_final_c[c])
             k_final_batch<<<(unsigned) L.n_final_c[c], kFinalThreads, L.smem_final_c[c], st>>>(
                 ps, items + L.n_sync + L.n_scan + at);
-    lat_batch_final(lps, litems, L.n_lfinal_c, {L.lat_final_smem0, L.lat_smem.final}, early, st);
+    lat_batch_final(lps, litems, L.n_lfinal_c[0], L.lat_final_smem0, st);
+    lat_batch_final(lps, litems + L.n_lfinal_c[0], L.n_lfinal_c[1], L.lat_smem.final, st);
     timing_mark(5, st);
     if (g_timing.on && g_timing.used < g_timing.cap) ++g_timing.used;
     g_last_launches = (regions ? 1 : 0) + (L.n_lat ? 3 : 0) + (L.n_lfinal_c[0] ? 1 : 0) +

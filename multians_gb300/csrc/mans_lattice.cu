@@ -63,7 +63,6 @@ __device__ __forceinline__ void lat_load_params(LatParams& dst, const LatParams*
 __global__ void __launch_bounds__(kLatPrepThreads) k_lat_prep_batch(const LatParams* ps,
                                                                     const LatItem* items) {
     __shared__ LatParams sp;
-    follow_previous();
     const LatItem it = items[blockIdx.x];
     lat_load_params(sp, ps + it.stream);
     if (it.index == 0) {
@@ -91,7 +90,6 @@ __global__ void __launch_bounds__(kLatThreads) k_lat_sync_batch(const LatParams*
                                                                 const LatItem* items) {
     __shared__ LatParams sp;
     __shared__ uint32_t s_next;
-    follow_previous();
     const LatItem it = items[blockIdx.x];
     if (threadIdx.x == 0) s_next = it.index;
     lat_load_params(sp, ps + it.stream);
@@ -107,7 +105,6 @@ __global__ void __launch_bounds__(kLatScanThreads) k_lat_scan_batch(const LatPar
                                                                     uint32_t* ticket) {
     __shared__ LatParams sp;
     __shared__ uint32_t s_item;
-    follow_previous();
     if (threadIdx.x == 0) s_item = atomicAdd(ticket, 1u);
     __syncthreads();
     const LatItem it = items[s_item];
@@ -127,23 +124,14 @@ __device__ __forceinline__ void lat_final_any(const LatParams& p, const LatItem&
     else lat_final_body<kRev, 32>(p, it.index, it.count);
 }
 
-// index: the CTA of the stream's count.  kBeside: the list that follows
-// another list of the same pass, whose kernel has seen the scan's end and
-// shares nothing with this one: it runs beside that one and waits at its end
-// (one after the other, 14 + 21 us in a call of 48 streams).
-template <bool kBeside>
+// index: the CTA of the stream's count.
 __global__ void __launch_bounds__(kLatFinalThreads) k_lat_final_batch(const LatParams* ps,
                                                                       const LatItem* items) {
     __shared__ LatParams sp;
-    if (!kBeside) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
     const LatItem it = items[blockIdx.x];
     lat_load_params(sp, ps + it.stream);
     if (sp.flags & MANS_DECODE_SOURCE_ORDER) lat_final_any<true>(sp, it);
     else lat_final_any<false>(sp, it);
-    if (kBeside) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 static_assert(kLatThreads == 32 * kLatBatchWarps, "batch items");
@@ -232,8 +220,7 @@ void lat_attributes() {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int) kLatFinalSmemMax);
     };
-    set(k_lat_prep); set(k_lat_prep_batch);
-    set(k_lat_final_batch<false>); set(k_lat_final_batch<true>);
+    set(k_lat_prep); set(k_lat_prep_batch); set(k_lat_final_batch);
     set(batch_sync(false, false)); set(batch_sync(false, true));
     set(batch_sync(true, false)); set(batch_sync(true, true));
     for (uint32_t B = 4; B <= 32; B *= 2)
@@ -386,9 +373,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     k_lat_prep<<<gz, kLatPrepThreads, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
     mark(1, st);
     const uint32_t width = lat_width(plan.nseed, sms);
-    // short: the sync pass leaves room beside it (4 KB 75 -> 67 us; where it
-    // fills the GPU waiting CTAs cost more: 256 MB 541 -> 582, 16 MB 178 -> 185)
-    const bool early = width < 32;
+    const bool early = width < 32;   // short: the sync pass leaves room beside it
     // sync pass
     {
         const uint32_t th = plan.nseed <= width * 4 * sms ? 32 : kLatThreads;
@@ -483,26 +468,17 @@ void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSme
     if (n) k_lat_prep_batch<<<(unsigned) n, kLatPrepThreads, sm.prep, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t width, bool deep, bool early, cudaStream_t st) {
-    if (n)
-        launch_after(batch_sync(width < 32, deep), (unsigned) n, kLatThreads, sm.sync, st, early,
-                     (const LatParams*) ps, items);
+                    uint32_t width, bool deep, cudaStream_t st) {
+    if (n) batch_sync(width < 32, deep)<<<(unsigned) n, kLatThreads, sm.sync, st>>>((const LatParams*) ps, items);
 }
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    bool deep, uint32_t* ticket, bool early, cudaStream_t st) {
-    if (n)
-        launch_after(deep ? k_lat_scan_batch<true> : k_lat_scan_batch<false>, (unsigned) n,
-                     kLatScanThreads, sm.scan, st, early, (const LatParams*) ps, items, ticket);
+                    bool deep, uint32_t* ticket, cudaStream_t st) {
+    auto* k = deep ? k_lat_scan_batch<true> : k_lat_scan_batch<false>;
+    if (n) k<<<(unsigned) n, kLatScanThreads, sm.scan, st>>>((const LatParams*) ps, items, ticket);
 }
-void lat_batch_final(const void* ps, const LatItem* items, const size_t (&n)[2],
-                     const size_t (&smem)[2], bool early, cudaStream_t st) {
-    if (n[0])
-        launch_after(k_lat_final_batch<false>, (unsigned) n[0], kLatFinalThreads, smem[0], st, early,
-                     (const LatParams*) ps, items);
-    if (n[1])
-        launch_after(n[0] ? k_lat_final_batch<true> : k_lat_final_batch<false>, (unsigned) n[1],
-                     kLatFinalThreads, smem[1], st, n[0] || early, (const LatParams*) ps,
-                     items + n[0]);
+void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st) {
+    if (n)
+        k_lat_final_batch<<<(unsigned) n, kLatFinalThreads, smem, st>>>((const LatParams*) ps, items);
 }
 
 }  // namespace mans

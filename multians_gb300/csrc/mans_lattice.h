@@ -91,15 +91,12 @@ uint32_t lat_scan_tiles(const LatPlan& plan);
 uint32_t lat_final_ctas(const LatPlan& plan);
 LatSmem lat_batch_smem(const LatCall& call, const LatPlan& plan);
 void lat_batch_init();
-// early: launched before the kernel ahead has ended (nothing else may stand
-// between the passes on the stream).
 void lat_batch_prep(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
                     cudaStream_t st);
 void lat_batch_sync(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    uint32_t width, bool deep, bool early, cudaStream_t st);
+                    uint32_t width, bool deep, cudaStream_t st);
 void lat_batch_scan(const void* ps, const LatItem* items, size_t n, const LatSmem& sm,
-                    bool deep, uint32_t* ticket, bool early, cudaStream_t st);
-void lat_batch_final(const void* ps, const LatItem* items, const size_t (&n)[2],
-                     const size_t (&smem)[2], bool early, cudaStream_t st);
+                    bool deep, uint32_t* ticket, cudaStream_t st);
+void lat_batch_final(const void* ps, const LatItem* items, size_t n, size_t smem, cudaStream_t st);
 
 }  // namespace mans
