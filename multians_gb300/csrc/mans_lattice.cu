@@ -373,7 +373,9 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     k_lat_prep<<<gz, kLatPrepThreads, (size_t) call.L * 12, st>>>(p, (uint4*) (base + a.ctr), n16);
     mark(1, st);
     const uint32_t width = lat_width(plan.nseed, sms);
-    const bool early = width < 32;   // short: the sync pass leaves room beside it
+    // short: the sync pass leaves room beside it (4 KB 75 -> 67 us; where it
+    // fills the GPU waiting CTAs cost more: 256 MB 541 -> 582, 16 MB 178 -> 185)
+    const bool early = width < 32;
     // sync pass
     {
         const uint32_t th = plan.nseed <= width * 4 * sms ? 32 : kLatThreads;
