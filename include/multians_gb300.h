@@ -331,6 +331,10 @@ int mans_batch_create(const mans_stream_desc* streams, uint32_t n, const mans_cf
  * parameters are uploaded asynchronously on `stream`; the host images stay
  * in the batch object until mans_batch_destroy. */
 int mans_batch_slice_size(const mans_stream_desc* stream, const mans_cfg* hint, size_t* bytes);
+/* What each of n streams needs of its slice when they are decoded together
+ * (bytes[n]): never more than its mans_batch_slice_size. */
+int mans_batch_data_sizes(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hint,
+                          size_t* bytes);
 int mans_batch_header_size(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hint,
                            size_t* bytes);
 int mans_batch_create_split(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hint,

@@ -3018,6 +3018,7 @@ struct BatchStreamPlan {
     size_t data_off;     // offset of this stream's slice in the data region
     size_t flags_off;    // word offset of its scan flags in the flag array
     uint32_t stage_cap;
+    size_t own;          // its slice: the workspace of its own plan, whatever is beside it
     bool active;
     bool lattice;        // decoded by the lattice kernels (mans_lattice.h)
     int lat_class;
@@ -3047,9 +3048,19 @@ struct BatchLayout {
     uint32_t walk_grid;   // persistent merge-walk grid
 };
 
+// Region workspace of a stream planned with c.
+static size_t region_bytes(size_t n_units, const mans_cfg& c, size_t capture_bytes) {
+    const size_t nblk = num_blocks(n_units, c.block_units);
+    const size_t nreg = (nblk + c.region_blocks - 1) / c.region_blocks;
+    return layout_for(nblk, nreg, c.walk_slots, capture_bytes, false).total;
+}
+
+// Bytes of a stream's slice that its decode in this batch may touch: never
+// more than its own plan's (lattices are cut to that, regions lengthened only
+// where they then take no more), which is what mans_batch_slice_size gives.
 static size_t stream_data_bytes(const BatchStreamPlan& sp) {
     const AuxLayout a = layout_for(sp.nblk, sp.nreg, sp.cfg.walk_slots, sp.cfg.capture_bytes, false);
-    return sp.lattice ? std::max(a.total, sp.lat.bytes) : a.total;
+    return sp.lattice ? std::min(std::max(a.total, sp.lat.bytes), sp.own) : a.total;
 }
 
 static LatCall lat_call(const mans_stream_desc& d) {
@@ -3105,13 +3116,9 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
     const auto meet = [&](uint32_t i) {
         return mean_meeting_units(d[i].L, 32.0 * (double) d[i].n_units / (double) d[i].n_out);
     };
-    // a lattice stays in the workspace the stream's own plan has
-    const auto room = [&](uint32_t i) {
-        const mans_cfg& c = plans[i].cfg;
-        const size_t nblk = num_blocks(d[i].n_units, c.block_units);
-        return layout_for(nblk, (nblk + c.region_blocks - 1) / c.region_blocks, c.walk_slots, 0,
-                          false).total;
-    };
+    // a lattice stays in the workspace the stream's own plan has (less symbol
+    // capture, so within its slice)
+    const auto room = [&](uint32_t i) { return region_bytes(d[i].n_units, plans[i].cfg, 0); };
     for (uint32_t i = 0; i < n; ++i) {
         BatchStreamPlan& sp = plans[i];
         sp.active = d[i].n_out > 0;
@@ -3125,6 +3132,7 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
         const mans_cfg h = stream_hint(d[i]);
         int rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &sp.cfg);
         if (rc != MANS_OK) return rc;
+        sp.own = region_bytes(d[i].n_units, sp.cfg, sp.cfg.capture_bytes);
         if (free_hint && !(d[i].flags & MANS_DECODE_CAPTURE))
             // as many starts as its share of the batch's symbols has of the
             // lanes side by side
@@ -3178,8 +3186,12 @@ static int plan_batch(const mans_stream_desc* d, uint32_t n, const mans_cfg* hin
                     (uint32_t) std::max<uint64_t>(1, std::min<uint64_t>(want, d[i].n_units + B) / B) | 1u;
                 h.walk_slots = 0;
                 h.capture_bytes = 0;
-                rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &sp.cfg);
+                mans_cfg longer;
+                rc = mans_plan(d[i].n_units, d[i].n_out, d[i].L, &h, &longer);
                 if (rc != MANS_OK) return rc;
+                // with capture, rounding up to whole regions may cost more
+                if (region_bytes(d[i].n_units, longer, longer.capture_bytes) <= sp.own)
+                    sp.cfg = longer;
             }
         }
         sp.cfg.flags = d[i].flags & (MANS_DECODE_SOURCE_ORDER | MANS_DECODE_START_OFFSET);
@@ -3296,7 +3308,22 @@ int mans_batch_slice_size(const mans_stream_desc* stream, const mans_cfg* hint, 
     BatchLayout lay;
     int rc = plan_batch(stream, 1, hint, plans, lay);
     if (rc != MANS_OK) return rc;
-    *bytes = lay.total - lay.data;
+    *bytes = align256(plans[0].own);
+    return MANS_OK;
+}
+
+int mans_batch_data_sizes(const mans_stream_desc* streams, uint32_t n, const mans_cfg* hint,
+                          size_t* bytes) {
+    if (!streams || !bytes || n == 0) return MANS_ERR_ARG;
+    std::vector<BatchStreamPlan> plans;
+    BatchLayout lay;
+    int rc = plan_batch(streams, n, hint, plans, lay);
+    if (rc != MANS_OK) return rc;
+    for (uint32_t i = 0; i < n; ++i) {
+        const BatchStreamPlan& sp = plans[i];
+        bytes[i] = !sp.active ? 0 : sp.lattice ? std::max(sp.lat.bytes, stream_data_bytes(sp))
+                                               : stream_data_bytes(sp);
+    }
     return MANS_OK;
 }
 
