@@ -27,6 +27,7 @@
 // to completion; each launch slot keeps a preallocated header buffer
 // (parameters, work items, status and scan flags of one batch).  Nothing on
 // the request path calls cudaMalloc or cudaFree.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <time.h>
 
@@ -43,6 +44,7 @@
 
 #include "mans_arena.h"
 #include "mans_copy.cuh"
+#include "mans_pinned.h"
 #include "multians_gb300.h"
 
 namespace {
@@ -72,21 +74,34 @@ bool is_pinned_host(const void* p) {
     return a.type == cudaMemoryTypeHost;
 }
 
-// The address kernels reach a buffer at, if it is pinned host memory from its
-// first byte to its last and small enough to be copied by k_copy_list (null if
-// not: a buffer that is registered in part stays with the copy engine).
+// The address kernels reach a buffer at, if one pinned allocation or
+// registration holds all of it and it is small enough to be copied by
+// k_copy_list (null if not: it stays with the copy engine).  The driver's
+// entry point is asked for the range (59 ns; the runtime's query knows only
+// the byte it is given, so it would miss a hole between two registrations).
 void* kernel_address(const void* p, uint64_t bytes) {
-    if (bytes == 0 || bytes > mans::kCopyBytesMax) return nullptr;
-    cudaPointerAttributes a, z;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-        cudaPointerGetAttributes(&z, (const char*) p + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault,
+                                             &r) != cudaSuccess) {
+            cudaGetLastError();
+            return (Query) nullptr;
+        }
+        return r == cudaDriverEntryPointSuccess ? (Query) f : nullptr;
+    }();
+    if (bytes == 0 || bytes > mans::kCopyBytesMax || !query) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* into[4] = {&type, &dev, &start, &size};
+    if (query(4, what, into, (CUdeviceptr) p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST ||
+        dev != (CUdeviceptr) p || !mans::range_covers(start, size, (uint64_t) p, bytes))
         return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer ||
-        (char*) z.devicePointer != (char*) a.devicePointer + (bytes - 1))
-        return nullptr;
-    return a.devicePointer;
+    return (void*) dev;
 }
 
 struct Table {
