@@ -2115,8 +2115,8 @@ static void set_kernel_attributes() {
     if (dev < 64) done |= 1ull << dev;
 }
 
-// seeds: room for the seeded walks' records (plain decodes; batches run
-// without seeds)
+// seeds: room for the seeded walks' records (plain decodes that may run with
+// seeds; batches run without)
 static AuxLayout layout_for(size_t nblk, size_t nreg, size_t dmax, size_t cap_bytes,
                             bool seeds = true) {
     AuxLayout a;
@@ -2143,6 +2143,8 @@ static AuxLayout layout_for(size_t nblk, size_t nreg, size_t dmax, size_t cap_by
     a.total = o;
     return a;
 }
+
+static bool may_seed(const mans_cfg& c) { return !(c.flags & MANS_DECODE_NO_SEEDS); }
 
 static uint32_t pow2_floor(uint64_t x) {
     uint32_t r = 1;
@@ -2414,8 +2416,9 @@ size_t mans_aux_size(size_t n_units, const mans_cfg* cfg) {
         return 0;
     const size_t nblk = num_blocks(n_units, cfg->block_units);
     const size_t nreg = (nblk + cfg->region_blocks - 1) / cfg->region_blocks;
-    const size_t with_capture = layout_for(nblk, nreg, cfg->walk_slots, cfg->capture_bytes).total;
-    const size_t regions = layout_for(nblk, nreg, cfg->walk_slots, 0).total;
+    const size_t with_capture =
+        layout_for(nblk, nreg, cfg->walk_slots, cfg->capture_bytes, may_seed(*cfg)).total;
+    const size_t regions = layout_for(nblk, nreg, cfg->walk_slots, 0, may_seed(*cfg)).total;
     // a lattice decode with all its slots (less when it gives up slots)
     if ((cfg->flags & MANS_DECODE_LATTICE) && cfg->walk_slots == kMaxWalkSlots &&
         cfg->block_units >= 8)
@@ -2534,7 +2537,8 @@ static int decode_impl(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
     if (rc != MANS_OK) return rc;
     const size_t nblk = num_blocks(n_units, cfg.block_units);
     const size_t nreg = (nblk + cfg.region_blocks - 1) / cfg.region_blocks;
-    const AuxLayout lay = layout_for(nblk, nreg, cfg.walk_slots, cfg.capture_bytes);
+    const AuxLayout lay =
+        layout_for(nblk, nreg, cfg.walk_slots, cfg.capture_bytes, may_seed(cfg));
     if (aux_bytes < lay.total) return MANS_ERR_AUX_SMALL;
     if ((uint64_t) nblk * cfg.block_units * 32 >= (1ull << 40)) return MANS_ERR_ARG;
 
@@ -2809,7 +2813,8 @@ int mans_sync_stats_get(const void* d_aux, size_t aux_bytes, size_t n_units, siz
     if (rc != MANS_OK) return rc;
     const size_t nblk = num_blocks(n_units, cfg.block_units);
     const size_t nreg = (nblk + cfg.region_blocks - 1) / cfg.region_blocks;
-    const AuxLayout lay = layout_for(nblk, nreg, cfg.walk_slots, cfg.capture_bytes);
+    const AuxLayout lay =
+        layout_for(nblk, nreg, cfg.walk_slots, cfg.capture_bytes, may_seed(cfg));
     if (aux_bytes < lay.total) return MANS_ERR_AUX_SMALL;
     LatPlan lp;
     if (lattice_plan(cfg, n_units, n_out, L, aux_bytes, &lp)) {
@@ -3651,6 +3656,7 @@ int mans_batch_fixup(mans_batch* b, void* stream, uint32_t* n_redone) {
         const size_t slice_bytes = stream_data_bytes(sp);
         mans_cfg hint = sp.cfg;
         hint.region_blocks = sp.cfg.region_blocks * 4;   // longer regions, same slots
+        hint.flags |= MANS_DECODE_NO_SEEDS;              // for which a slice has no room
         uint32_t dev_status = 0;
         const int rc = mans_decode_sync(p.units, p.n_units, p.out, p.n_out, p.table, p.L,
                                         p.first_idx + p.L,
