@@ -113,10 +113,11 @@ typedef struct {
 /* Lattice decode, set by the planner in plans that fix no geometry, capture
  * or seeds: trajectories start at many places and each ends at the first
  * other one it meets (a chain several times shorter than a region and its
- * merge walk).  The plan's geometry and capture then stand for the decode
- * that follows when the path runs out of slots (MANS_DEV_SYNC_OVERFLOW) or
- * the workspace is too small for the lattice.  The output is identical
- * either way. */
+ * merge walk).  The plan's geometry and capture are those of the region
+ * decode that runs where the workspace is too small for the lattice; where
+ * the path runs out of slots (MANS_DEV_SYNC_OVERFLOW) the blocking calls
+ * decode by regions of four times that length, as after merge walks that
+ * did.  The output is identical either way. */
 #define MANS_DECODE_LATTICE 0x80u
 
 /* Fills `out` with the geometry the decoder uses for this call: the built-in

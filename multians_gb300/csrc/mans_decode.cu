@@ -2969,11 +2969,19 @@ int mans_decode_sync(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
         if (rc != MANS_OK) return rc;
         if (!(st & MANS_DEV_SYNC_OVERFLOW)) break;
         // a walk outran its slots: longer regions, same slot count (and a
-        // capture slice sized for them)
+        // capture slice sized for them).  After a lattice the region plan with
+        // its own slot count, as if it had failed as well (16 M of eight
+        // equal symbols, L = 1024: 34.7 -> 30.4 ms against a lattice's 16).
+        if (plan.flags & MANS_DECODE_LATTICE) {
+            c = plan;
+            c.flags &= ~MANS_DECODE_LATTICE;
+            c.walk_slots = hint ? hint->walk_slots : 0;
+            rc = mans_plan(n_units, n_out, L, &c, &plan);
+            if (rc != MANS_OK) return rc;
+        }
         c = plan;
         c.region_blocks = plan.region_blocks * 4;
         c.capture_bytes = 0;
-        c.flags &= ~MANS_DECODE_LATTICE;
     }
     if (status_out) *status_out = st;
     return mans_status_code(st);

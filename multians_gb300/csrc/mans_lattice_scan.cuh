@@ -291,7 +291,8 @@ struct LatTile {
 // until it meets a trajectory that has a slot, the tile is followed from
 // that node, and so on to its end.  Sequential work, so bounded: past
 // repair_blocks() over the whole stream the path is given up
-// (MANS_DEV_SYNC_OVERFLOW).  Later tiles wait for this one's end as always.
+// (MANS_DEV_SYNC_OVERFLOW), at once and not at the end of a stretch (16 M of
+// two symbols, L = 4096: 1024 blocks in one stretch, 38 ms).  Later tiles wait for this one's end as always.
 template <class P, uint32_t kD>
 __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
                                         typename LatTile<P, kD>::Shared& sh, uint32_t first) {
@@ -318,7 +319,9 @@ __device__ __noinline__ void lat_repair(const P& p, LatTile<P, kD>& tl,
         __syncthreads();
         if (threadIdx.x == 0) {
             uint32_t x = b, e = ent, slot = kNone;
-            while (x < stop) {
+            const uint32_t had = *(volatile uint32_t*) (p.ctr + kLatRepaired);
+            const uint32_t left = p.repair_blocks() > had ? p.repair_blocks() - had : 0;
+            while (x < stop && x - b <= left) {
                 unsigned long long n = 0;
                 s_over[x - first].x = e;
                 if (x + 1 < p.nblk) p.advance(lat_repair_sm, x, e, n);
