@@ -12,7 +12,11 @@ plan: units per block B in {4, 8, 16}, shortest region in mean merge
 distances m in {1.5, 2, 3, 4, 6, 8, 12}, symbol capture off / on (on only
 for L <= 4096, where its rings fit in shared memory).  Candidates that give
 the same geometry are timed once; a candidate whose merge walks run out of
-slots is dropped.  Each plan is timed with CUDA events over three decodes
+slots is dropped.  These are region plans: a lattice decode
+(MANS_DECODE_LATTICE), which plans that fix no geometry start with, has a
+geometry of its own, so the flag is taken off every candidate, and the table
+decides what runs where the lattice does not (a hint that rules it out, a
+workspace too small for it) or has given up.  Each plan is timed with CUDA events over three decodes
 after one warm-up, inputs resident in HBM; the fastest one is checked
 bit-exact against the source and written as the entry of (L, bits per
 symbol, size class) in the C header the planner compiles (mans_plan reads
@@ -68,6 +72,29 @@ def _time_plan(mg, st, units, table, out, aux, cfg, stream, reps=3):
     return e0.elapsed_time(e1) / reps
 
 
+def region_plan(mg, n_units, n, L, cfg):
+    """The plan's own region decode: without the lattice, and with the walk
+    slots its regions take."""
+    return mg.plan(n_units, n, L, dict(cfg, flags=cfg["flags"] & ~mg.DECODE_LATTICE, walk_slots=0))
+
+
+def candidates(mg, n_units, n, L):
+    """The candidate plans of a stream, one per geometry."""
+    cands, seen = [], set()
+    for cap in (False, True):
+        if cap and L > CAPTURE_MAX_L:
+            continue
+        for B in BLOCKS:
+            for m in MEET_MULTS:
+                cfg = region_plan(mg, n_units, n, L, mg.plan_tuned(n_units, n, L, B, m, cap))
+                key = (cfg["block_units"], cfg["region_blocks"], cfg["walk_slots"],
+                       cfg["capture_bytes"] > 0)
+                if key not in seen:
+                    seen.add(key)
+                    cands.append({"block_units": B, "meet_mult": m, "capture": cap, "cfg": cfg})
+    return cands
+
+
 def sweep_stream(mg, st, log):
     """Times every candidate plan on one stream; returns the record."""
     import torch
@@ -77,19 +104,7 @@ def sweep_stream(mg, st, log):
     units = torch.from_numpy(st.units.view(np.int32)).to(dev)
     table = torch.from_numpy(st.table.view(np.int32)).to(dev)
     out = torch.empty(max(1, st.n), dtype=torch.uint8, device=dev)
-    cands, seen = [], {}
-    for cap in (False, True):
-        if cap and st.L > CAPTURE_MAX_L:
-            continue
-        for B in BLOCKS:
-            for m in MEET_MULTS:
-                cfg = mg.plan_tuned(st.n_units, st.n, st.L, B, m, cap)
-                key = (cfg["block_units"], cfg["region_blocks"], cfg["walk_slots"],
-                       cfg["capture_bytes"] > 0)
-                if key in seen:
-                    continue
-                seen[key] = len(cands)
-                cands.append({"block_units": B, "meet_mult": m, "capture": cap, "cfg": cfg})
+    cands = candidates(mg, st.n_units, st.n, st.L)
     model = mg.plan(st.n_units, st.n, st.L, {"flags": mg.PLAN_MODEL})
     need = max([mg.aux_size(st.n_units, c["cfg"]) for c in cands] +
                [mg.aux_size(st.n_units, model)])
