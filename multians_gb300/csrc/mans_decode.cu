@@ -2467,21 +2467,38 @@ int mans_table_check(const uint32_t* t, uint32_t L) {
     return loops == (int) L ? 1 : -1;
 }
 
-// The plan a decode with these arguments runs with: the planner's, or the
-// same without symbol capture when capture was the planner's choice and
-// its slices do not fit the workspace (a workspace of mans_aux_size_max
-// bytes always suffices then).
+// The plan a decode with these arguments runs with: the planner's, or where
+// its own choices do not fit the workspace the first of these that does: a
+// lattice without room for symbol capture, regions with capture, regions
+// without (a workspace of mans_aux_size_max bytes always suffices for a
+// lattice or regions without capture).
 static int resolve_plan(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* cfg_in,
                         size_t aux_bytes, mans_cfg* cfg) {
     int rc = mans_plan(n_units, n_out, L, cfg_in, cfg);
-    if (rc != MANS_OK) return rc;
-    if (cfg->capture_bytes && !(cfg_in && cfg_in->capture_bytes) &&
-        mans_aux_size(n_units, cfg) > aux_bytes) {
-        mans_cfg h = cfg_in ? *cfg_in : mans_cfg{0, 0, 0, 0, 0, 0};
-        h.flags |= MANS_DECODE_NO_CAPTURE;
-        h.capture_bytes = 0;
+    if (rc != MANS_OK || mans_aux_size(n_units, cfg) <= aux_bytes) return rc;
+    const mans_cfg in = cfg_in ? *cfg_in : mans_cfg{0, 0, 0, 0, 0, 0};
+    const bool lattice = (cfg->flags & MANS_DECODE_LATTICE) && !(in.flags & MANS_DECODE_LATTICE);
+    const bool capture = cfg->capture_bytes && !in.capture_bytes;
+    const mans_cfg whole = *cfg;
+    const auto plan = [&](bool with_lattice, bool with_capture) {
+        mans_cfg h = in;
+        if (lattice && (with_lattice || with_capture == capture)) {   // the same geometry
+            h = whole;
+            if (!with_lattice) {
+                h.flags &= ~MANS_DECODE_LATTICE;
+                h.walk_slots = in.walk_slots;
+            }
+        }
+        if (!with_capture) {
+            h.flags |= MANS_DECODE_NO_CAPTURE;
+            h.capture_bytes = 0;
+        }
         rc = mans_plan(n_units, n_out, L, &h, cfg);
-    }
+        return rc != MANS_OK || mans_aux_size(n_units, cfg) <= aux_bytes;
+    };
+    if (lattice && capture && plan(true, false)) return rc;
+    if (lattice && plan(false, capture)) return rc;
+    if (capture) plan(false, false);
     return rc;
 }
 
@@ -2944,7 +2961,8 @@ int mans_decode_sync(const uint32_t* d_units, size_t n_units, uint8_t* d_out,
     mans_cfg plan;
     uint32_t st = 0;
     for (int attempt = 0; attempt < 8; ++attempt) {
-        int rc = mans_plan(n_units, n_out, L, &c, &plan);
+        int rc = attempt == 0 ? resolve_plan(n_units, n_out, L, &c, aux_bytes, &plan)
+                              : mans_plan(n_units, n_out, L, &c, &plan);
         if (rc != MANS_OK) return rc;
         if (mans_aux_size(n_units, &plan) > aux_bytes) {
             if (plan.capture_bytes) {
