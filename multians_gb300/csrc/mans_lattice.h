@@ -27,7 +27,8 @@ bool lat_plan(size_t n_units, size_t n_out, uint32_t L, double meet, uint32_t la
 
 // A short stream leaves the GPU idle and takes as long as its longest
 // trajectory, which ends sooner the more others it can meet: the geometry
-// with 32 slots a block and starts closer by a quarter at least.  False when
+// with 32 slots a block and starts closer by a quarter at least, on up to 512
+// scan tiles.  False when
 // there is none in `bytes`.  For streams whose chain is longer than the work
 // of everything that runs beside it (lat_cost): sync pass of 146 KB at 3.1
 // bits per symbol, L = 4096: 290 -> 132 us, of 5 MB at 2.5 576 -> 308; on all

@@ -18,15 +18,23 @@ def _arr(batch, specs):
     return (batch.StreamDesc * len(ds))(*ds)
 
 
-def _check(mg, specs):
+def _inside(mg, specs):
+    """Bytes of each stream in the batch, and the descriptors."""
     from multians_gb300 import batch
     lib = batch._sig()
     vp, sz = ctypes.c_void_p, ctypes.POINTER(ctypes.c_size_t)
-    lib.mans_batch_slice_size.argtypes = [vp, vp, sz]
     lib.mans_batch_data_sizes.argtypes = [vp, ctypes.c_uint32, vp, sz]
     arr = _arr(batch, specs)
     inside = (ctypes.c_size_t * len(specs))()
     assert lib.mans_batch_data_sizes(arr, len(specs), None, inside) == 0
+    return list(inside), arr
+
+
+def _check(mg, specs):
+    inside, arr = _inside(mg, specs)
+    lib = mg.lib()
+    lib.mans_batch_slice_size.argtypes = [ctypes.c_void_p, ctypes.c_void_p,
+                                          ctypes.POINTER(ctypes.c_size_t)]
     v = ctypes.c_size_t()
     for i in range(len(specs)):
         assert lib.mans_batch_slice_size(ctypes.byref(arr[i]), None, ctypes.byref(v)) == 0
@@ -51,3 +59,15 @@ def test_random_batches(mg, seed, flags):
             specs.append((max(1, int(n_out * bps / 32)), n_out,
                           int(rng.choice([64, 1024, 2048, 4096, 8192])), flags))
         _check(mg, specs)
+
+
+@pytest.mark.parametrize("k,deep", [(0.1, True), (0.25, False), (1.0, False)])
+def test_long_streams_have_no_deep_lattice(mg, k, deep):
+    """The sparse company above asks for 32 slots a block (blocks of 16 units,
+    eight bytes a slot), whose scan goes from tile to tile in order: not past
+    512 tiles of 1024 blocks."""
+    n_units = int(58_198_146 * k)
+    inside, _ = _inside(mg, [(n_units, int(935_418_631 * k), 1024, 0)] +
+                        [(int(1_500_000 * k), int(800_000_000 * k), 1024, 0)] * 12)
+    assert (n_units // 16 <= 512 * 1024) == deep
+    assert (inside[0] >= n_units // 16 * 32 * 8) == deep
