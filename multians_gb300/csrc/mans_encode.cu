@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
     const uint32_t D = p.D, L = p.L;
 
     bool on = false, exhausted = false;
-    uint32_t b = 0, x = 0, q = 0, val = 0, cas = 0, prev = 0, pbits = 0, life = 0, max_life = 0;
+    uint32_t b = 0, x = 0, q = 0, val = 0, cas = 0, pbits = 0, life = 0, max_life = 0;
+    uint32_t* prev = nullptr;   // node of the block before (its index may need more than 32 bits)
     bool has_prev = false, first = false;
     for (;;) {
         const uint32_t idle = __ballot_sync(0xffffffffu, !on && lane < p.width);
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
             if (cas == val) found = true;
             else q = lat_take(p.key + (size_t) b * D, q + 1, lat_usable(kEncSlots), val, found);
         }
-        if (has_prev) p.node[prev] = pbits | (q << kLatNodeShift);
+        if (has_prev) *prev = pbits | (q << kLatNodeShift);
         if (found || q == kLatDead || !more) {
             if (!more && !found && q != kLatDead)
                 p.end[q] = {x, bits, x_in & ((1u << len) - 1u), len};
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
             max_life = max(max_life, life);
             continue;
         }
-        prev = b * D + q;
+        prev = p.node + (size_t) b * D + q;
         has_prev = true;
         pbits = bits;
         val = kLatKeyUsed | (x - L);
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kEncThreads) k_enc_sync(EncParams p) {
         if (kn.w == val) hit = 3;
         ++b;
         if (hit != kLatDead) {
-            p.node[prev] = pbits | (hit << kLatNodeShift);
+            *prev = pbits | (hit << kLatNodeShift);
             on = false;
             max_life = max(max_life, life);
             continue;
@@ -642,7 +643,7 @@ int mans_encode(const uint8_t* d_sym, size_t n, const uint32_t* d_enc_blob, uint
         (L & (L - 1)) != 0 || ((uintptr_t) d_sym & 15) != 0 || ((uintptr_t) d_enc_blob & 3) != 0)
         return MANS_ERR_ARG;
     const EncPlan e = enc_plan(n, L, chunk_hint);
-    if ((unsigned long long) e.nblk * e.D > 0xffffffffull) return MANS_ERR_ARG;
+    if (e.nblk > 0xfffff000u) return MANS_ERR_ARG;   // 549 GB
     const EncLayout lay = enc_layout(e);
     if (aux_bytes < lay.total) return MANS_ERR_AUX_SMALL;
     if (cap_units < mans_encode_max_units(n, L)) return MANS_ERR_AUX_SMALL;
