@@ -703,7 +703,8 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     // (16 warps an SM don't cover the copy's latency: 217 -> 211 us)
     if ((uint64_t) b + step * 32 < p.nblk) {
         const uint32_t nx = b + step * 32;
-        if (kB == 32 || (lane & (32 / kB - 1)) == 0)
+        // (a stream that ends with a block has one more, without units)
+        if ((kB == 32 || (lane & (32 / kB - 1)) == 0) && (uint64_t) nx * kB < p.n_units)
             asm volatile("prefetch.global.L2 [%0];" :: "l"(p.units + (uint64_t) nx * kB));
         if ((lane & 15) == 0) asm volatile("prefetch.global.L2 [%0];" :: "l"(p.start + nx));
     }
