@@ -700,11 +700,11 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     __syncwarp();
     lat_turn_rows<kB>(tile, lane);
     // the next group's units and starts on their way into L2 meanwhile
-    // (16 warps an SM don't cover the copy's latency: 217 -> 211 us)
-    if ((uint64_t) b + step * 32 < p.nblk) {
+    // (16 warps an SM don't cover the copy's latency: 217 -> 211 us); not those
+    // of the last block, which has none where the stream ends with a block
+    if ((uint64_t) b + step * 32 + 1 < p.nblk) {
         const uint32_t nx = b + step * 32;
-        // (a stream that ends with a block has one more, without units)
-        if ((kB == 32 || (lane & (32 / kB - 1)) == 0) && (uint64_t) nx * kB < p.n_units)
+        if (kB == 32 || (lane & (32 / kB - 1)) == 0)
             asm volatile("prefetch.global.L2 [%0];" :: "l"(p.units + (uint64_t) nx * kB));
         if ((lane & 15) == 0) asm volatile("prefetch.global.L2 [%0];" :: "l"(p.start + nx));
     }
