@@ -91,7 +91,7 @@ struct LatParams {
     // 179, 143, 127).  Short streams are repaired to their end: 600,000 of two
     // symbols 10 ms, by regions 32.
     __device__ __forceinline__ uint32_t repair_blocks() const {
-        return n_units <= 32768 ? ~0u : (L <= 1024 ? max(L / 4, 64u) : max(L / 8, 256u));
+        return n_units <= 32768 ? ~0u : max(L / 8, 256u);
     }
     __device__ __forceinline__ void finish(uint32_t, unsigned long long) const {}
     __device__ __forceinline__ void finish_seq(const uint32_t*, uint32_t, unsigned long long) const {}
