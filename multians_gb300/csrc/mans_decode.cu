@@ -2229,6 +2229,18 @@ constexpr double kSeedMinBits = 1.0;
 constexpr double kSeedMaxBits = 4.5;
 constexpr double kSeedMaxBitsLarge = 7.0;   // L >= 4096
 
+// Whether every code is eight bits long (a table of one state a symbol, the
+// longest code it has): every start stands at the true path's phase, as a unit
+// holds four, walks end at once, and a decode that captures its symbols does
+// all the work once.  Where capture is planned it keeps such streams (128 MB 284
+// us, lattice 335; 512 MB 905, 1173; in batches, which plan regions without
+// the table's figures, 401 and 377, 1300 and 1310).  A few shorter codes put the starts at all
+// phases (16 MB at 7.96 bits: lattice 245 us, regions run out of walk slots), as
+// do lengths that do not divide a unit (L = 128 at 6.99 bits: 236, 315).
+static bool eight_bit_codes(uint32_t L, size_t n_units, size_t n_out) {
+    return L == 256 && n_units > n_out / 4;
+}
+
 // The planner's choices a measured table entry overrides (see
 // mans_tune_table.h): units per block, the shortest region in mean meeting
 // distances, and symbol capture.
@@ -2252,9 +2264,9 @@ static int plan_core(size_t n_units, size_t n_out, uint32_t L, const mans_cfg* h
              : (n_out > 0 && L <= kCaptureMaxL && bps >= kCaptureMinBits &&
                 (n_units >= kCaptureMinUnits || (c.flags & MANS_DECODE_CAPTURE)))));
     // the lattice decode where the plan is the planner's own (a plan given
-    // back as a hint keeps its choice)
+    // back as a hint keeps its choice), and capture does not beat it
     const bool lattice =
-        n_out > 0 &&
+        n_out > 0 && !(capture && !(c.flags & MANS_DECODE_LATTICE) && eight_bit_codes(L, n_units, n_out)) &&
         ((c.flags & MANS_DECODE_LATTICE) ||
          (c.block_units == 0 && c.region_blocks == 0 && c.walk_slots == 0 && c.capture_bytes == 0 &&
           !(c.flags & (MANS_DECODE_SEEDS | MANS_DECODE_NO_SEEDS | MANS_DECODE_NO_CAPTURE |
