@@ -796,12 +796,18 @@ __device__ __forceinline__ void lat_final_body(const LatParams& p, uint32_t cta,
     extern __shared__ __align__(16) uint32_t lat_sm[];
     const uint32_t st = *(volatile uint32_t*) p.status;
     if (st & MANS_DEV_DEGENERATE) {
-        // single-symbol table: every state decodes that symbol
-        const uint8_t sym = (uint8_t) (__ldg(p.table) >> 16);
+        // single-symbol table: every state decodes that symbol.  Such a stream is
+        // one unit long and has one CTA, so the stores are as wide as they get
+        // (128 MB by bytes 35.5 ms)
+        const uint32_t v = (__ldg(p.table) >> 16 & 0xffu) * 0x01010101u;
         const unsigned long long stride = (unsigned long long) nctas * blockDim.x;
-        for (unsigned long long i = (unsigned long long) cta * blockDim.x + threadIdx.x;
-             i < p.n_out; i += stride)
-            p.out[i] = sym;
+        const unsigned long long t = (unsigned long long) cta * blockDim.x + threadIdx.x;
+        const unsigned long long head = min(p.n_out, (unsigned long long) ((16 - ((uintptr_t) p.out & 15)) & 15));
+        const unsigned long long nv = (p.n_out - head) >> 4;
+        uint4* q = reinterpret_cast<uint4*>(p.out + head);
+        for (unsigned long long i = t; i < nv; i += stride) q[i] = make_uint4(v, v, v, v);
+        for (unsigned long long i = t; i < head; i += stride) p.out[i] = (uint8_t) v;
+        for (unsigned long long i = head + 16 * nv + t; i < p.n_out; i += stride) p.out[i] = (uint8_t) v;
         return;
     }
     if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_SYNC_OVERFLOW | MANS_DEV_SCAN_TIMEOUT)) return;
