@@ -81,17 +81,17 @@ struct LatParams {
 
     // scan hooks (mans_lattice_scan.cuh): an entry is the bit offset from the
     // block start and the state index << 8, an offset counts symbols
-    // 10 us a block at L = 1024, up to 37 at 4096.  A blocking call then
+    // 7 us a block at L = 256, 10 at 1024, up to 37 at 4096.  A blocking call then
     // decodes by regions four times the plan's, which on such data also fail at
     // their plain length and take that long to (L = 1024 3 to 6 ms, L = 4096 9
     // to 18): it loses no time to the lattice.  No stream that plain regions
-    // decode was seen to need more (256 blocks at most, 2 to 256 symbols of
-    // about equal frequency, up to 64 MB).  With 4096 blocks 16 M of eight such
+    // decode was seen to need more (2 to 256 symbols of about equal
+    // frequency, L = 8 to 8192, up to 64 MB).  With 4096 blocks 16 M of eight such
     // symbols, L = 1024, took 70 ms a call, by regions alone 32, now 30 (L = 4096:
     // 179, 143, 127).  Short streams are repaired to their end: 600,000 of two
     // symbols 10 ms, by regions 32.
     __device__ __forceinline__ uint32_t repair_blocks() const {
-        return n_units <= 32768 ? ~0u : max(L / 8, 256u);
+        return n_units <= 32768 ? ~0u : L <= 1024 ? max(L / 4, 128u) : max(L / 8, 256u);
     }
     __device__ __forceinline__ void finish(uint32_t, unsigned long long) const {}
     __device__ __forceinline__ void finish_seq(const uint32_t*, uint32_t, unsigned long long) const {}
