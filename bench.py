@@ -44,6 +44,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -197,12 +198,22 @@ def workload_config(args, n_symbols, n_units):
             "L": args.L, "seed": args.seed}
 
 
-def planner_report(mg, st, args):
-    """Where the decode's plan came from: the measured table entry the
-    planner used (multians_gb300/tune.py wrote it from GB300 timings), or the
-    model where the table has none or the run fixed the capture."""
+def planner_report(mg, st, args, cfg, sync):
+    """Which decode the plan is (and, for the lattice, its geometry from the
+    decode's own report), and where its region geometry came from: the measured
+    table entry the planner used (multians_gb300/tune.py wrote it from GB300
+    timings), or the model where the table has none or the run fixed the
+    capture.  A lattice decode uses that geometry only when it is retried."""
     entry = None if args.no_capture else mg.tune_lookup(st.L, st.bits_per_symbol, st.n)
-    return {"source": "measured table" if entry else "model", "entry": entry}
+    source = "measured table" if entry else "model"
+    if not cfg.get("flags", 0) & mg.DECODE_LATTICE:
+        return {"decode": "regions", "source": source, "entry": entry}
+    lattice = None
+    if sync.get("blocks"):
+        lattice = {"blocks": sync["blocks"], "starts": sync["regions"],
+                   "units_per_block": 1 << round(math.log2(st.n_units / sync["blocks"]))}
+    return {"decode": "lattice", "source": "model of the meeting distance", "lattice": lattice,
+            "regions": {"source": source, "entry": entry}}
 
 
 def make_workload(args, rank):
@@ -516,7 +527,7 @@ def run_ours(args, ws, rank, local):
         "stream": {"compressed_bytes": comp_bytes,
                    "bits_per_symbol": round(st.bits_per_symbol, 4)},
         "geometry": cfg,
-        "planner": planner_report(mg, st, args),
+        "planner": planner_report(mg, st, args, cfg, sync),
         "l2": "inputs larger than L2 (stream + output > 129 MB), no flush",
         "parallelism": "replicas" if ws > 1 else "single",
         "bit_exact": bit_exact,
