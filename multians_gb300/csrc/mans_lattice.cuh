@@ -1,6 +1,7 @@
-// Lattice decode: the sync and final passes of streams whose merges bound
-// them (every uncaptured plain decode with the planner's own plan, and
-// batches).
+// Lattice decode: the sync and final passes of every plain decode with the
+// planner's own plan (but for long streams of eight-bit codes, which symbol
+// capture keeps) and of the streams of a batch that fix no geometry, capture or
+// seeds.
 //
 // The stream is cut into blocks of B units.  Trajectories start from a
 // guess (bit 0, the stream's first state) every nb blocks, the first one
@@ -72,7 +73,7 @@ struct LatParams {
     uint32_t first_pos;
     uint32_t B;                     // units per block: 4, 8, 16 or 32
     uint32_t nb;                    // blocks between starts
-    uint32_t D;                     // slots per block: 4, 8, 12 or 16
+    uint32_t D;                     // slots per block: 4, 8, 12, 16 or 32
     uint32_t nblk;
     uint32_t nseed;
     uint32_t stage_cap;             // final-pass staging bytes per warp
@@ -275,8 +276,8 @@ struct LatMid {
 
 // Two steps with one unit load and one refill: the second step's window is
 // cut from both units (offset < 32 + 16, code <= 16 bits), and two codes pass
-// at most one unit.  4.0 cycles a warp and step with the shared pipe full
-// against 4.5 for single steps, 47 against 47.5 alone.
+// at most one unit.  Against single steps 4.0 cycles a warp and step
+// for 4.5 with the shared pipe full, and half a cycle less alone.
 __device__ __forceinline__ void lat_pair(LatCursor& c, uint32_t col, uint32_t mask, uint32_t& y1,
                                          uint32_t& y2, LatMid& m) {
     m.u = lds32(col + ((c.pos & mask) << 2));
@@ -375,8 +376,9 @@ __host__ __device__ constexpr uint32_t lat_ring_bytes(uint32_t B) { return 2 * B
 // close up into fewer warps (128 MB at 1.5 bits per symbol, L = 4096: sync
 // pass 990 -> 893 us; 256 threads a CTA instead of 128: 16 MB 91 -> 106, a
 // batch 579 -> 683).  Bound by the longest trajectory's chain of lookups on
-// short streams (57 cycles a step with the block's bookkeeping, 47 for the
-// loop alone, against 62 to 83 for the 8-byte entries and a test per step)
+// short streams (36 cycles a step, and 1200 to 3000 a block beside its steps;
+// 47 a step before the code's bits were cut out by one instruction, 62 to 83
+// with 8-byte entries and a test per step)
 // and by the L1 data pipe (4.0 passes a warp and step for the lookups, about
 // two more for the lanes' own loads of units and slots) once 16 warps run
 // on every SM.  The slots of the next block and the units of the
@@ -701,8 +703,9 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     lat_turn_rows<kB>(tile, lane);
     // the next group's units and starts on their way into L2 meanwhile
     // (16 warps an SM don't cover the copy's latency: 217 -> 211 us); not those
-    // of the last block, which has none where the stream ends with a block
-    if ((uint64_t) b + step * 32 + 1 < p.nblk) {
+    // of the last block, which has none where the stream ends with a block (the
+    // test written with + 1 on the left: 256 MB at 0.67 bits 270 -> 274 us)
+    if ((uint64_t) b + step * 32 < p.nblk - 1) {
         const uint32_t nx = b + step * 32;
         if (kB == 32 || (lane & (32 / kB - 1)) == 0)
             asm volatile("prefetch.global.L2 [%0];" :: "l"(p.units + (uint64_t) nx * kB));
@@ -790,24 +793,30 @@ __device__ __forceinline__ bool lat_final_warp(const LatParams& p, uint32_t tb, 
     return true;
 }
 
+// The CTA's share of an output of one symbol.  Such a stream is one unit long
+// and has one CTA, so the stores are as wide as they get (128 MB by bytes 35.5
+// ms, so 2.0).  Not inlined: it would cost the batched pass registers (69 -> 80).
+__device__ __noinline__ void lat_fill(uint8_t* out, unsigned long long n, uint32_t sym, uint32_t cta,
+                                      uint32_t nctas) {
+    const uint32_t v = sym * 0x01010101u;
+    const unsigned long long stride = (unsigned long long) nctas * blockDim.x;
+    const unsigned long long t = (unsigned long long) cta * blockDim.x + threadIdx.x;
+    const unsigned long long head = min(n, (unsigned long long) ((16 - ((uintptr_t) out & 15)) & 15));
+    const unsigned long long nv = (n - head) >> 4;
+    uint4* q = reinterpret_cast<uint4*>(out + head);
+    for (unsigned long long i = t; i < nv; i += stride) q[i] = make_uint4(v, v, v, v);
+    for (unsigned long long i = t; i < head; i += stride) out[i] = (uint8_t) v;
+    for (unsigned long long i = head + 16 * nv + t; i < n; i += stride) out[i] = (uint8_t) v;
+}
+
 // Shared memory of a final-pass CTA: table, unit tiles, staging buffers.
 template <bool kRev, uint32_t kB>
 __device__ __forceinline__ void lat_final_body(const LatParams& p, uint32_t cta, uint32_t nctas) {
     extern __shared__ __align__(16) uint32_t lat_sm[];
     const uint32_t st = *(volatile uint32_t*) p.status;
     if (st & MANS_DEV_DEGENERATE) {
-        // single-symbol table: every state decodes that symbol.  Such a stream is
-        // one unit long and has one CTA, so the stores are as wide as they get
-        // (128 MB by bytes 35.5 ms)
-        const uint32_t v = (__ldg(p.table) >> 16 & 0xffu) * 0x01010101u;
-        const unsigned long long stride = (unsigned long long) nctas * blockDim.x;
-        const unsigned long long t = (unsigned long long) cta * blockDim.x + threadIdx.x;
-        const unsigned long long head = min(p.n_out, (unsigned long long) ((16 - ((uintptr_t) p.out & 15)) & 15));
-        const unsigned long long nv = (p.n_out - head) >> 4;
-        uint4* q = reinterpret_cast<uint4*>(p.out + head);
-        for (unsigned long long i = t; i < nv; i += stride) q[i] = make_uint4(v, v, v, v);
-        for (unsigned long long i = t; i < head; i += stride) p.out[i] = (uint8_t) v;
-        for (unsigned long long i = head + 16 * nv + t; i < p.n_out; i += stride) p.out[i] = (uint8_t) v;
+        // single-symbol table: every state decodes that symbol
+        lat_fill(p.out, p.n_out, __ldg(p.table) >> 16 & 0xffu, cta, nctas);
         return;
     }
     if (st & (MANS_DEV_BAD_TABLE | MANS_DEV_SYNC_OVERFLOW | MANS_DEV_SCAN_TIMEOUT)) return;
