@@ -2851,7 +2851,7 @@ int mans_sync_stats_get(const void* d_aux, size_t aux_bytes, size_t n_units, siz
         // decoded past the first time as walks
         mans_sync_stats s{};
         uint64_t visits = 0, longest = 0;
-        if (!lat_stats(lp, d_aux, (cudaStream_t) stream, &visits, &longest)) return MANS_ERR_CUDA;
+        if (!lat_stats(d_aux, (cudaStream_t) stream, &visits, &longest)) return MANS_ERR_CUDA;
         s.regions = lp.nseed;
         s.blocks = lp.nblk;
         s.walks = lp.nseed - 1;

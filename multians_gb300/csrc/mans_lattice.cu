@@ -428,14 +428,12 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
     return cudaGetLastError() == cudaSuccess ? 4u : 0u;
 }
 
-bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t st, uint64_t* visits,
-               uint64_t* longest) {
+bool lat_stats(const void* d_aux, cudaStream_t st, uint64_t* visits, uint64_t* longest) {
     uint32_t c[8] = {};
     if (cudaMemcpyAsync(c, (const char*) d_aux + 256, sizeof(c), cudaMemcpyDeviceToHost, st) !=
             cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return false;
-    (void) plan;
     *visits = c[kLatVisits];
     *longest = c[kLatMaxLife];
     return true;

@@ -64,8 +64,7 @@ uint32_t lat_decode(const LatCall& call, const LatPlan& plan, void* d_aux, cudaS
 
 // What the trajectories of the last lattice decode in d_aux cost (waits for
 // the stream): blocks decoded by all of them, blocks of the longest.
-bool lat_stats(const LatPlan& plan, const void* d_aux, cudaStream_t stream, uint64_t* visits,
-               uint64_t* longest);
+bool lat_stats(const void* d_aux, cudaStream_t stream, uint64_t* visits, uint64_t* longest);
 
 // Batched decodes.  The parameters of a stream are lat_params_size() bytes;
 // the batch keeps one array of them and lists of work items on the device.
