@@ -3047,9 +3047,9 @@ int mans_decode_loop(const mans_stream_desc* streams, uint32_t n, const mans_cfg
 // the whole batch).  Streams that neither ask for capture nor fix a geometry go
 // through the lattice kernels (mans_lattice.cu), the others through the
 // BatchItem kernels above.  Measured, regions and walks -> lattice: 256
-// streams of 4 KB to 4 MB, L = 1024 1922 -> 932 us; 1024 of them 3555 -> 2296;
-// 48 streams of 1 to 256 KB, L = 1024 and 4096, in one call 2690 -> 770; 64
-// requests up to 8 MB through the serving loop 4621 -> 1770.
+// streams of 4 KB to 4 MB, L = 1024 1986 -> 834 us; 48 streams of 1 to 256 KB,
+// L = 1024 and 4096, in one call 2721 -> 418; 64 requests up to 8 MB through the
+// serving loop 4954 -> 1008.
 
 }  // extern "C"
 

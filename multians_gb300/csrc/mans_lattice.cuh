@@ -27,11 +27,11 @@
 // against 7000.  The price is work: every unit is decoded sqrt(2 T / s)
 // times, so starts are spread no closer than the GPU has idle lanes for.
 //
-// Measured on GB300, whole decodes, regions and walks -> lattice: 4 KB 151 ->
-// 87 us, 128 KB at 3.8 bits per symbol 463 -> 156, 16 MB at 6 bits 328 ->
-// 190, 128 MB at 1.5 bits and L = 4096 4171 -> 1133, 256 MB at 0.67 bits and
-// L = 4096 2478 -> 946; against regions with symbol capture, 256 MB at 6 bits
-// 693 -> 619, 512 MB at 8.6 bits 1440 -> 1168.
+// Measured on GB300, whole decodes, regions and walks -> lattice: 4 KB 144 ->
+// 72 us, 128 KB at 3.8 bits per symbol 477 -> 113, 16 MB at 6 bits 353 ->
+// 171, 128 MB at 1.5 bits and L = 4096 4340 -> 990, 256 MB at 0.67 bits and
+// L = 4096 2621 -> 916; against regions with symbol capture, 256 MB at 6 bits
+// 690 -> 536, 512 MB at 8.6 bits 1447 -> 1036.
 #pragma once
 
 #include <cstdint>
